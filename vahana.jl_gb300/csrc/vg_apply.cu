@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <type_traits>
 
 #include "vg_internal.h"
 
@@ -210,7 +211,21 @@ struct RedArgs {
   double init_f;
   int64_t neut_i;   // neutral element of op for the partial reductions
   double neut_f;
+  // `arg` for comparisons with integers of up to 32 bits, which are then
+  // compared as integers (a 64-bit conversion and comparison per element
+  // would go to the FP64 pipe): x < arg as x < ceil(arg), x > arg as
+  // x > floor(arg), x == arg never when arg is no such integer
+  int64_t thr;
 };
+
+int64_t integer_threshold(int kind, double arg) {
+  const double far = 1099511627776.0;  // 2^40: beyond every such integer
+  if (std::isnan(arg)) return kind == VG_MAP_LT ? -(1ll << 40) : 1ll << 40;
+  if (kind == VG_MAP_EQ || kind == VG_MAP_NE)
+    return std::fabs(arg) < far && arg == std::floor(arg) ? (int64_t)arg : 1ll << 40;
+  const double t = kind == VG_MAP_LT ? std::ceil(arg) : std::floor(arg);
+  return (int64_t)std::min(std::max(t, -far), far);
+}
 
 // pass 1: per-block partial (deterministic block order): each thread folds
 // its strided elements, each warp combines its 32 lanes by shuffles in a
@@ -225,26 +240,82 @@ __device__ __forceinline__ void warp_combine(int op, int64_t &vi, double &vf) {
   }
 }
 
-__global__ void k_reduce_partial(RedArgs a, int64_t *pi, double *pf) {
+// The field itself as column type E (no per-element type switch), RED_U
+// loads in flight per thread.  Bound: instruction issue (about 20 per
+// element).  One element at a time, its type looked up for each and every
+// value also taken through the FP64 pipe, took 51 us for 5e6 Int32; this
+// takes 21 us.  The elements of a thread are folded in index order.
+constexpr int RED_U = 8;
+
+template <class E>
+__device__ __forceinline__ void map_elem(const RedArgs &a, E e, int64_t *vi, double *vf) {
+  constexpr bool isf = std::is_floating_point<E>::value;
+  *vi = 0;
+  *vf = 0.0;
+  if (a.kind == VG_MAP_FIELD) {
+    if (!a.float_acc) *vi = (int64_t)e;
+    else *vf = isf ? (double)e : (double)(int64_t)e;
+    return;
+  }
+  bool r = false;
+  if (!isf && sizeof(E) <= 4) {
+    const int64_t x = (int64_t)e;
+    switch (a.kind) {
+      case VG_MAP_EQ: r = x == a.thr; break;
+      case VG_MAP_NE: r = x != a.thr; break;
+      case VG_MAP_LT: r = x < a.thr; break;
+      case VG_MAP_GT: r = x > a.thr; break;
+    }
+  } else {
+    const double x = isf ? (double)e : (double)(int64_t)e;
+    switch (a.kind) {
+      case VG_MAP_EQ: r = x == a.arg; break;
+      case VG_MAP_NE: r = x != a.arg; break;
+      case VG_MAP_LT: r = x < a.arg; break;
+      case VG_MAP_GT: r = x > a.arg; break;
+    }
+  }
+  if (a.float_acc) *vf = r;
+  else *vi = r;
+}
+
+template <class E>
+__global__ void __launch_bounds__(TPB) k_reduce_partial(RedArgs a, int64_t *pi, double *pf) {
   __shared__ int64_t si[TPB / 32];
   __shared__ double sf[TPB / 32];
   int64_t acc_i = a.neut_i;
   double acc_f = a.neut_f;
   bool have = false;
+  const E *col = (const E *)a.p;
   uint64_t chunk = (a.n + gridDim.x - 1) / gridDim.x;
   uint64_t b = (uint64_t)blockIdx.x * chunk, e = min(a.n, b + chunk);
-  for (uint64_t i = b + threadIdx.x; i < e; i += blockDim.x) {
-    if (a.died && a.died[i]) continue;
-    int64_t vi;
-    double vf;
-    map_val(a.kind, a.arg, a.p, a.dt, i, a.float_acc, &vi, &vf);
-    if (!have) {
-      acc_i = vi;
-      acc_f = vf;
-      have = true;
-    } else {
-      acc_i = red_i(a.op, vi, acc_i);
-      acc_f = red_f(a.op, vf, acc_f);
+  for (uint64_t i0 = b + threadIdx.x; i0 < e; i0 += (uint64_t)RED_U * TPB) {
+    E v[RED_U];
+    bool use[RED_U];
+#pragma unroll
+    for (int u = 0; u < RED_U; u++) {
+      const uint64_t i = i0 + (uint64_t)u * TPB;
+      use[u] = i < e;
+      v[u] = use[u] ? col[i] : E(0);
+    }
+    if (a.died) {
+#pragma unroll
+      for (int u = 0; u < RED_U; u++) use[u] = use[u] && !a.died[i0 + (uint64_t)u * TPB];
+    }
+#pragma unroll
+    for (int u = 0; u < RED_U; u++) {
+      if (!use[u]) continue;
+      int64_t vi;
+      double vf;
+      map_elem<E>(a, v[u], &vi, &vf);
+      if (!have) {
+        acc_i = vi;
+        acc_f = vf;
+        have = true;
+      } else {
+        if (!a.float_acc) acc_i = red_i(a.op, vi, acc_i);
+        else acc_f = red_f(a.op, vf, acc_f);
+      }
     }
   }
   // empty threads contribute the neutral element
@@ -270,21 +341,40 @@ __global__ void k_reduce_partial(RedArgs a, int64_t *pi, double *pf) {
   }
 }
 
-__global__ void k_reduce_final(const int64_t *pi, const double *pf, int nb, int op,
-                               int64_t init_i, double init_f, int64_t *oi, double *of) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int64_t ai = init_i;
-  double af = init_f;
-  for (int b = 0; b < nb; b++) {
-    ai = red_i(op, pi[b], ai);
-    af = red_f(op, pf[b], af);
+// pass 2: the blocks' results by one block in the same fixed tree, then the
+// reduction's init.  Threads without a partial hold what changes no other
+// value (-0.0 for Float +: x + -0.0 is x for every x).  One thread folding
+// 1024 partials, each a load and an operation behind the last, took 97 us.
+constexpr int RED_BLOCKS = 1024;
+
+__global__ void __launch_bounds__(RED_BLOCKS) k_reduce_final(const int64_t *pi, const double *pf,
+                                                             int nb, RedArgs a, int64_t *oi,
+                                                             double *of) {
+  __shared__ int64_t si[32];
+  __shared__ double sf[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double fill = a.op == VG_OP_ADD ? -0.0 : a.neut_f;
+  int64_t vi = (int)threadIdx.x < nb ? pi[threadIdx.x] : a.neut_i;
+  double vf = (int)threadIdx.x < nb ? pf[threadIdx.x] : fill;
+  warp_combine(a.op, vi, vf);
+  if (lane == 0) {
+    si[wid] = vi;
+    sf[wid] = vf;
   }
-  *oi = ai;
-  *of = af;
+  __syncthreads();
+  if (wid) return;
+  vi = si[lane];
+  vf = sf[lane];
+  warp_combine(a.op, vi, vf);
+  if (lane == 0) {
+    *oi = red_i(a.op, vi, a.init_i);
+    *of = red_f(a.op, vf, a.init_f);
+  }
 }
 
 // Sequential left fold in index order, reduced = op(f(x), reduced), the
-// reference's loop: one chain of dependent operations on thread 0.  The
+// reference's loop, for Float * and for folds that are asked to be ordered
+// (Float + takes vg_fold.cuh): one chain of dependent operations on thread 0.  The
 // block's other warps map the next tile of elements into shared memory
 // (value bits and whether the element counts) while thread 0 folds the
 // current tile, so the chain never waits for global memory.
@@ -317,10 +407,7 @@ __global__ void __launch_bounds__(ORD_TPB) k_reduce_ordered(RedArgs a, int64_t *
       if (t + 1 < ntiles) stage(t + 1, b ^ 1);
     } else if (threadIdx.x == 0) {
       const uint32_t m = (uint32_t)min((uint64_t)ORD_TILE, a.n - t * ORD_TILE);
-      if (a.float_acc && a.op == VG_OP_ADD) {
-        for (uint32_t k = 0; k < m; k++)
-          if (live[b][k]) af = __dadd_rn(__longlong_as_double(vbuf[b][k]), af);
-      } else if (a.float_acc) {
+      if (a.float_acc) {
         for (uint32_t k = 0; k < m; k++)
           if (live[b][k]) af = red_f(a.op, __longlong_as_double(vbuf[b][k]), af);
       } else {
@@ -335,6 +422,14 @@ __global__ void __launch_bounds__(ORD_TPB) k_reduce_ordered(RedArgs a, int64_t *
     *of = af;
   }
 }
+
+}  // namespace
+}  // namespace vg
+
+#include "vg_fold.cuh"
+
+namespace vg {
+namespace {
 
 void identity_for(int op, int out_dtype, int has_init, double init, int64_t *ii,
                   double *fi) {
@@ -396,29 +491,67 @@ bool fold_in_order(int flags, bool float_acc, int op) {
   return float_acc && (op == VG_OP_ADD || op == VG_OP_MUL);
 }
 
+// Columns of at most FOLD_SHORT tiles go straight to the chain: the three
+// launches that predict and map the tiles cost more than cutting one or two
+// tiles finer in the chain itself.
+constexpr uint64_t FOLD_SHORT = 2;
+
+template <bool F64>
+void launch_fold(const RedArgs &a, void *ws, int64_t *oi, double *of, cudaStream_t st) {
+  const uint64_t nt = (a.n + FOLD_TILE - 1) / FOLD_TILE;
+  if (nt <= FOLD_SHORT) {
+    k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, nullptr, nullptr, oi, of);
+    return;
+  }
+  FoldMap *maps = (FoldMap *)ws;
+  float *tsum = (float *)(maps + nt);
+  int *frame = (int *)(tsum + nt);
+  k_fold_sums<F64><<<(unsigned)nt, FOLD_TPB, 0, st>>>(a, tsum);
+  k_fold_frames<<<1, FOLD_CHAIN_TPB, 0, st>>>(tsum, nt, a.init_f, frame);
+  k_fold_tiles<F64><<<(unsigned)nt, FOLD_TPB, 0, st>>>(a, frame, maps);
+  k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, frame, maps, oi, of);
+}
+
 void run_reduce(Sim &s, RedArgs a, int out_dtype, bool ordered, void *out) {
   neutral_for(a.op, &a.neut_i, &a.neut_f);
   int64_t ri = a.init_i;
   double rf = a.init_f;
   if (a.n > 0) {
-    int64_t *d = nullptr;
-    VG_CUDA(cudaMallocAsync((void **)&d, 16 + 2 * 8 * 1024, s.stream));
-    int64_t *oi = d;
-    double *of = (double *)(d + 1);
-    if (ordered) {
+    const uint64_t tiles = (a.n + FOLD_TILE - 1) / FOLD_TILE;
+    // the simulation's workspace: the result, then partials or tile maps
+    char *d = (char *)s.scratch(64 + std::max<uint64_t>(2 * 8 * RED_BLOCKS,
+                                                        tiles * (sizeof(FoldMap) + 8)));
+    int64_t *oi = (int64_t *)d;
+    double *of = (double *)(d + 8);
+    if (ordered && a.float_acc && a.op == VG_OP_ADD) {
+      if (a.dt == VG_F64 && a.kind == VG_MAP_FIELD) launch_fold<true>(a, d + 64, oi, of, s.stream);
+      else launch_fold<false>(a, d + 64, oi, of, s.stream);
+    } else if (ordered) {
       k_reduce_ordered<<<1, ORD_TPB, 0, s.stream>>>(a, oi, of);
     } else {
-      int nb = (int)std::min<uint64_t>(1024, (a.n + TPB - 1) / TPB);
-      int64_t *pi = d + 2;
-      double *pf = (double *)(d + 2 + 1024);
-      k_reduce_partial<<<nb, TPB, 0, s.stream>>>(a, pi, pf);
-      k_reduce_final<<<1, 32, 0, s.stream>>>(pi, pf, nb, a.op, a.init_i, a.init_f, oi, of);
+      int nb = (int)std::min<uint64_t>(RED_BLOCKS, (a.n + TPB - 1) / TPB);
+      int64_t *pi = (int64_t *)(d + 64);
+      double *pf = (double *)(d + 64 + 8 * RED_BLOCKS);
+      a.thr = integer_threshold(a.kind, a.arg);
+      switch (a.dt) {
+        case VG_BOOL: case VG_U8: k_reduce_partial<uint8_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        case VG_I8: k_reduce_partial<int8_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        case VG_U16: k_reduce_partial<uint16_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        case VG_I16: k_reduce_partial<int16_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        case VG_U32: k_reduce_partial<uint32_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        case VG_I32: k_reduce_partial<int32_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        case VG_F32: k_reduce_partial<float><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        case VG_F64: k_reduce_partial<double><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
+        default: k_reduce_partial<int64_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf);
+      }
+      k_reduce_final<<<1, RED_BLOCKS, 0, s.stream>>>(pi, pf, nb, a, oi, of);
     }
     VG_CUDA(cudaGetLastError());
-    VG_CUDA(cudaMemcpyAsync(&ri, oi, 8, cudaMemcpyDeviceToHost, s.stream));
-    VG_CUDA(cudaMemcpyAsync(&rf, of, 8, cudaMemcpyDeviceToHost, s.stream));
-    VG_CUDA(cudaFreeAsync(d, s.stream));
+    int64_t res[2];
+    VG_CUDA(cudaMemcpyAsync(res, d, 16, cudaMemcpyDeviceToHost, s.stream));
     VG_CUDA(cudaStreamSynchronize(s.stream));
+    ri = res[0];
+    std::memcpy(&rf, &res[1], 8);
   }
   if (out_dtype == VG_F64) *(double *)out = a.float_acc ? rf : (double)ri;
   else if (out_dtype == VG_BOOL) *(uint8_t *)out = (a.float_acc ? rf : (double)ri) != 0;
