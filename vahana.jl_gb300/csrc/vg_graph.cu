@@ -947,6 +947,19 @@ __global__ void k_slice_deg(const uint32_t *rp, uint64_t nrows, const uint32_t *
   slots[sl] = 32ull * dm;
 }
 
+// flag the slices of at least thr slots
+__global__ void k_flag_long(const uint32_t *sdeg, uint64_t nslices, uint32_t thr, uint32_t *flag) {
+  uint64_t sl = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (sl < nslices) flag[sl] = sdeg[sl] >= thr ? 1u : 0u;
+}
+
+// sort key of a listed slice: descending length
+__global__ void k_long_keys(const uint32_t *sdeg, const uint32_t *list, uint64_t m,
+                            uint32_t *keys) {
+  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < m) keys[k] = 0xFFFFFFFFu - sdeg[list[k]];
+}
+
 // copy each row's edges into its slice, column-major; padding source 0,
 // weight 0
 __global__ void k_sell_fill(const uint32_t *__restrict__ rp, uint64_t nrows,
@@ -1015,6 +1028,9 @@ void ensure_schedule(Sim &s, CSR &c, uint32_t thr, uint32_t big_thr, uint64_t n)
   c.slice_deg.release();
   c.sell_src.release();
   c.sell_w.release();
+  c.long_slices.release();
+  c.long_slots.clear();
+  c.long_hubs.clear();
   c.nhub = c.norder = c.nslices = c.nbig = 0;
   c.range_block.clear();
   c.range_rows.clear();
@@ -1022,23 +1038,33 @@ void ensure_schedule(Sim &s, CSR &c, uint32_t thr, uint32_t big_thr, uint64_t n)
   c.hub_rows_sorted.clear();
   if (n > 0 && c.row_ptr.p) {
     const uint32_t *rp = c.row_ptr.as<uint32_t>();
+    // (a launch that folds other graphs' edges too only takes longer slices)
+    const uint32_t long_min = opinion_long_slots(c.nedges);
     // hub rows by descending degree
     c.nhub = select_rows(s, c, n, thr, 0xFFFFFFFFu, c.hub_rows);
-    if (c.nhub > 1) {
+    if (c.nhub) {
+      const uint32_t *rows = c.hub_rows.as<uint32_t>();
       Tmp<uint32_t> keys(c.nhub, st);
-      k_hub_keys<<<nblk(c.nhub), TPB, 0, st>>>(rp, c.hub_rows.as<uint32_t>(), c.nhub, keys.p);
+      k_hub_keys<<<nblk(c.nhub), TPB, 0, st>>>(rp, rows, c.nhub, keys.p);
       radix_sort_pairs_u32(keys.p, c.hub_rows.as<uint32_t>(), c.nhub, 32, st, s);
-    }
-    c.nbig = 0;
-    if (c.nhub && big_thr != 0xFFFFFFFFu) {  // the leading hubs above the block threshold
-      Tmp<unsigned> cnt(1, st);
-      VG_CUDA(cudaMemsetAsync(cnt.p, 0, 4, st));
-      k_count_above<<<nblk(c.nhub), TPB, 0, st>>>(rp, c.hub_rows.as<uint32_t>(), c.nhub,
-                                                  big_thr, cnt.p);
-      unsigned h = 0;
-      VG_CUDA(cudaMemcpyAsync(&h, cnt.p, 4, cudaMemcpyDeviceToHost, st));
+      // the leading hubs above the block threshold, and those that may take
+      // a block of the long launch
+      Tmp<unsigned> cnt(2, st);
+      VG_CUDA(cudaMemsetAsync(cnt.p, 0, 8, st));
+      k_count_above<<<nblk(c.nhub), TPB, 0, st>>>(rp, rows, c.nhub, big_thr, cnt.p);
+      k_count_above<<<nblk(c.nhub), TPB, 0, st>>>(rp, rows, c.nhub, 32 * long_min - 1,
+                                                  cnt.p + 1);
+      unsigned h[2] = {0, 0};
+      VG_CUDA(cudaMemcpyAsync(h, cnt.p, 8, cudaMemcpyDeviceToHost, st));
       VG_CUDA(cudaStreamSynchronize(st));
-      c.nbig = h;
+      c.nbig = h[0];
+      if (h[1]) {
+        c.long_hubs.resize(h[1]);
+        VG_CUDA(cudaMemcpyAsync(c.long_hubs.data(), keys.p, (uint64_t)h[1] * 4,
+                                cudaMemcpyDeviceToHost, st));
+        VG_CUDA(cudaStreamSynchronize(st));
+        for (uint32_t &k : c.long_hubs) k = 0xFFFFFFFFu - k;  // the sort's keys
+      }
     }
     // the other rows by descending degree in windows of 2^13 rows (or
     // more, so that the window number stays below the sentinel)
@@ -1065,7 +1091,30 @@ void ensure_schedule(Sim &s, CSR &c, uint32_t thr, uint32_t big_thr, uint64_t n)
       uint64_t total = 0;
       VG_CUDA(cudaMemcpyAsync(&total, c.slice_base.as<uint64_t>() + ns, 8, cudaMemcpyDeviceToHost,
                               st));
-      VG_CUDA(cudaStreamSynchronize(st));
+      // the long slices, listed longest first (no slice has more than thr slots)
+      if (thr >= long_min) {
+        Tmp<uint32_t> flag(ns + 1, st), pos(ns + 1, st);
+        VG_CUDA(cudaMemsetAsync(flag.p + ns, 0, 4, st));
+        k_flag_long<<<nblk(ns), TPB, 0, st>>>(c.slice_deg.as<uint32_t>(), ns, long_min, flag.p);
+        exclusive_scan_u32(flag.p, pos.p, ns + 1, st, s);
+        uint32_t nlong = 0;
+        VG_CUDA(cudaMemcpyAsync(&nlong, pos.p + ns, 4, cudaMemcpyDeviceToHost, st));
+        VG_CUDA(cudaStreamSynchronize(st));
+        if (nlong) {
+          Tmp<uint32_t> lkeys(nlong, st);
+          c.long_slices.alloc((uint64_t)nlong * 4, &s.footprint);
+          k_compact_rows<<<nblk(ns), TPB, 0, st>>>(flag.p, pos.p, ns,
+                                                   c.long_slices.as<uint32_t>());
+          k_long_keys<<<nblk(nlong), TPB, 0, st>>>(c.slice_deg.as<uint32_t>(),
+                                                   c.long_slices.as<uint32_t>(), nlong, lkeys.p);
+          radix_sort_pairs_u32(lkeys.p, c.long_slices.as<uint32_t>(), nlong, 32, st, s);
+          c.long_slots.resize(nlong);
+          VG_CUDA(cudaMemcpyAsync(c.long_slots.data(), lkeys.p, (uint64_t)nlong * 4,
+                                  cudaMemcpyDeviceToHost, st));  // (read after the wait below)
+        }
+      } else {
+        VG_CUDA(cudaStreamSynchronize(st));
+      }
       c.sell_src.alloc(std::max<uint64_t>(total, 1) * 4, &s.footprint);
       c.sell_w.alloc(std::max<uint64_t>(total, 1) * 8, &s.footprint);
       k_sell_fill<<<nblk(ns * 32), TPB, 0, st>>>(
@@ -1078,6 +1127,7 @@ void ensure_schedule(Sim &s, CSR &c, uint32_t thr, uint32_t big_thr, uint64_t n)
     }
     VG_CUDA(cudaGetLastError());
     VG_CUDA(cudaStreamSynchronize(st));
+    for (uint32_t &k : c.long_slots) k = 0xFFFFFFFFu - k;  // the sort's keys
   }
   c.sched_n = n;
   c.hub_threshold = thr;

@@ -188,6 +188,12 @@ struct CSR {
   DevBuf slice_base;  // u64 [nslices + 1]: first column-major slot of each slice
   DevBuf slice_deg;   // u32 [nslices]: the slice's largest degree
   uint64_t nslices = 0;
+  // slices of opinion_long_slots(nedges) slots or more, longest first, and
+  // their slots
+  DevBuf long_slices;  // u32
+  std::vector<uint32_t> long_slots;
+  // in-degrees of the leading hub rows with 32 times as many edges or more
+  std::vector<uint32_t> long_hubs;
   DevBuf sell_src;  // u32 [slots]
   DevBuf sell_w;    // f64 [slots]
   uint64_t sched_n = 0;  // agent count the layout covers
@@ -420,6 +426,22 @@ void tr_bounded_confidence(ApplyCtx &ctx);  // vg_opinion.cu
 // split across a warp (1e-12 relative), rows at or below it fold in order
 // (bit-exact); 1536 measured fastest on the benchmark graph
 constexpr uint32_t OPINION_HUB_DEFAULT = 1536;
+
+// Slices of at least this many slots take a block each when `edges` edges
+// are folded in one launch.  A slice of D slots takes a warp 340 ns D, the
+// launch at its full rate 4.5 ps per edge: a slice that would take more than
+// about 0.6 of the launch is long (edges / 125000 slots).  Measured, us per
+// step with the slices from 96, 192, 400, 800 and 1200 slots on in blocks,
+// and none: 2*10^7 edges 190, 176, 175, 280, 383, 491; 6*10^7 335, 315, 306,
+// 383, 521, 651; 10^8 555, 521, 502, 479, 577, 709; 2*10^8 1215, 1152, 1114,
+// 1094, 985 and 898: there the launch hides its longest rows (up to 1536
+// slots), and the blocks' shared memory would only take L1 from the gathers.
+// A hub row's warp takes 8 ns per edge: hub rows of 32 times as many edges
+// are long.
+inline uint32_t opinion_long_slots(uint64_t edges) {
+  const uint64_t slots = edges / 125000;
+  return slots < 96 ? 96u : slots < (1u << 26) ? (uint32_t)slots : 1u << 26;
+}
 
 struct OpinionJob {
   Sim *sim;

@@ -70,6 +70,12 @@ struct OpinionArgs {
   const uint32_t *__restrict__ sell_src;
   const double *__restrict__ sell_w;
   uint64_t nslices;
+  // the first nlong slices of this list (those of long_slots slots or more)
+  // and the first long_hubs hub rows after the block-wide ones take a block
+  // of k_opinion_long each
+  const uint32_t *__restrict__ long_slices;
+  unsigned nlong, long_hubs;
+  uint32_t long_slots;
   uint32_t hub_thr;
   unsigned hub_blocks;   // blocks of the other hub rows, 4 per block
   double eps, a, b;
@@ -290,6 +296,24 @@ __device__ __forceinline__ void sell_slice(const OpinionArgs &p, uint64_t sl) {
   p.xo[r] = any ? finish(p, xi, bits(a.sw), bits(a.swx)) : xi;
 }
 
+// the 32 lane sums of a hub row combined in a fixed tree (lane l receives
+// lane l + off); the result is on lane 0
+__device__ __forceinline__ uint32_t hub_tree(uint64_t &sw, uint64_t &swx, uint32_t cnt) {
+  const unsigned lane = threadIdx.x & 31;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    uint64_t osw = __shfl_down_sync(0xffffffffu, sw, off);
+    uint64_t oswx = __shfl_down_sync(0xffffffffu, swx, off);
+    uint32_t ocnt = __shfl_down_sync(0xffffffffu, cnt, off);
+    if ((lane & (2 * off - 1)) == 0 && ocnt) {
+      sw = add_rn(sw, osw);
+      swx = add_rn(swx, oswx);
+      cnt += ocnt;
+    }
+  }
+  return cnt;
+}
+
 // One warp per hub row (degree > hub_thr): lane l folds edges l, l + 32,
 // l + 64, ... in order (coalesced loads), the 32 lane sums are combined in a
 // fixed tree.
@@ -331,18 +355,7 @@ __device__ __forceinline__ void hub_warp(const OpinionArgs &p, uint32_t r) {
   }
   uint64_t sw = bits(dsw);
   uint64_t swx = bits(dswx);
-  // fixed tree: lane l receives lane l + off
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    uint64_t osw = __shfl_down_sync(0xffffffffu, sw, off);
-    uint64_t oswx = __shfl_down_sync(0xffffffffu, swx, off);
-    uint32_t ocnt = __shfl_down_sync(0xffffffffu, cnt, off);
-    if ((lane & (2 * off - 1)) == 0 && ocnt) {
-      sw = add_rn(sw, osw);
-      swx = add_rn(swx, oswx);
-      cnt += ocnt;
-    }
-  }
+  cnt = hub_tree(sw, swx, cnt);
   if (lane == 0) p.xo[r] = cnt ? finish(p, xi, sw, swx) : xi;
 }
 
@@ -558,7 +571,8 @@ __device__ __noinline__ void hub_block(const OpinionArgs &p, uint32_t r) {
 // are run by their own launch (k_opinion_big) and the range starts at the
 // warp hubs, so that this kernel needs no shared memory (its L1 keeps the
 // whole unified array).
-template <bool GRID, bool BIG>
+// LONG: the long slices run in k_opinion_long's blocks.
+template <bool GRID, bool BIG, bool LONG>
 __device__ __forceinline__ void opinion_block(const OpinionArgs &p, unsigned blk) {
   if (BIG) {
     if (blk < p.nbig) {  // block-wide hub rows (whole blocks: the test is uniform)
@@ -569,22 +583,146 @@ __device__ __forceinline__ void opinion_block(const OpinionArgs &p, unsigned blk
   }
   const uint64_t warp = (uint64_t)blk * (TPB / 32) + (threadIdx.x >> 5);
   if (blk < p.hub_blocks) {
-    if (p.nbig + warp < p.nhub) hub_warp<GRID>(p, p.hub_rows[p.nbig + warp]);
+    const uint64_t h = p.nbig + (LONG ? p.long_hubs : 0) + warp;
+    if (h < p.nhub) hub_warp<GRID>(p, p.hub_rows[h]);
     return;
   }
   const uint64_t sl = warp - (uint64_t)p.hub_blocks * (TPB / 32);
-  if (sl < p.nslices) sell_slice<GRID>(p, sl);
+  if (sl < p.nslices && !(LONG && p.slice_deg[sl] >= p.long_slots)) sell_slice<GRID>(p, sl);
 }
 
+// One block per long slice, or per hub row.  A warp that folds a slice by
+// itself (sell_slice) has two groups of two slots in flight, so a slot costs
+// it 340 ns of memory latency whatever the graph's size: rows of 1000
+// in-edges set the step of every graph below a few million agents.  Here
+// LONG_WARPS warps gather, test and multiply the slots (4 per warp and
+// round, the sources and weights of the next round and the opinions of this
+// one in flight) and leave the terms in shared memory, -0.0 for a rejected
+// edge or a padding slot (x + -0.0 is x); two more warps add them up, one the
+// weights, one the products, each row's terms in insertion order -- the same
+// additions as sell_slice, bit for bit.  The sums go to two warps because a
+// scheduler takes 36 ns per binary64 warp addition.  A hub row is 32 such
+// rows: lane l adds the edges l, l + 32, ... and the lanes' sums are combined
+// in hub_warp's tree.
+// Bound: the chain of the longest slice or hub row, 36 ns per slot.
+// Measured, us per step before -> now, mean degree 20: N = 3000 335 -> 70,
+// 3*10^4 366 -> 80, 10^6 479 -> 123, 3*10^6 643 -> 301,
+// 5*10^6 703 -> 479.
+constexpr int LONG_WARPS = 8;
+constexpr int LONG_U = 4;                          // slots per warp and round
+constexpr int LONG_ROUND = LONG_WARPS * LONG_U;    // 32 slots
+constexpr int LONG_TPB = (LONG_WARPS + 2) * 32;
+
+struct LongShared {
+  double w[2][LONG_ROUND][32], p[2][LONG_ROUND][32];
+  double swx[32];
+  uint32_t cnt[32];
+};
+
+// what: a slice, or with HUB a row
+template <bool GRID, bool HUB>
+__device__ __forceinline__ void long_fold(const OpinionArgs &p, uint32_t what, LongShared &S) {
+  const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t *cs = p.src;
+  const double *cw = p.w;
+  uint32_t r = what, d, D;  // the lane's row, its terms, the block's slots
+  bool live = true;
+  if (HUB) {
+    const uint32_t b = p.rp[r], deg = p.rp[r + 1] - b;
+    cs += b + lane;
+    cw += b + lane;
+    D = (deg + 31) / 32;
+    d = (deg + 31 - lane) / 32;
+  } else {
+    const uint64_t pos = (uint64_t)what * 32 + lane;
+    live = pos < p.norder;
+    r = live ? p.order[pos] : 0u;
+    d = live ? p.order_deg[pos] : 0u;
+    D = p.slice_deg[what];
+    cs = p.sell_src + p.slice_base[what] + lane;
+    cw = p.sell_w + p.slice_base[what] + lane;
+  }
+  const double xi = live ? p.x[r] : 0.0;
+  const uint32_t rounds = (D + LONG_ROUND - 1) / LONG_ROUND;
+  if (threadIdx.x < 32) S.cnt[lane] = 0;
+  __syncthreads();
+  double acc = 0.0;
+  if (wid < LONG_WARPS) {
+    bool xi_ok;
+    const float fxi = hi_float(xi, xi_ok);
+    const uint64_t pol = policy_evict_first(), pol_keep = policy_evict_last();
+    uint32_t j[LONG_U], cnt = 0;
+    double wn[LONG_U];
+    auto load = [&](uint32_t k) {  // the warp's slots of round k
+#pragma unroll
+      for (int u = 0; u < LONG_U; u++) {
+        const uint32_t q = k * LONG_ROUND + wid * LONG_U + u;
+        j[u] = q < d ? ld_stream(cs + 32ull * q, pol) : 0u;
+        wn[u] = q < d ? ld_stream(cw + 32ull * q, pol) : 0.0;
+      }
+    };
+    load(0);
+    for (uint32_t k = 0; k <= rounds; k++) {
+      if (k < rounds) {
+        double x[LONG_U], w[LONG_U];
+#pragma unroll
+        for (int u = 0; u < LONG_U; u++) {
+          x[u] = ld_keep(p.x + j[u], pol_keep);  // (a padding slot's source is 0)
+          w[u] = wn[u];
+        }
+        load(k + 1);
+#pragma unroll
+        for (int u = 0; u < LONG_U; u++) {
+          const uint32_t q = k * LONG_ROUND + wid * LONG_U + u;
+          const bool in = q < d && within(x[u], xi, fxi, xi_ok, p);
+          bool ok;
+          const uint64_t pk = GRID ? emu_mul_grid(bits(w[u]), bits(x[u]), ok)
+                                   : emu_mul_fast(bits(w[u]), bits(x[u]), ok);
+          const double pkd = ok ? dbl(pk) : (in ? mul_hw(w[u], x[u]) : 0.0);
+          S.w[k & 1][wid * LONG_U + u][lane] = in ? w[u] : -0.0;
+          S.p[k & 1][wid * LONG_U + u][lane] = in ? pkd : -0.0;
+          cnt += in;
+        }
+      }
+      __syncthreads();
+    }
+    if ((HUB || !GRID) && cnt) atomicAdd(&S.cnt[lane], cnt);
+  } else {
+    const bool sums_w = wid == LONG_WARPS;
+    for (uint32_t k = 0; k <= rounds; k++) {
+      if (k) {
+        const double(*t)[32] = sums_w ? S.w[(k - 1) & 1] : S.p[(k - 1) & 1];
+#pragma unroll
+        for (int u = 0; u < LONG_ROUND; u++) acc = __dadd_rn(acc, t[u][lane]);
+      }
+      __syncthreads();
+    }
+    if (!sums_w) S.swx[lane] = acc;
+  }
+  __syncthreads();
+  if (wid != LONG_WARPS) return;
+  uint64_t sw = bits(acc), swx = bits(S.swx[lane]);
+  if (HUB) {
+    const uint32_t cnt = hub_tree(sw, swx, S.cnt[lane]);
+    if (lane == 0) p.xo[r] = cnt ? finish(p, xi, sw, swx) : xi;
+    return;
+  }
+  if (!live) return;
+  const bool any = GRID ? sw != 0 : S.cnt[lane] != 0;
+  p.xo[r] = any ? finish(p, xi, sw, swx) : xi;
+}
+
+// block blk of the long launch: hub rows, then slices
 template <bool GRID>
-__global__ void __launch_bounds__(TPB, 9) k_opinion(OpinionArgs p) {
-  opinion_block<GRID, false>(p, blockIdx.x);
+__device__ __forceinline__ void long_block(const OpinionArgs &p, unsigned blk, LongShared &S) {
+  if (blk < p.long_hubs) long_fold<GRID, true>(p, p.hub_rows[p.nbig + blk], S);
+  else long_fold<GRID, false>(p, p.long_slices[blk - p.long_hubs], S);
 }
 
 // Completion reports of one gather launch (apply! with host exchange): the
-// launch is k_opinion's (the same blocks, the same work); the hub warps'
-// blocks form range `nranges`, slice blocks below end[k] (and not below
-// end[k - 1]) range k.  A block reports once its rows are stored: after the
+// launches are k_opinion_long's and k_opinion's (the same blocks, the same
+// work); the long slices' and the hub warps' blocks form range `nranges`,
+// slice blocks below end[k] (and not below end[k - 1]) range k.  A block reports once its rows are stored: after the
 // block barrier its first thread fences (GPU scope, cumulative over the
 // block's stores) and adds 1 to its range's counter; the block that
 // completes a range makes the range visible system-wide and writes the
@@ -598,23 +736,58 @@ struct Notify {
   unsigned expect[XCHG_RANGES + 1];  // blocks per range
 };
 
-template <bool GRID>
+// by one thread, after its block's barrier
+__device__ __forceinline__ void report_range(const Notify &nt, unsigned r) {
+  __threadfence();
+  if (atomicAdd(nt.count + r, 1u) + 1 == nt.expect[r]) {
+    __threadfence_system();
+    *(volatile unsigned *)(nt.flag + r) = nt.gen;
+  }
+}
+
+// The long slices' launch goes first, the rest follows as its programmatic
+// dependent: its blocks start as soon as every long block runs, so the long
+// chains overlap everything else.  The two read the old opinions and write
+// disjoint rows; the second ends only after the first (its last block waits
+// for it), so whatever follows in the stream sees both.
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void end_after_previous() {
+  if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <bool GRID, bool REPORT>
+__global__ void __launch_bounds__(LONG_TPB) k_opinion_long(OpinionArgs p, Notify nt) {
+  __shared__ LongShared S;
+  let_next_start();
+  long_block<GRID>(p, blockIdx.x, S);
+  if (REPORT) {
+    __syncthreads();
+    if (threadIdx.x == 0) report_range(nt, nt.nranges);
+  }
+}
+
+template <bool GRID, bool LONG>
+__global__ void __launch_bounds__(TPB, 9) k_opinion(OpinionArgs p) {
+  opinion_block<GRID, false, LONG>(p, blockIdx.x);
+  if (LONG) end_after_previous();
+}
+
+template <bool GRID, bool LONG>
 __global__ void __launch_bounds__(TPB, 9) k_opinion_notify(OpinionArgs p, Notify nt) {
-  opinion_block<GRID, false>(p, blockIdx.x);
+  opinion_block<GRID, false, LONG>(p, blockIdx.x);
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
     const unsigned b = blockIdx.x;
     unsigned r = nt.nranges;  // the hub warps
     if (b >= nt.hub_blocks) {
       r = 0;
       while (r + 1 < nt.nranges && b >= nt.end[r]) r++;
     }
-    if (atomicAdd(nt.count + r, 1u) + 1 == nt.expect[r]) {
-      __threadfence_system();
-      *(volatile unsigned *)(nt.flag + r) = nt.gen;
-    }
+    report_range(nt, r);
   }
+  if (LONG) end_after_previous();
 }
 
 // the block-wide hub rows of one simulation, one block each
@@ -638,8 +811,23 @@ __global__ void __launch_bounds__(TPB, 9) k_opinion_jobs(const OpinionArgs *jobs
   JobTile t = tiles[blockIdx.x];
   if (threadIdx.x == 0) sp = jobs[t.job];
   __syncthreads();
-  if (sp.grid) opinion_block<true, false>(sp, t.blk);
-  else opinion_block<false, false>(sp, t.blk);
+  if (sp.grid) opinion_block<true, false, true>(sp, t.blk);
+  else opinion_block<false, false, true>(sp, t.blk);
+  end_after_previous();
+}
+
+// their long slices and hub rows: block i is long block tiles[i].blk of job
+// tiles[i].job
+__global__ void __launch_bounds__(LONG_TPB) k_opinion_jobs_long(const OpinionArgs *jobs,
+                                                                const JobTile *tiles) {
+  __shared__ OpinionArgs sp;
+  __shared__ LongShared S;
+  let_next_start();
+  const JobTile t = tiles[blockIdx.x];
+  if (threadIdx.x == 0) sp = jobs[t.job];
+  __syncthreads();
+  if (sp.grid) long_block<true>(sp, t.blk, S);
+  else long_block<false>(sp, t.blk, S);
 }
 
 
@@ -663,6 +851,37 @@ __global__ void k_check_grid(const double *w, uint64_t n, int *bad) {
 static unsigned opinion_args(Sim &s, int e, int T, double eps, double a, double b,
                              uint32_t thr, uint32_t big_thr, OpinionArgs &p,
                              cudaStream_t launch_stream);
+
+// which slices and hub rows take a block each, in a launch over `edges`
+// edges; returns the grid of the other blocks
+static unsigned split_long(OpinionArgs &p, uint64_t edges) {
+  auto at_least = [](const std::vector<uint32_t> &v, uint32_t t) {  // v descending
+    return (unsigned)(std::upper_bound(v.begin(), v.end(), t,
+                                       [](uint32_t a, uint32_t b) { return b < a; }) -
+                      v.begin());
+  };
+  p.long_slots = opinion_long_slots(edges);
+  p.nlong = at_least(p.csr->long_slots, p.long_slots);
+  const uint64_t hubs = at_least(p.csr->long_hubs, 32 * p.long_slots);
+  p.long_hubs = hubs > p.nbig ? (unsigned)(hubs - p.nbig) : 0;
+  p.hub_blocks = (unsigned)((p.nhub - p.nbig - p.long_hubs + (TPB / 32) - 1) / (TPB / 32));
+  return (unsigned)p.nbig + p.hub_blocks + (unsigned)((p.nslices + (TPB / 32) - 1) / (TPB / 32));
+}
+
+// a launch that may start before the preceding one of the stream has ended
+template <class... A, class... B>
+static void launch_dependent(void (*k)(A...), unsigned grid, cudaStream_t st, B... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(TPB);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  VG_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
+}
 // a gather launch whose finished row ranges are downloaded while it runs
 // (apply! with host exchange)
 static void launch_notified(Sim &s, OpinionArgs &p, unsigned grid, Sim::HostExchange &hx);
@@ -697,8 +916,8 @@ void tr_bounded_confidence(ApplyCtx &c) {
   double big_d = c.param(5, 4294967295.0);
   uint32_t big_thr = big_d >= 4294967295.0 ? 0xffffffffu : (uint32_t)big_d;
   OpinionArgs p{};
-  unsigned grid = opinion_args(s, e, c.call_type, eps, a, b, thr, big_thr, p, s.stream);
-  if (!grid) return;
+  if (!opinion_args(s, e, c.call_type, eps, a, b, thr, big_thr, p, s.stream)) return;
+  const unsigned grid = split_long(p, p.csr->nedges);
   // block-wide hubs (only with a block threshold) by their own launch, then
   // the rest: the two write disjoint rows and read only the old opinions
   const unsigned nbig = (unsigned)p.nbig;
@@ -712,9 +931,16 @@ void tr_bounded_confidence(ApplyCtx &c) {
     launch_notified(s, p, grid, *hx);
     return;
   }
-  if (grid > nbig) {
-    if (p.grid) k_opinion<true><<<grid - nbig, TPB, 0, s.stream>>>(p);
-    else k_opinion<false><<<grid - nbig, TPB, 0, s.stream>>>(p);
+  const unsigned nl = p.long_hubs + p.nlong;
+  if (nl) {
+    if (p.grid) k_opinion_long<true, false><<<nl, LONG_TPB, 0, s.stream>>>(p, Notify{});
+    else k_opinion_long<false, false><<<nl, LONG_TPB, 0, s.stream>>>(p, Notify{});
+    VG_CUDA(cudaGetLastError());
+    launch_dependent(p.grid ? k_opinion<true, true> : k_opinion<false, true>, grid - nbig, s.stream,
+                     p);
+  } else if (grid > nbig) {
+    if (p.grid) k_opinion<true, false><<<grid - nbig, TPB, 0, s.stream>>>(p);
+    else k_opinion<false, false><<<grid - nbig, TPB, 0, s.stream>>>(p);
   }
   VG_CUDA(cudaGetLastError());
 }
@@ -789,10 +1015,19 @@ static void launch_notified(Sim &s, OpinionArgs &p, unsigned grid, Sim::HostExch
     nt.end[k] = (unsigned)cs.range_block[k + 1];
     nt.expect[k] = (unsigned)(cs.range_block[k + 1] - cs.range_block[k]);
   }
-  nt.expect[K] = p.hub_blocks;
+  const unsigned nl = p.long_hubs + p.nlong;
+  nt.expect[K] = p.hub_blocks + nl;
   VG_CUDA(cudaMemsetAsync(nt.count, 0, (K + 1) * 4, s.stream));
-  if (p.grid) k_opinion_notify<true><<<grid, TPB, 0, s.stream>>>(p, nt);
-  else k_opinion_notify<false><<<grid, TPB, 0, s.stream>>>(p, nt);
+  if (nl) {
+    if (p.grid) k_opinion_long<true, true><<<nl, LONG_TPB, 0, s.stream>>>(p, nt);
+    else k_opinion_long<false, true><<<nl, LONG_TPB, 0, s.stream>>>(p, nt);
+    VG_CUDA(cudaGetLastError());
+    launch_dependent(p.grid ? k_opinion_notify<true, true> : k_opinion_notify<false, true>, grid,
+                     s.stream, p, nt);
+  } else {
+    if (p.grid) k_opinion_notify<true, false><<<grid, TPB, 0, s.stream>>>(p, nt);
+    else k_opinion_notify<false, false><<<grid, TPB, 0, s.stream>>>(p, nt);
+  }
   VG_CUDA(cudaGetLastError());
 
   const uint64_t n = std::min<uint64_t>(hx.n, p.n);
@@ -810,7 +1045,9 @@ static void launch_notified(Sim &s, OpinionArgs &p, unsigned grid, Sim::HostExch
     hi[k] = std::max(prev, k + 1 == K ? n : std::min(n, cs.range_rows[k]));
     auto it = std::lower_bound(cs.hub_rows_sorted.begin(), cs.hub_rows_sorted.end(),
                                (uint32_t)lo[k]);
-    needs_hubs[k] = p.hub_blocks && it != cs.hub_rows_sorted.end() && *it < hi[k];
+    // (every window may hold long slices)
+    needs_hubs[k] = p.nlong || ((p.hub_blocks || p.long_hubs) &&
+                                it != cs.hub_rows_sorted.end() && *it < hi[k]);
     unsigned j = 0;
     while (j < k && (j + 1 < K ? cs.range_window[j + 1] : 0xFFFFFFFFu) < cs.range_window[k]) j++;
     first[k] = j;
@@ -825,7 +1062,7 @@ static void launch_notified(Sim &s, OpinionArgs &p, unsigned grid, Sim::HostExch
   };
   unsigned left = K;
   for (uint64_t poll = 0; left; poll++) {
-    const bool hubs_done = p.hub_blocks == 0 || flag[K] == nt.gen;
+    const bool hubs_done = nt.expect[K] == 0 || flag[K] == nt.gen;
     for (unsigned k = 0; k < K; k++) {
       if (issued[k] || (needs_hubs[k] && !hubs_done)) continue;
       bool ready = true;
@@ -910,6 +1147,7 @@ static unsigned opinion_args(Sim &s, int e, int T, double eps, double a, double 
   p.sell_src = cs.sell_src.as<uint32_t>();
   p.sell_w = cs.sell_w.as<double>();
   p.nslices = cs.nslices;
+  p.long_slices = cs.long_slices.as<uint32_t>();
   p.hub_blocks = (unsigned)((cs.nhub - cs.nbig + (TPB / 32) - 1) / (TPB / 32));
   p.csr = &cs;
   return (unsigned)cs.nbig + p.hub_blocks + (unsigned)((cs.nslices + (TPB / 32) - 1) / (TPB / 32));
@@ -932,17 +1170,24 @@ void prepare_opinion_job(const OpinionJob &j) {
 void launch_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_t st, DevBuf &args_buf,
                          DevBuf &tiles_buf, uint64_t *fp) {
   std::vector<OpinionArgs> args;
-  std::vector<JobTile> tiles;
+  std::vector<JobTile> tiles, longs;
+  uint64_t edges = 0;  // of all jobs: they share the launch
+  for (auto &j : jobs) edges += csr_view(*j.sim, j.edge_type, j.type_nr).nedges;
   for (size_t j = 0; j < jobs.size(); j++) {
     OpinionArgs p{};
     unsigned g = opinion_args(*jobs[j].sim, jobs[j].edge_type, jobs[j].type_nr, jobs[j].eps,
                               jobs[j].a, jobs[j].b, jobs[j].hub_thr, jobs[j].block_thr, p, st);
     if (p.nbig)
       fail(VG_ERR_ARG, "the multi-job gather runs no block-wide hub rows (block threshold)");
+    if (g) g = split_long(p, edges);
     args.push_back(p);
     for (unsigned k = 0; k < g; k++) tiles.push_back({(uint32_t)j, k});
+    for (unsigned k = 0; k < p.long_hubs + p.nlong; k++) longs.push_back({(uint32_t)j, k});
   }
   if (tiles.empty()) return;
+  // (one buffer: the long slices' tiles behind the others)
+  const size_t ntiles = tiles.size();
+  for (const JobTile &t : longs) tiles.push_back(t);
   if (args_buf.bytes < args.size() * sizeof(OpinionArgs))
     args_buf.alloc(args.size() * sizeof(OpinionArgs) * 2, fp);
   if (tiles_buf.bytes < tiles.size() * sizeof(JobTile))
@@ -951,8 +1196,15 @@ void launch_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_t st, D
                           cudaMemcpyHostToDevice, st));
   VG_CUDA(cudaMemcpyAsync(tiles_buf.p, tiles.data(), tiles.size() * sizeof(JobTile),
                           cudaMemcpyHostToDevice, st));
-  k_opinion_jobs<<<(unsigned)tiles.size(), TPB, 0, st>>>(args_buf.as<OpinionArgs>(),
-                                                        tiles_buf.as<JobTile>());
+  const OpinionArgs *da = args_buf.as<OpinionArgs>();
+  const JobTile *dt = tiles_buf.as<JobTile>();
+  if (!longs.empty()) {
+    k_opinion_jobs_long<<<(unsigned)longs.size(), LONG_TPB, 0, st>>>(da, dt + ntiles);
+    VG_CUDA(cudaGetLastError());
+  }
+  // (with no long block before it, its dependency is the copies above)
+  if (longs.empty()) k_opinion_jobs<<<(unsigned)ntiles, TPB, 0, st>>>(da, dt);
+  else launch_dependent(k_opinion_jobs, (unsigned)ntiles, st, da, dt);
   VG_CUDA(cudaGetLastError());
   // no wait: a copy from pageable host memory is staged before the call
   // returns, so the host vectors may go; the device buffers are rewritten by
