@@ -9,7 +9,9 @@
 // left-to-right order, so results are bit-identical to the sequential CPU
 // fold (the library is also compiled with -fmad=false).
 #include <algorithm>
+#include <array>
 #include <cstring>
+#include <map>
 #include <vector>
 
 #include "vg_internal.h"
@@ -696,6 +698,8 @@ __global__ void __launch_bounds__(256) k_life2d_x4(const uint32_t *__restrict__ 
   }
 }
 
+// Moore neighbourhood, one cell per thread: smaller rasters, and UInt8 cells,
+// whose values are summed as they are.
 __global__ void k_life2d(const uint8_t *__restrict__ a, uint8_t *__restrict__ o,
                          int64_t W, int64_t H, int periodic) {
   int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -722,6 +726,261 @@ __global__ void k_life2d(const uint8_t *__restrict__ a, uint8_t *__restrict__ o,
   }
   uint8_t alive = a[y * W + x];
   o[y * W + x] = (cnt == 3 || (alive && cnt == 2)) ? 1 : 0;
+}
+
+// Implicit stencils of any metric on Bool cells, distance up to ROW_D_MAX,
+// 1 to 4 dimensions of any size.  A stencil of the reference's metrics is a
+// set of rows along the first dimension, each an interval of cells [-r, r]
+// around the centre (the centre's own row without the centre): the count is
+// the sum of the rows' window sums minus the cell.  Four cells are the bytes
+// of a 32-bit word (Bool cells are 0 or 1, and at most 128 offsets fit a
+// byte); a window sum grows by two byte-shifted words per step of r.  A
+// block of 32 x 8 threads takes a tile of 128 cells x 32 rows of one plane
+// (third and fourth coordinate); for every plane the stencil touches it
+// stages the tile and its halo in shared memory, wrapping or zeroing outside
+// positions there, and each thread adds the rows to the four rows of its
+// word column.
+// Rows of any length: global words are read aligned and shifted into place,
+// and results leave as aligned words put together from two lanes (lane 0
+// computes the word before the tile for that), byte by byte only at a row's
+// ends.
+// Bound: instruction issue, about 50 per cell word of a thread's four and the
+// set-up and loads of a tile (ncu: 2.5 instructions per cycle on the busy
+// SMs, 55 % of the launch busy).  The kernel before took one cell per thread
+// with a 64-bit division and modulo per dimension and a byte load per
+// offset.  Measured, us per launch, 2047 x 1531 bounded, euclidean distance
+// 2: 100 before, 9.3 now (2, 4, 8 rows per thread: 9.4, 9.3, 11.5).
+constexpr int ROW_D_MAX = 4;
+constexpr int ROW_RY = 4, ROW_TY = 8 * ROW_RY;
+constexpr int ROW_TX = 124;      // cells of a tile: lanes 1 .. 31, lane 0 the word before
+constexpr int ROW_WORDS = 34;    // the lanes' words and one on each side
+constexpr int ROW_PLANES = 128;
+
+struct RowStencil {
+  int64_t dims[MAX_DIMS];  // 1 beyond the raster's dimensions
+  uint32_t tx, ty;         // tiles along the first two
+  int nplanes, periodic;
+  uint32_t birth, survive;
+  int noff;
+  // the rules as bytes for counts 0 .. 31: entry 8 g + k in byte k of the
+  // 64-bit word g (two registers of a byte permutation)
+  uint32_t birth_tab[8], survive_tab[8];
+  // the planes: offset in the third and fourth dimension, the window radii by
+  // dy + D (-1: no row) and the same as row_code (-1: not expressible).  What
+  // a launch over one plane reads fits the first lines of the constant bank:
+  // each line is a miss of its own at every launch.
+  struct Plane {
+    int8_t z, v;
+    int16_t code;
+    int8_t rad[2 * ROW_D_MAX + 1];
+  } plane[ROW_PLANES];
+};
+
+// radii of the rows dy = 0, +-1, +-2 (-1: no row) of a plane within that
+// reach, symmetric in dy
+__host__ __device__ constexpr int row_code(int r0, int r1, int r2) {
+  return (r0 + 1) | (r1 + 1) << 4 | (r2 + 1) << 8;
+}
+
+// adds the plane's rows to the thread's ROW_RY words; CODE -1: radii from rad
+template <int D, int CODE>
+__device__ __forceinline__ void row_sums(const uint32_t *rows, const int8_t *rad,
+                                         uint32_t (&acc)[ROW_RY]) {
+  int r[2 * D + 1];
+#pragma unroll
+  for (int dy = -D; dy <= D; dy++) {
+    const int ady = dy < 0 ? -dy : dy;
+    r[dy + D] = CODE < 0 ? rad[dy + D] : ady > 2 ? -1 : ((CODE >> (4 * ady)) & 15) - 1;
+  }
+#pragma unroll
+  for (int i = 0; i < ROW_RY + 2 * D; i++) {
+    const uint32_t l = rows[i * ROW_WORDS], c = rows[i * ROW_WORDS + 1],
+                   n = rows[i * ROW_WORDS + 2];
+    uint32_t h[D + 1];
+    h[0] = c;
+#pragma unroll
+    for (int k = 1; k <= D; k++)
+      h[k] = h[k - 1] + (k < 4 ? __funnelshift_l(l, c, 8 * k) : l) +
+             (k < 4 ? __funnelshift_r(c, n, 8 * k) : n);
+#pragma unroll
+    for (int j = 0; j < ROW_RY; j++) {
+      const int dy = i - j;  // dy + D
+      if (dy < 0 || dy > 2 * D) continue;
+#pragma unroll
+      for (int k = 0; k <= D; k++)
+        if (r[dy] == k) acc[j] += h[k];
+    }
+  }
+}
+
+// the next state of a word's four cells: byte permutations look the four
+// counts up in the rule's table, eight entries at a time
+__device__ __forceinline__ uint32_t row_rule(const RowStencil &s, uint32_t self, uint32_t cnt) {
+  if (s.noff > 31) {
+    uint32_t w = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const uint32_t rule = self & (1u << (8 * c)) ? s.survive : s.birth;
+      w |= ((rule >> min((cnt >> (8 * c)) & 0xffu, 31u)) & 1u) << (8 * c);
+    }
+    return w;
+  }
+  const uint32_t k = cnt & 0x07070707u, pairs = k | (k >> 4);
+  const uint32_t sel = __byte_perm(pairs, 0, 0x4420);  // the four counts' low bits as selectors
+  const uint32_t alive = self * 0xffu;
+  auto look = [&](int g) {
+    const uint32_t b = __byte_perm(s.birth_tab[2 * g], s.birth_tab[2 * g + 1], sel);
+    const uint32_t v = __byte_perm(s.survive_tab[2 * g], s.survive_tab[2 * g + 1], sel);
+    return (v & alive) | (b & ~alive);
+  };
+  uint32_t w = look(0);
+  if (s.noff > 7) {
+    const uint32_t b3 = ((cnt >> 3) & 0x01010101u) * 0xffu;
+    w = (w & ~b3) | (look(1) & b3);
+    if (s.noff > 15) {
+      const uint32_t b4 = ((cnt >> 4) & 0x01010101u) * 0xffu;
+      w = (w & ~b4) | (((look(2) & ~b3) | (look(3) & b3)) & b4);
+    }
+  }
+  return w;
+}
+
+// CODE: the row code of a stencil of one plane (rasters of up to two
+// dimensions), -1: any planes
+template <int D, int CODE>
+__global__ void __launch_bounds__(256, 4) k_life_rows(const uint8_t *__restrict__ a,
+                                                   uint8_t *__restrict__ o,
+                                                   const __grid_constant__ RowStencil s) {
+  constexpr int ROWS = ROW_TY + 2 * D, LOADS = (ROWS + 7) / 8;
+  __shared__ uint32_t t[ROWS * ROW_WORDS];
+  const int lane = threadIdx.x;
+  const int W = (int)s.dims[0], H = (int)s.dims[1], Z = (int)s.dims[2], V = (int)s.dims[3];
+  uint32_t blk = blockIdx.x;
+  const int x0 = (int)(blk % s.tx) * ROW_TX;
+  blk /= s.tx;
+  const int y0 = (int)(blk % s.ty) * ROW_TY;
+  blk /= s.ty;
+  const int z = (int)(blk % (uint32_t)Z), v = (int)(blk / (uint32_t)Z);
+  uint32_t acc[ROW_RY], self[ROW_RY];
+#pragma unroll
+  for (int j = 0; j < ROW_RY; j++) acc[j] = self[j] = 0;
+  const int nplanes = CODE >= 0 ? 1 : s.nplanes;
+  for (int p = 0; p < nplanes; p++) {
+    int pz = z + (CODE >= 0 ? 0 : s.plane[p].z), pv = v + (CODE >= 0 ? 0 : s.plane[p].v);
+    if (pz < 0 || pz >= Z || pv < 0 || pv >= V) {
+      if (!s.periodic) continue;  // (block-uniform)
+      pz += pz < 0 ? Z : pz >= Z ? -Z : 0;
+      pv += pv < 0 ? V : pv >= V ? -V : 0;
+    }
+    const uint8_t *base = a + (uint64_t)(pv * (int64_t)Z + pz) * ((uint64_t)H * W);
+    if (p) __syncthreads();  // the previous plane is read
+    // Warp y loads the rows y, y + 8, ..: lane l the word l, lanes 0 and 1
+    // also the last two; every load is issued before the first is used.
+    // Words not whole inside their row (and the array's last, whose second
+    // aligned word would lie behind it) are left 0 here.
+    const uint8_t *end = a + (uint64_t)V * Z * H * W;
+    const bool xin = x0 >= 8 && x0 + ROW_TX + 8 <= W;  // (block-uniform) no such word
+    uint32_t w0[LOADS][2], w1[LOADS][2], sh[LOADS];
+#pragma unroll
+    for (int u = 0; u < LOADS; u++) {
+      const int r = u * 8 + (int)threadIdx.y;  // warp-uniform
+      int y = y0 - D + r;
+      const bool use = r < ROWS && ((y >= 0 && y < H) || (s.periodic && y < H + D));
+      y += y < 0 ? H : y >= H ? -H : 0;
+      const uint8_t *row = base + (uint64_t)(use ? y : 0) * W;
+      sh[u] = 8 * ((uint32_t)(uint64_t)(row + x0) & 3u);
+      const int x = x0 - 8 + 4 * lane;
+      const uint32_t *q = (const uint32_t *)((uint64_t)(row + x) & ~3ull);
+      const bool in = use && (xin || (x >= 0 && x + 4 <= W && row + x + 8 <= end));
+      w0[u][0] = in ? q[0] : 0u;
+      w1[u][0] = in ? q[1] : 0u;
+      const bool in2 = use && lane < 2 &&
+                       (xin || (x + 128 >= 0 && x + 132 <= W && row + x + 136 <= end));
+      w0[u][1] = in2 ? q[32] : 0u;
+      w1[u][1] = in2 ? q[33] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < LOADS; u++) {
+      const int r = u * 8 + (int)threadIdx.y;
+      if (r >= ROWS) continue;
+      t[r * ROW_WORDS + lane] = __funnelshift_r(w0[u][0], w1[u][0], sh[u]);
+      if (lane < 2) t[r * ROW_WORDS + lane + 32] = __funnelshift_r(w0[u][1], w1[u][1], sh[u]);
+    }
+    if (!xin) {
+      // the words at the row's ends byte by byte, wrapped or zero outside:
+      // the first two of the tile and those around cell W
+      __syncthreads();
+      const int jr = (W - (x0 - 8)) / 4;
+      for (int i = threadIdx.y * 32 + lane; i < ROWS * 8; i += 256) {
+        const int r = i / 8, k = i % 8, j = k < 2 ? k : jr + k - 4;
+        const int x = x0 - 8 + 4 * j;
+        int y = y0 - D + r;
+        if (j >= ROW_WORDS || (k >= 2 && j < 2) || !((y >= 0 && y < H) || (s.periodic && y < H + D)))
+          continue;
+        y += y < 0 ? H : y >= H ? -H : 0;
+        const uint8_t *row = base + (uint64_t)y * W;
+        if (x >= 0 && x + 4 <= W && row + x + 8 <= end) continue;
+        uint32_t w = 0;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          int xc = x + c;
+          const bool out = xc < 0 || xc >= W;
+          const bool use = !out || (s.periodic && xc >= -D && xc < W + D);
+          xc += xc < 0 ? W : out ? -W : 0;
+          w |= (use ? (uint32_t)row[xc] : 0u) << (8 * c);
+        }
+        t[r * ROW_WORDS + j] = w;
+      }
+    }
+    __syncthreads();
+    const uint32_t *rows = t + threadIdx.y * ROW_RY * ROW_WORDS + lane;
+    if (CODE >= 0) {
+      row_sums<D, CODE>(rows, nullptr, acc);
+    } else if (D <= 2) {
+      switch (s.plane[p].code) {  // (uniform) the planes of the metrics at distance 1 and 2
+        case row_code(1, 1, -1): row_sums<D, row_code(1, 1, -1)>(rows, nullptr, acc); break;
+        case row_code(1, 0, -1): row_sums<D, row_code(1, 0, -1)>(rows, nullptr, acc); break;
+        case row_code(0, -1, -1): row_sums<D, row_code(0, -1, -1)>(rows, nullptr, acc); break;
+        default: row_sums<D, -1>(rows, s.plane[p].rad, acc);
+      }
+    } else {
+      row_sums<D, -1>(rows, s.plane[p].rad, acc);
+    }
+    if (CODE >= 0 || (s.plane[p].z == 0 && s.plane[p].v == 0)) {
+#pragma unroll
+      for (int j = 0; j < ROW_RY; j++) self[j] = rows[(j + D) * ROW_WORDS + 1];
+    }
+  }
+  const bool border = x0 == 0 || x0 + ROW_TX >= W;  // (block-uniform)
+#pragma unroll
+  for (int j = 0; j < ROW_RY; j++) {
+    const int y = y0 + (int)threadIdx.y * ROW_RY + j;
+    if (y >= H) break;  // warp-uniform
+    const uint32_t w = row_rule(s, self[j], acc[j] - self[j]);  // (no byte is below its cell)
+    // Cells x0 - 4 + 4 lane ..: shifted by the row's misalignment m, every
+    // lane but 0 stores the aligned word of cells x0 - 4 + 4 lane - m ..;
+    // a row's tiles are shifted alike, so its words are stored once.  At the
+    // row's ends the words that are not all in the row go byte by byte.
+    const uint64_t row = ((uint64_t)(v * (int64_t)Z + z) * H + y) * W;
+    const int m = (int)(row + x0) & 3;
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, w, 1);
+    const uint32_t u = __funnelshift_l(prev, w, 8 * m);
+    const int x = x0 - 4 + 4 * lane - m;
+    if (!border) {
+      if (lane) *(uint32_t *)(o + row + x) = u;
+    } else {
+      // the last tile also stores the m cells its last word leaves over
+      const bool last = x0 + ROW_TX >= W;
+      if (lane && x >= 0 && x + 4 <= W) {
+        *(uint32_t *)(o + row + x) = u;
+      } else if (lane) {
+        for (int c = max(0, -x); c < 4 && x + c < W; c++) o[row + x + c] = (uint8_t)(u >> (8 * c));
+      }
+      if (last && lane == 31)
+        for (int c = 4 - m; c < 4 && x0 + 120 + c < W; c++)
+          o[row + x0 + 120 + c] = (uint8_t)(w >> (8 * c));
+    }
+  }
 }
 
 // general implicit stencil (any dims, offsets): count of alive sources
@@ -1163,6 +1422,86 @@ void tr_sir(ApplyCtx &c) {
   s.sir_epoch = s.csr_epoch;
 }
 
+// Where k_life_rows is the faster form.  Measured, us per step, rows and the
+// cell-per-thread kernels: Moore neighbourhood (k_life2d) 601 x 600 8.0 and
+// 7.8, 801 x 800 9.0 and 9.0, 1001 x 1000 9.0 and 11.1; 4 offsets
+// (k_life_stencil) 101 x 100 7.0 and 6.9, 401 x 400 7.0 and 7.0, 601 x 600
+// 7.1 and 10.8; 12 offsets 101 x 100 7.0 and 10.0; 26 offsets 11^3 9.5 and
+// 23.4.  Short rows leave a tile's lanes idle: 4 offsets 9 x 40000 17.2 and
+// 11.1, 17 x 40000 17.3 and 17.2, 33 x 40000 17.3 and 28.5; 12 offsets
+// 5 x 100000 36.9 and 33.0, 9 x 40000 19.2 and 25.5.
+bool rows_pay(const StencilDesc &st, uint64_t ncells, bool moore2d) {
+  if (moore2d) return ncells >= 640000 && st.dims[0] >= 9;
+  return st.noff * std::min<int64_t>(st.dims[0], ROW_TX) >= 72 &&
+         (st.noff >= 8 || ncells * st.noff >= 1000000);
+}
+
+// The stencil as rows for k_life_rows; false when it is none (an offset
+// beyond ROW_D_MAX, a dimension no larger than the reach, where a position
+// can wrap more than once, or a row that is no interval).
+bool row_stencil(const StencilDesc &st, int birth, int survive, RowStencil &rs, int &reach) {
+  reach = 0;
+  for (int v : st.offsets) reach = std::max(reach, std::abs(v));
+  if (reach < 1 || reach > ROW_D_MAX || st.noff > 128) return false;
+  for (int i = 0; i < MAX_DIMS; i++) {
+    rs.dims[i] = i < st.ndims ? st.dims[i] : 1;
+    if (i < st.ndims && (rs.dims[i] <= reach || rs.dims[i] >= 1 << 30)) return false;
+  }
+  // the cells of each (plane, dy) row as a bit set of dx
+  std::map<std::array<int, 3>, uint32_t> rows;  // (dv, dz, dy)
+  for (int k = 0; k < st.noff; k++) {
+    int q[MAX_DIMS] = {0, 0, 0, 0};  // a source lies at minus the offset
+    for (int i = 0; i < st.ndims; i++) q[i] = -st.offsets[k * st.ndims + i];
+    rows[{q[3], q[2], q[1]}] |= 1u << (q[0] + reach);
+  }
+  rs.nplanes = 0;
+  for (auto &r : rows) {
+    const bool centre = r.first == std::array<int, 3>{0, 0, 0};
+    const uint32_t bits = r.second | (centre ? 1u << reach : 0u);
+    if (centre && (r.second >> reach & 1u)) return false;
+    int rad = -1;
+    for (int k = 0; k <= reach; k++) {
+      uint32_t window = 0;
+      for (int x = -k; x <= k; x++) window |= 1u << (x + reach);
+      if (bits == window) rad = k;
+    }
+    if (rad < 0) return false;
+    int p = 0;
+    while (p < rs.nplanes && (rs.plane[p].z != r.first[1] || rs.plane[p].v != r.first[0])) p++;
+    if (p == rs.nplanes) {
+      if (p == ROW_PLANES) return false;
+      rs.nplanes++;
+      rs.plane[p].z = (int8_t)r.first[1];
+      rs.plane[p].v = (int8_t)r.first[0];
+      std::fill(rs.plane[p].rad, rs.plane[p].rad + 2 * ROW_D_MAX + 1, (int8_t)-1);
+    }
+    rs.plane[p].rad[r.first[2] + reach] = (int8_t)rad;
+  }
+  for (int p = 0; p < rs.nplanes; p++) {
+    const int8_t *r = rs.plane[p].rad + reach;
+    bool fits = true;
+    for (int dy = 0; dy <= reach; dy++) fits = fits && r[dy] == r[-dy] && (dy <= 2 || r[dy] < 0);
+    rs.plane[p].code = fits ? (int16_t)row_code(r[0], reach > 0 ? r[1] : -1, reach > 1 ? r[2] : -1) : -1;
+  }
+  if (!rows.count({0, 0, 0})) return false;  // (the kernel takes the cell out of its own row)
+  rs.periodic = st.periodic;
+  rs.birth = (uint32_t)birth & 0x7fffffffu;  // counts of 31 and more are no rule's
+  rs.survive = (uint32_t)survive & 0x7fffffffu;
+  rs.noff = st.noff;
+  for (int k = 0; k < 8; k++) {
+    rs.birth_tab[k] = rs.survive_tab[k] = 0;
+    for (int c = 0; c < 4; c++) {
+      rs.birth_tab[k] |= (rs.birth >> (4 * k + c) & 1u) << (8 * c);
+      rs.survive_tab[k] |= (rs.survive >> (4 * k + c) & 1u) << (8 * c);
+    }
+  }
+  const uint64_t tx = (rs.dims[0] + ROW_TX - 1) / ROW_TX, ty = (rs.dims[1] + ROW_TY - 1) / ROW_TY;
+  if (tx * ty * rs.dims[2] * rs.dims[3] >= 1ull << 31) return false;
+  rs.tx = (uint32_t)tx;
+  rs.ty = (uint32_t)ty;
+  return true;
+}
+
 void tr_life(ApplyCtx &c) {
   Sim &s = *c.sim;
   const AgentTypeDesc &ad = s.model->at(c.call_type);
@@ -1190,6 +1529,8 @@ void tr_life(ApplyCtx &c) {
       if (std::abs(ox) > 1 || std::abs(oy) > 1) moore2d = false;
     }
   }
+  RowStencil rs;
+  int reach = 0;
   if (moore2d && st.dims[0] % 4 == 0 && ((uintptr_t)in % 4) == 0 && ((uintptr_t)out % 4) == 0) {
     const int64_t Wq = st.dims[0] / 4;
     dim3 blk(32, 8);
@@ -1197,6 +1538,18 @@ void tr_life(ApplyCtx &c) {
              (unsigned)((st.dims[1] + 8 * LIFE_ROWS - 1) / (8 * LIFE_ROWS)));
     k_life2d_x4<<<grd, blk, 0, s.stream>>>((const uint32_t *)in, (uint32_t *)out, Wq, st.dims[1],
                                           st.periodic);
+  } else if (ad.fields[0].dtype == VG_BOOL && rows_pay(st, R.ncells, moore2d) &&
+             row_stencil(st, birth, survive, rs, reach)) {
+    const uint64_t blocks = (uint64_t)rs.tx * rs.ty * rs.dims[2] * rs.dims[3];
+    dim3 blk(32, 8);
+    const int code = rs.nplanes == 1 ? rs.plane[0].code : -1;
+    auto k = reach == 1 ? k_life_rows<1, -1> : reach == 2 ? k_life_rows<2, -1>
+             : reach == 3 ? k_life_rows<3, -1> : k_life_rows<4, -1>;
+    if (reach == 1 && code == row_code(1, 1, -1)) k = k_life_rows<1, row_code(1, 1, -1)>;
+    if (reach == 1 && code == row_code(1, 0, -1)) k = k_life_rows<1, row_code(1, 0, -1)>;
+    if (reach == 2 && code == row_code(2, 2, 2)) k = k_life_rows<2, row_code(2, 2, 2)>;
+    if (reach == 2 && code == row_code(2, 1, 0)) k = k_life_rows<2, row_code(2, 1, 0)>;
+    k<<<(unsigned)blocks, blk, 0, s.stream>>>(in, out, rs);
   } else if (moore2d) {
     dim3 blk(32, 8);
     dim3 grd((unsigned)((st.dims[0] + 31) / 32), (unsigned)((st.dims[1] + 7) / 8));
