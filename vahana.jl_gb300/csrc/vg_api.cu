@@ -397,6 +397,7 @@ int vg_sim_create(vg_model *m, const char *name, void *stream, vg_sim **out) {
 Sim::~Sim() {
   if (copy_stream) cudaStreamDestroy(copy_stream);
   if (xchg_flags_host) cudaFreeHost(xchg_flags_host);
+  if (reports_host) cudaFreeHost(reports_host);
 }
 
 int vg_sim_destroy(vg_sim *s) {
@@ -447,6 +448,7 @@ int vg_write_agents(vg_sim *h, int nr, const void *const *fields, uint64_t n) {
   if (s.intransition) fail(VG_ERR_ASSERT, "agent states cannot be set inside a transition");
   AgentStore &a = s.agents[nr - 1];
   if (n > a.n) fail(VG_ERR_ARG, "more values than agent slots");
+  forget_record_spread(s);
   for (size_t f = 0; f < ad.fields.size(); f++) {
     if (!fields || !fields[f]) continue;
     VG_CUDA(cudaMemcpyAsync(a.rd[f].p, fields[f], n * ad.fields[f].size, cudaMemcpyHostToDevice,

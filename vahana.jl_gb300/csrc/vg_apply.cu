@@ -37,11 +37,10 @@ EdgeAppend *ApplyCtx::append_for(int e, uint64_t capacity, bool ordered) {
   const EdgeTypeDesc &ed = s.model->et(e);
   auto it = s.append_spare.find(e);
   if (it != s.append_spare.end() && it->second->cap >= capacity &&
-      it->second->ordered == ordered) {
+      it->second->ordered == ordered && !it->second->typed) {
     std::unique_ptr<EdgeAppend> a = std::move(it->second);
     s.append_spare.erase(it);
     a->fixed_count = 0;
-    a->target_type = a->src_type = 0;
     VG_CUDA(cudaMemsetAsync(a->counter.p, 0, 8, s.stream));
     appends.push_back(std::move(a));
     return appends.back().get();
@@ -58,6 +57,59 @@ EdgeAppend *ApplyCtx::append_for(int e, uint64_t capacity, bool ordered) {
   for (int f = 0; f < nf; f++) a->payload[f].alloc(a->cap * ed.fields[f].size, &s.footprint);
   a->counter.alloc(8, &s.footprint);
   VG_CUDA(cudaMemsetAsync(a->counter.p, 0, 8, s.stream));
+  appends.push_back(std::move(a));
+  return appends.back().get();
+}
+
+bool ApplyCtx::typed_ok(int e, int T, int S, uint64_t slots) const {
+  Sim &s = *sim;
+  const EdgeTypeDesc &ed = s.model->et(e);
+  const EdgeStore &es = s.edges[e];
+  for (auto &a : appends)
+    if (a->edge_type == e) return false;
+  if (ncalls != 1 || T < 1 || S < 1 || T > (int)s.model->atypes.size() || es.implicit ||
+      ed.singleedge() || (ed.singletype() && T != ed.target))
+    return false;
+  uint64_t total = slots;
+  if (es.add_existing)
+    for (int U = 1; U < (int)es.csr.size(); U++) {
+      const CSR &c = es.csr[U];
+      if (!c.row_ptr.p) continue;
+      if (U != T || c.nrows > s.agents[T - 1].n ||
+          (c.nedges && ed.stores_src() && c.src_type_const != S))
+        return false;
+      total += c.nedges;
+    }
+  return total < (1ull << 31) && s.agents[T - 1].n < (1ull << 31);
+}
+
+EdgeAppend *ApplyCtx::append_typed(int e, int T, int S, uint64_t slots, bool holes, bool tiled) {
+  Sim &s = *sim;
+  const EdgeTypeDesc &ed = s.model->et(e);
+  std::unique_ptr<EdgeAppend> a;
+  auto it = s.append_spare.find(e);
+  if (it != s.append_spare.end() && it->second->typed) {
+    a = std::move(it->second);
+    s.append_spare.erase(it);
+  } else {
+    a = std::make_unique<EdgeAppend>();
+    a->edge_type = e;
+    a->typed = true;
+  }
+  a->target_type = T;
+  a->src_type = S;
+  a->fixed_count = slots;
+  a->holes = holes;
+  a->tiled = tiled;
+  a->planned = false;
+  if (!tiled && (a->cap < slots || !a->to.p)) {
+    a->cap = std::max<uint64_t>(slots + slots / 8, 1);  // (slack: a growing network)
+    a->to.alloc(a->cap * 4, &s.footprint);
+    a->from.alloc(a->cap * 4, &s.footprint);
+    const int nf = ed.stores_payload() ? (int)ed.fields.size() : 0;
+    a->payload.resize(nf);
+    for (int f = 0; f < nf; f++) a->payload[f].alloc(a->cap * ed.fields[f].size, &s.footprint);
+  }
   appends.push_back(std::move(a));
   return appends.back().get();
 }
@@ -644,6 +696,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
     return std::find(v.begin(), v.end(), r) != v.end();
   };
   std::vector<int> C(call, call + ncall);
+  ctx.ncalls = ncall;
   for (int c : C) {
     if (is_edge_ref(c)) fail(VG_ERR_ARG, "call holds agent types only");
     if (in(ctx.add_existing, c))
@@ -706,6 +759,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
     std::swap(a.rd, a.wr);
     if (ad.immortal() || a.n == 0) continue;
     std::swap(a.died_rd, a.died_wr);
+    if (!ctx.may_die) continue;  // no agent can have died in this transition
     // agents that died in this transition, in index order (writereuseable)
     uint32_t *flag = nullptr, *pos = nullptr;
     VG_CUDA(cudaMallocAsync((void **)&flag, (a.n + 1) * 4, s.stream));
@@ -744,6 +798,10 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
     EdgeAppend *ap = nullptr;
     for (auto &x : ctx.appends)
       if (x->edge_type == e) ap = x.get();
+    if (ap && ap->typed) {
+      build_csr_typed(s, e, *ap);
+      continue;
+    }
     uint64_t n = 0;
     if (ap) {
       if (ap->ordered) {
@@ -755,13 +813,8 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
       if (n > ap->cap) fail(VG_ERR_DEVICE, "edge append buffer overflow");
     }
     bool merge = s.edges[e].add_existing;
-    bool removals = false;
     for (auto &r : ctx.removals)
-      if (r->edge_type == e) {
-        apply_edge_removals(s, e, *r, ap, n, merge);
-        removals = true;
-      }
-    if (ap && !removals && build_csr_typed(s, e, *ap, n)) continue;
+      if (r->edge_type == e) apply_edge_removals(s, e, *r, ap, n, merge);
     std::vector<const void *> pl;
     if (ap)
       for (auto &b : ap->payload) pl.push_back(b.p);
@@ -799,6 +852,7 @@ int vg_apply_host(vg_sim *h, const char *tname, const int *call, int ncall, cons
   AgentStore &a = s.agents[type_nr - 1];
   if (n > a.n) fail(VG_ERR_ARG, "more values than agent slots");
   if (s.async) check_device_status(s, "asynchronous transition");
+  forget_record_spread(s);
   for (size_t f = 0; f < ad.fields.size(); f++) {
     if (!in_fields || !in_fields[f]) continue;
     VG_CUDA(cudaMemcpyAsync(a.rd[f].p, in_fields[f], n * ad.fields[f].size,

@@ -12,7 +12,9 @@
 // 897-920) and, for edge types that store the source, edges whose source
 // died (_remove_edges_agent_source!, :606-631).
 #include <algorithm>
+#include <cstring>
 
+#include "vg_bucket.cuh"
 #include "vg_internal.h"
 
 namespace vg {
@@ -244,61 +246,619 @@ uint64_t csr_edges_total(const EdgeStore &es) {
   return t;
 }
 
-// ---------------------------------------- fast rebuild from typed records
+// ---------------------------------------- rebuild from typed records
 namespace {
-// row key of each record (target agent_nr - 1); a record of another type or
-// beyond the rows sets the status word (the records come from kernels that
-// declare their types)
-// key: the target row; value: the source's agent_nr - 1, which the stable
-// sort then carries straight into the CSR's source column.  With
-// digit_counts, the kernel also counts the keys' 8-bit digits of `passes`
-// sort passes (the radix sort's upfront count: per block in shared memory,
-// then added to digit_counts[256 p + digit]); the grid then strides.
-__global__ void k_typed_keys(const uint64_t *to, const uint64_t *from, uint64_t n,
-                             uint32_t target_type, uint32_t src_type, uint64_t nrows,
-                             uint32_t *keys, uint32_t *src, int *status,
-                             uint32_t *digit_counts, int passes) {
-  __shared__ uint32_t h[4 * 256];
-  if (digit_counts) {
-    for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) h[i] = 0;
-    __syncthreads();
+constexpr int BB_TPB = 256;
+constexpr uint32_t BB_SPAN = 8192;  // rows counted in shared memory at a time
+constexpr uint32_t BB_TILES = 512;  // tiles whose pieces are listed at a time
+constexpr uint32_t BB_NONE = 0xFFFFu;
+constexpr uint32_t BB_U = 4;         // records per thread of a large span, staged once
+constexpr uint32_t BB_FEW = 8;
+
+struct BuildArgs {
+  BucketPlan p;
+  uint64_t nrows;
+  uint32_t span, chunk;
+  uint32_t *rp, *src;        // src null: sources are not kept
+  const uint32_t *slot_src;  // null: a record's value is its source, else its slot
+  int npay;
+  int psize[MAX_FIELDS];
+  const void *pin[MAX_FIELDS];  // by slot
+  void *pout[MAX_FIELDS];
+  // the container that add_existing carries over (null: none)
+  const uint32_t *old_rp, *old_src;
+  uint64_t old_nrows;
+  uint32_t old_ne;
+  const void *old_pay[MAX_FIELDS];
+};
+
+// Rows of the span in shared memory: thread t owns the 4 Q consecutive rows
+// from 4 Q t on, as Q chunks of 16 bytes, chunk q of thread t at q ^ (t mod Q)
+// so that both the per-thread and the consecutive accesses avoid bank
+// conflicts.  Q = 8 for spans of 2048 rows and more, 1 below.
+template <int Q>
+__device__ __forceinline__ uint32_t bb_slot(uint32_t i) {
+  if (Q == 1) return i;
+  const uint32_t t = i / (4 * Q), q = (i >> 2) & (Q - 1);
+  return t * 4 * Q | ((q ^ (t & (Q - 1))) << 2) | (i & 3u);
+}
+
+__device__ __forceinline__ uint32_t bb_reduce(uint32_t v, uint32_t *ws) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  uint32_t t = 0;
+#pragma unroll
+  for (int w = 0; w < BB_TPB / 32; w++) t += ws[w];
+  return t;
+}
+
+// exclusive sum over the block's threads; *total: of all
+__device__ __forceinline__ uint32_t bb_scan(uint32_t v, uint32_t *ws, uint32_t *total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
+  __syncthreads();
+  if (lane == 31) ws[w] = x;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (int w2 = 0; w2 < BB_TPB / 32; w2++) {
+    before += w2 < w ? ws[w2] : 0u;
+    all += ws[w2];
+  }
+  *total = all;
+  return before + x - v;
+}
+
+__device__ __forceinline__ void bb_copy(int size, const void *in, uint64_t i, void *out,
+                                        uint64_t o) {
+  switch (size) {
+    case 1: ((uint8_t *)out)[o] = ((const uint8_t *)in)[i]; break;
+    case 2: ((uint16_t *)out)[o] = ((const uint16_t *)in)[i]; break;
+    case 4: ((uint32_t *)out)[o] = ((const uint32_t *)in)[i]; break;
+    case 8: ((uint64_t *)out)[o] = ((const uint64_t *)in)[i]; break;
+  }
+}
+
+// the value of the record q at place i
+__device__ __forceinline__ uint32_t bb_value(const BucketPlan &p, uint64_t i, uint32_t q) {
+  return p.vals ? p.vals[i] : ((uint32_t)i & ~(uint32_t)(BK_TILE - 1)) + (q >> p.shift);
+}
+
+// lists the bucket's pieces of the tiles from t0 on (pre: records before each,
+// first: its place in its tile); returns their records, *before: the records
+// of earlier buckets in these tiles
+__device__ __forceinline__ uint32_t bb_pieces(const BucketPlan &p, uint32_t b, uint32_t t0,
+                                              uint32_t *pre, uint16_t *first, uint32_t *ws,
+                                              uint32_t *before) {
+  const uint32_t tid = threadIdx.x;
+  uint32_t run = 0, bsum = 0;
+#pragma unroll
+  for (uint32_t r = 0; r < BB_TILES; r += BB_TPB) {
+    const uint32_t t = t0 + r + tid;
+    uint32_t len = 0;
+    if (t < p.ntiles) {
+      const uint16_t *o = p.offs + (uint64_t)t * p.pitch + b;
+      const uint32_t o0 = o[0];
+      first[r + tid] = (uint16_t)o0;
+      len = o[1] - o0;
+      bsum += o0;
+    }
+    uint32_t all;
+    pre[r + tid] = run + bb_scan(len, ws, &all);
+    run += all;
+    if (r + BB_TPB < BB_TILES && t0 + r + BB_TPB >= p.ntiles) break;  // (the rest is not read)
+  }
+  if (tid == 0) pre[min(BB_TILES, p.ntiles - t0)] = run;
+  if (before) *before = bb_reduce(bsum, ws);
+  __syncthreads();
+  return run;
+}
+
+// place of record j of the listed pieces among the tiles' records
+__device__ __forceinline__ uint64_t bb_find(const BucketPlan &p, uint32_t t0, uint32_t j,
+                                            const uint32_t *pre, const uint16_t *first) {
+  uint32_t lo = 0, hi = min(BB_TILES, p.ntiles - t0);  // pre[lo] <= j < pre[hi]
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (pre[mid] <= j) lo = mid;
+    else hi = mid;
+  }
+  return (uint64_t)(t0 + lo) * BK_TILE + first[lo] + (j - pre[lo]);
+}
+
+// One block per bucket (vg_bucket.cuh).  The bucket's records, in order, are
+// its pieces of the tiles one after the other.  They are staged `chunk` at a
+// time, once when all of them fit.
+//   Small spans, staged once: each warp ranks its eighth of the records in
+// order against counters of its own; the counters' sums over the warps are
+// the rows' counts.
+//   Large spans, staged once: each thread keeps its records in registers,
+// counts them with atomics on 16-bit counters and takes the counters' sums
+// as positions.  A row of several records (most of a sparse container's rows
+// have at most one) orders them by comparing each with the row's others, up
+// to BB_FEW; more are walked as below.
+//   Otherwise the records are counted with atomics, in half the span (32-bit
+// counters); ranks within 32 records come from match.any, and the first warp
+// walks the 32s in order, keeping each row's next position.
+// Old edges (add_existing) stay ahead of the new ones in their row.
+// Bound: the row pointers' write for a sparse container (67 MB for 16.8 M
+// cells), the latency of a block's steps for a dense one (pieces, records,
+// ranks, payload: about ten dependent memory accesses).  A bucket of more
+// records than a chunk takes 35 ns per 32 of them, one after the other:
+// records that crowd into few buckets are placed at that rate.
+// Measured, us per launch (and of the tile pass before it): 10^6 records into
+// 16.8 M rows 27 (17; the sort by 8 bits of the row and the row pointers
+// before it took 77 together), 10^6 and 2*10^6 records with payload into 10^5
+// rows 30 on average (16; 64-bit order keys and rows sorted before: 165), 4*10^4
+// new records among 10^6 old edges 19.  Blocks per SM: 4, 5, 6, 7, 8 took 28,
+// 27, 29, 33, 33 (large spans), 2 to 6 took 58, 33, 33, 33, 30 (small).
+template <bool MERGE, int Q>
+__device__ __forceinline__ void bucket_build(const BuildArgs &a, uint32_t span, uint32_t chunk) {
+  extern __shared__ __align__(16) unsigned char bb_smem[];
+  constexpr int BB_WARPS = BB_TPB / 32;
+  uint32_t *cnt = (uint32_t *)bb_smem;             // [span] counts, then positions
+  uint32_t *val = cnt + max(span, 4u);           // [chunk]
+  uint32_t *pos = val + chunk;                   // [chunk]
+  uint32_t *pre = pos + chunk;                   // [BB_TILES + 1] records before a piece
+  uint16_t *first = (uint16_t *)(pre + BB_TILES + 2);  // [BB_TILES] a piece's place in its tile
+  uint16_t *rowl = first + BB_TILES;               // [chunk] row in the span
+  uint16_t *rk = rowl + chunk;                   // [chunk] ranks
+  uint16_t *wc = rk + chunk;                     // Q == 1: [BB_WARPS][span]
+  __shared__ uint32_t ws[BB_WARPS];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const BucketPlan &p = a.p;
+  const uint32_t b = blockIdx.x;
+  const uint64_t row0 = (uint64_t)b << p.shift;
+  // stages records j0 .. of the listed pieces; returns how many
+  auto stage = [&](uint32_t t0, uint32_t j0, uint32_t mr, uint64_t R0) {
+    const uint32_t mc = min(chunk, mr - j0);
+    for (uint32_t j = tid; j < mc; j += BB_TPB) {
+      const uint64_t i = bb_find(p, t0, j0 + j, pre, first);
+      const uint32_t q = p.recs[i];
+      // (wraps when below the span)
+      const uint32_t r = (q & ((1u << p.shift) - 1u)) - (uint32_t)(R0 - row0);
+      rowl[j] = (uint16_t)(r < span ? r : BB_NONE);
+      val[j] = bb_value(p, i, q);
+    }
+    __syncthreads();
+    return mc;
+  };
+  uint32_t base = 0, m = 0;  // records of earlier buckets, of this one
+  const bool one_list = p.ntiles <= BB_TILES;
+  if (one_list) {
+    if (p.ntiles) m = bb_pieces(p, b, 0, pre, first, ws, &base);
+  } else {
+    for (uint32_t t = tid; t < p.ntiles; t += BB_TPB) {
+      const uint16_t *o = p.offs + (uint64_t)t * p.pitch + b;
+      base += o[0];
+      m += (uint32_t)o[1] - o[0];
+    }
+    base = bb_reduce(base, ws);
+    m = bb_reduce(m, ws);
+  }
+  const uint64_t rows_end = min((unsigned long long)a.nrows,
+                                (unsigned long long)(row0 + (1ull << p.shift)));
+  const bool once = m <= chunk && one_list && (1ull << p.shift) <= span;
+  const bool by_warps = Q == 1 && once;
+  if (!once && tid == 0) *(volatile unsigned *)&p.report->crowded = 1;
+  unsigned dmax = 0;
+  for (uint64_t R0 = row0; R0 < rows_end || R0 == row0; R0 += span) {
+    const uint64_t R1 = min((unsigned long long)(R0 + span), (unsigned long long)rows_end);
+    const uint32_t nr = R1 > R0 ? (uint32_t)(R1 - R0) : 0u;
+    uint32_t mc = 0;
+    // warp w's records, by_warps: a whole number of 32s
+    uint32_t share = 0;
+    if (by_warps) {
+      for (uint32_t i = tid; i < BB_WARPS * span / 2; i += BB_TPB) ((uint32_t *)wc)[i] = 0;
+      mc = m ? stage(0, 0, m, R0) : 0u;
+      __syncthreads();
+      share = ((mc + 31) / 32 + BB_WARPS - 1) / BB_WARPS * 32;
+      uint16_t *mine = wc + wid * span;
+      const uint32_t j1 = min(mc, (wid + 1) * share);
+      for (uint32_t j0 = wid * share; j0 < j1; j0 += 32) {
+        const uint32_t j = j0 + lane;
+        const uint32_t r = j < j1 ? rowl[j] : BB_NONE;
+        const unsigned peers = __match_any_sync(0xffffffffu, r);
+        uint32_t at = 0;
+        if (j < j1) at = mine[r];
+        __syncwarp();
+        if (j < j1) {
+          rk[j] = (uint16_t)(at + __popc(peers & lt));
+          if ((peers & lt) == 0) mine[r] = (uint16_t)(at + __popc(peers));
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+      for (uint32_t i = tid; i < span; i += BB_TPB) {
+        uint32_t run = 0;
+#pragma unroll
+        for (int w = 0; w < BB_WARPS; w++) {
+          const uint32_t c = wc[w * span + i];
+          wc[w * span + i] = (uint16_t)run;
+          run += c;
+        }
+        cnt[i] = run;
+      }
+      if (span < 4 && tid < 4 && tid >= span) cnt[tid] = 0;
+    } else {
+      for (uint32_t i = tid; i < max(span, 4u) / 4; i += BB_TPB)
+        ((uint4 *)cnt)[i] = make_uint4(0, 0, 0, 0);
+      __syncthreads();
+      for (uint32_t t0 = 0; t0 < p.ntiles && m; t0 += BB_TILES) {
+        const uint32_t mr = one_list ? m : bb_pieces(p, b, t0, pre, first, ws, nullptr);
+        for (uint32_t j0 = 0; j0 < mr; j0 += chunk) {
+          mc = stage(t0, j0, mr, R0);
+          for (uint32_t j = tid; j < mc; j += BB_TPB)
+            if (rowl[j] != BB_NONE) atomicAdd(&cnt[bb_slot<Q>(rowl[j])], 1u);
+          __syncthreads();
+        }
+      }
+    }
+    __syncthreads();
+    // counts into exclusive sums
+    const uint32_t r_lo = tid * 4 * Q;
+    uint4 v[Q];
+    uint32_t sum = 0, here;
+    if (r_lo < span) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        v[q] = ((uint4 *)cnt)[tid * Q + (q ^ (tid & (Q - 1)))];
+        if (MERGE) {
+          const uint32_t c[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const uint64_t r = R0 + r_lo + 4 * q + k;
+            const uint32_t old = r < a.old_nrows ? a.old_rp[r + 1] - a.old_rp[r] : 0u;
+            dmax = max(dmax, r < a.nrows ? c[k] + old : 0u);
+          }
+        } else {
+          dmax = max(dmax, max(max(v[q].x, v[q].y), max(v[q].z, v[q].w)));
+        }
+        sum += v[q].x + v[q].y + v[q].z + v[q].w;
+      }
+    }
+    uint32_t run = bb_scan(sum, ws, &here);
+    if (r_lo < span) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const uint4 c = v[q];
+        uint4 e;
+        e.x = run;
+        e.y = e.x + c.x;
+        e.z = e.y + c.y;
+        e.w = e.z + c.z;
+        run = e.w + c.w;
+        ((uint4 *)cnt)[tid * Q + (q ^ (tid & (Q - 1)))] = e;
+      }
+    }
+    __syncthreads();
+    if (!MERGE && Q == 8 && nr == span && ((uintptr_t)(a.rp + R0) & 15) == 0) {
+      uint4 *out = (uint4 *)(a.rp + R0);
+      for (uint32_t c = tid; c < span / 4; c += BB_TPB) {
+        uint4 e = ((const uint4 *)cnt)[bb_slot<Q>(4 * c) >> 2];
+        e.x += base;
+        e.y += base;
+        e.z += base;
+        e.w += base;
+        out[c] = e;
+      }
+    } else {
+      for (uint32_t i = tid; i < nr; i += BB_TPB) {
+        uint32_t e = base + cnt[bb_slot<Q>(i)];
+        if (MERGE) e += R0 + i < a.old_nrows ? a.old_rp[R0 + i] : a.old_ne;
+        a.rp[R0 + i] = e;
+      }
+    }
+    if (MERGE && R0 < a.old_nrows) {
+      // old edge k of row r moves up by the new records of the rows before
+      const uint64_t O1 = min((unsigned long long)R1, (unsigned long long)a.old_nrows);
+      const uint32_t k0 = a.old_rp[R0], k1 = a.old_rp[O1];
+      for (uint32_t k = k0 + tid; k < k1; k += BB_TPB) {
+        uint32_t lo = 0, hi = (uint32_t)(O1 - R0);  // old_rp[R0 + lo] <= k < old_rp[R0 + hi]
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (a.old_rp[R0 + mid] <= k) lo = mid;
+          else hi = mid;
+        }
+        const uint64_t o = (uint64_t)k + base + cnt[bb_slot<Q>(lo)];
+        if (a.src) a.src[o] = a.old_src[k];
+        for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.old_pay[f], k, a.pout[f], o);
+      }
+    }
+    // one record into the container
+    auto put = [&](uint32_t j, uint32_t at) {
+      uint64_t o = (uint64_t)base + at;
+      if (MERGE) {
+        const uint64_t r = R0 + rowl[j];
+        o += r < a.old_nrows ? a.old_rp[r + 1] : a.old_ne;
+      }
+      const uint32_t u = val[j];
+      if (a.src) a.src[o] = a.slot_src ? a.slot_src[u] : u;
+      for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.pin[f], u, a.pout[f], o);
+    };
+    if (by_warps) {
+      // in place order, so that consecutive threads write consecutive edges
+      for (uint32_t j = tid; j < mc; j += BB_TPB)
+        pos[cnt[rowl[j]] + wc[j / share * span + rowl[j]] + rk[j]] = j;
+      __syncthreads();
+      for (uint32_t at = tid; at < mc; at += BB_TPB) put(pos[at], at);
+    } else {
+      __syncthreads();
+      for (uint32_t t0 = 0; t0 < p.ntiles && m; t0 += BB_TILES) {
+        const uint32_t mr = once || one_list ? m : bb_pieces(p, b, t0, pre, first, ws, nullptr);
+        for (uint32_t j0 = 0; j0 < mr; j0 += chunk) {
+          if (!once) mc = stage(t0, j0, mr, R0);
+          const uint32_t groups = (mc + 31) / 32;
+          for (uint32_t c = wid; c < groups; c += BB_WARPS) {
+            const uint32_t j = c * 32 + lane;
+            const uint32_t r = j < mc ? rowl[j] : BB_NONE;
+            const unsigned peers = __match_any_sync(0xffffffffu, r);
+            if (j < mc) rk[j] = (uint16_t)(__popc(peers & lt) | (__popc(peers) - 1) << 5);
+          }
+          __syncthreads();
+          if (wid == 0) {
+            for (uint32_t c = 0; c < groups; c++) {
+              const uint32_t j = c * 32 + lane;
+              const uint32_t r = j < mc ? rowl[j] : BB_NONE, q = j < mc ? rk[j] : 0u;
+              if (__all_sync(0xffffffffu, r == BB_NONE)) continue;  // (other parts of the span)
+              const uint32_t sl = r == BB_NONE ? 0u : bb_slot<Q>(r);
+              const uint32_t at = cnt[sl];
+              __syncwarp();
+              if (r != BB_NONE) {
+                if ((q & 31u) == 0) cnt[sl] = at + (q >> 5) + 1;
+                pos[j] = at + (q & 31u);
+              }
+              __syncwarp();
+            }
+          }
+          __syncthreads();
+          for (uint32_t j = tid; j < mc; j += BB_TPB)
+            if (rowl[j] != BB_NONE) put(j, pos[j]);
+          __syncthreads();
+        }
+      }
+    }
+    base += here;
+  }
+  if (b + 1 == p.nbuckets && tid == 0) a.rp[a.nrows] = base + (MERGE ? a.old_ne : 0u);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) dmax = max(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+  if (lane == 0 && dmax) atomicMax(a.p.maxdeg, dmax);
+}
+
+template <bool MERGE, int Q>
+__global__ void __launch_bounds__(BB_TPB, 6) k_bucket_build(const __grid_constant__ BuildArgs a) {
+  bucket_build<MERGE, Q>(a, a.span, a.chunk);
+}
+
+// out of line: k_bucket_rows' own path keeps its registers
+__device__ __noinline__ void bucket_build_apart(const BuildArgs &a, uint32_t span, uint32_t chunk) {
+  bucket_build<false, 8>(a, span, chunk);
+}
+
+// A bucket of 2048 R rows whose records fit the threads' registers: 16-bit
+// counters, the thread's 8 R rows as R chunks of 16 bytes (chunk q at an
+// exclusive-or with the thread's number that keeps 16-byte accesses of eight
+// threads apart).
+template <int R>
+__device__ __forceinline__ uint32_t br_chunk(uint32_t t, uint32_t q) {
+  return t * R + (R == 1 ? 0u : q ^ (t / (8 / R) & (R - 1)));
+}
+template <int R>
+__device__ __forceinline__ uint32_t br_slot(uint32_t row) {
+  return br_chunk<R>(row / (8 * R), row / 8 & (R - 1)) * 8 + (row & 7u);
+}
+
+template <int R>
+__global__ void __launch_bounds__(BB_TPB, 5) k_bucket_rows(const __grid_constant__ BuildArgs a) {
+  constexpr uint32_t SPAN = 2048 * R;
+  extern __shared__ __align__(16) unsigned char bb_smem[];
+  uint4 *cnt4 = (uint4 *)bb_smem;                      // [BB_TPB R]
+  uint16_t *cnt = (uint16_t *)cnt4;                    // [SPAN], by br_slot
+  uint32_t *pre = (uint32_t *)(cnt4 + BB_TPB * R);     // [BB_TILES + 2]
+  uint16_t *first = (uint16_t *)(pre + BB_TILES + 2);  // [BB_TILES]
+  uint16_t *lst = first + BB_TILES;                    // [BB_U BB_TPB]
+  uint16_t *pos = lst + BB_U * BB_TPB;                 // [BB_U BB_TPB]
+  __shared__ uint32_t ws[BB_TPB / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, b = blockIdx.x;
+  const BucketPlan &p = a.p;
+  uint32_t base = 0, m = 0;
+  if (p.ntiles && p.ntiles <= BB_TILES) m = bb_pieces(p, b, 0, pre, first, ws, &base);
+  if (p.ntiles > BB_TILES || m > BB_U * BB_TPB || 1u << p.shift != SPAN) {
+    __syncthreads();
+    if (tid == 0) *(volatile unsigned *)&p.report->crowded = 1;
+    bucket_build_apart(a, SPAN / 2, 512);
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < R; q++) cnt4[tid + BB_TPB * q] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  const uint64_t R0 = (uint64_t)b << p.shift;
+  uint32_t row[BB_U], val[BB_U], arr[BB_U];
+#pragma unroll
+  for (int u = 0; u < BB_U; u++) {
+    const uint32_t j = tid + BB_TPB * u;
+    row[u] = BB_NONE;
+    if (j < m) {
+      const uint64_t i = bb_find(p, 0, j, pre, first);
+      const uint32_t q = p.recs[i];
+      row[u] = q & (SPAN - 1);
+      val[u] = bb_value(p, i, q);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < BB_U; u++)
+    if (row[u] != BB_NONE) {
+      const uint32_t sl = br_slot<R>(row[u]), sh = 16 * (sl & 1u);
+      arr[u] = atomicAdd((uint32_t *)cnt + (sl >> 1), 1u << sh) >> sh & 0xffffu;
+    }
+  __syncthreads();
+  // exclusive sums of the thread's 8 R counters, two to a word
+  uint32_t c[4 * R], sum = 0, top = 0;
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const uint4 v = cnt4[br_chunk<R>(tid, q)];
+    c[4 * q] = v.x;
+    c[4 * q + 1] = v.y;
+    c[4 * q + 2] = v.z;
+    c[4 * q + 3] = v.w;
+  }
+#pragma unroll
+  for (int k = 0; k < 4 * R; k++) {
+    sum += c[k];  // (the two halves' sums stay below 2^16)
+    top = __vmaxu2(top, c[k]);
+  }
+  const uint32_t dmax = max(top & 0xffffu, top >> 16);
+  uint32_t all;
+  uint32_t run = bb_scan((sum & 0xffffu) + (sum >> 16), ws, &all);
+#pragma unroll
+  for (int k = 0; k < 4 * R; k++) {
+    const uint32_t lo = c[k] & 0xffffu, hi = c[k] >> 16;
+    c[k] = run | (run + lo) << 16;
+    run += lo + hi;
+  }
+#pragma unroll
+  for (int q = 0; q < R; q++)
+    cnt4[br_chunk<R>(tid, q)] = make_uint4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+  // 0: no row of two records, 1: none of more than BB_FEW, 2 or 3: some
+  const int crowd = __syncthreads_or(dmax > BB_FEW ? 2 : dmax > 1 ? 1 : 0);
+  const uint32_t nr = a.nrows > R0 ? (uint32_t)min((unsigned long long)SPAN,
+                                                   (unsigned long long)(a.nrows - R0)) : 0u;
+  // four rows per thread and round; a round's 1024 rows lie one behind the
+  // other in either layout
+  const uint2 *from = (const uint2 *)(cnt + br_slot<R>(4 * tid));
+  uint32_t *out = a.rp + R0 + 4 * tid;
+  auto sums = [&](int k) {
+    const uint2 v = from[k * BB_TPB];
+    return make_uint4(base + (v.x & 0xffffu), base + (v.x >> 16), base + (v.y & 0xffffu),
+                      base + (v.y >> 16));
+  };
+  if (nr == SPAN) {
+#pragma unroll
+    for (int k = 0; k < 2 * R; k++) *(uint4 *)(out + k * 4 * BB_TPB) = sums(k);
+  } else {
+    for (int k = 0; k < 2 * R; k++) {
+      const uint4 e = sums(k);
+      const uint32_t r = 4 * (tid + BB_TPB * k);
+      uint32_t *q = out + k * 4 * BB_TPB;
+      if (r < nr) q[0] = e.x;
+      if (r + 1 < nr) q[1] = e.y;
+      if (r + 2 < nr) q[2] = e.z;
+      if (r + 3 < nr) q[3] = e.w;
+    }
+  }
+  if (b + 1 == p.nbuckets && tid == 0) a.rp[a.nrows] = base + m;
+  uint32_t at[BB_U];
+  if (crowd < 2) {
+    if (crowd) {
+#pragma unroll
+      for (int u = 0; u < BB_U; u++)
+        if (row[u] != BB_NONE) lst[cnt[br_slot<R>(row[u])] + arr[u]] = (uint16_t)(tid + BB_TPB * u);
+      __syncthreads();
+    }
+#pragma unroll
+    for (int u = 0; u < BB_U; u++)
+      if (row[u] != BB_NONE) {
+        at[u] = cnt[br_slot<R>(row[u])];
+        if (crowd) {
+          const uint32_t end = row[u] + 1 < SPAN ? cnt[br_slot<R>(row[u] + 1)] : m;
+          uint32_t rank = 0;
+          for (uint32_t k = at[u]; k < end; k++) rank += lst[k] < tid + BB_TPB * u;
+          at[u] += rank;
+        }
+      }
+  } else {
+#pragma unroll
+    for (int u = 0; u < BB_U; u++) lst[tid + BB_TPB * u] = (uint16_t)row[u];
+    __syncthreads();
+    if (tid < 32) {
+      const unsigned lt = (1u << lane) - 1u;
+      for (uint32_t j = lane; j - lane < m; j += 32) {
+        const uint32_t r = lst[j];
+        const unsigned peers = __match_any_sync(0xffffffffu, r);
+        const uint32_t sl = r == BB_NONE ? 0u : br_slot<R>(r);
+        const uint32_t first_at = cnt[sl];
+        __syncwarp();
+        if (r != BB_NONE) {
+          pos[j] = (uint16_t)(first_at + __popc(peers & lt));
+          if ((peers & lt) == 0) cnt[sl] = (uint16_t)(first_at + __popc(peers));
+        }
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < BB_U; u++)
+      if (row[u] != BB_NONE) at[u] = pos[tid + BB_TPB * u];
+  }
+  // the values in place order (over the lists, which nobody reads any more),
+  // so that consecutive threads write consecutive edges
+  __syncthreads();
+  uint32_t *byplace = pre;  // [BB_U BB_TPB] 32-bit words over pre, first and lst
+#pragma unroll
+  for (int u = 0; u < BB_U; u++)
+    if (row[u] != BB_NONE) byplace[at[u]] = val[u];
+  __syncthreads();
+  for (uint32_t k = tid; k < m; k += BB_TPB) {
+    const uint64_t o = (uint64_t)base + k;
+    const uint32_t v = byplace[k];
+    if (a.src) a.src[o] = a.slot_src ? a.slot_src[v] : v;
+    for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.pin[f], v, a.pout[f], o);
+  }
+  unsigned d = dmax;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) d = max(d, __shfl_xor_sync(0xffffffffu, d, o));
+  if (lane == 0 && d) atomicMax(a.p.maxdeg, d);
+}
+
+// ------------------------------------- typed rebuild by a radix sort
+// For records that crowd into few buckets, that are too many for the buckets'
+// blocks, or of which it is not known yet (plan_buckets).
+// Keys and values of the slots (holes: key nrows, behind every row); the
+// kernel also counts the keys' 8-bit digits for the sort's passes (its
+// upfront count: per block in shared memory, then added to
+// digit_counts[256 p + digit]).
+__global__ void k_typed_keys(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ in,
+                             uint64_t n, uint64_t nrows, uint32_t *__restrict__ keys,
+                             uint32_t *__restrict__ vals, uint32_t *digit_counts, int passes) {
+  __shared__ uint32_t h[4 * 256];
+  for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) h[i] = 0;
+  __syncthreads();
   // four records per thread and round, their loads issued before the
   // shared-memory counts (which would otherwise order each load after the
   // previous record's atomics)
   constexpr int U = 4;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t k0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k0 < n; k0 += U * stride) {
-    uint64_t tv[U], fv[U];
+    uint32_t r[U], v[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint64_t k = k0 + u * stride;
-      tv[u] = k < n ? to[k] : 0;
-      fv[u] = k < n ? from[k] : 0;
+      r[u] = k < n ? rows[k] : 0u;
+      v[u] = k < n && in ? in[k] : (uint32_t)k;
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint64_t k = k0 + u * stride;
       if (k >= n) break;
-      const uint64_t t = tv[u], f = fv[u];
-      uint64_t r = (t & NR_MASK) - 1;
-      const bool bad = (uint32_t)(t >> SHIFT_TYPE) != target_type || r >= nrows ||
-                       (uint32_t)(f >> SHIFT_TYPE) != src_type;
-      if (bad) {
-        atomicCAS(status, 0, 501);
-        r = 0;
-      }
-      keys[k] = (uint32_t)r;
-      src[k] = (uint32_t)((f & NR_MASK) - 1);
-      if (digit_counts)
-        for (int p = 0; p < passes; p++) atomicAdd(&h[p * 256 + ((r >> (8 * p)) & 255u)], 1u);
+      const uint32_t key = r[u] == BK_HOLE ? (uint32_t)nrows : r[u];
+      keys[k] = key;
+      vals[k] = v[u];
+      for (int p = 0; p < passes; p++) atomicAdd(&h[p * 256 + ((key >> (8 * p)) & 255u)], 1u);
     }
   }
-  if (digit_counts) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < passes * 256; i += blockDim.x)
-      if (h[i]) atomicAdd(digit_counts + i, h[i]);
-  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < passes * 256; i += blockDim.x)
+    if (h[i]) atomicAdd(digit_counts + i, h[i]);
 }
 
 // row_ptr of the rows 0..nrows from the sorted row keys: rp[r] = the
@@ -344,9 +904,24 @@ __global__ void __launch_bounds__(TPB) k_rp_fill(const uint32_t *keys, uint64_t 
   uint4 *E4 = reinterpret_cast<uint4 *>(E);
   for (uint32_t i = tid; i < RP_ROWS / 4; i += TPB) E4[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  for (uint32_t k = k0 + tid; k < k1; k += TPB) {
-    const uint32_t key = keys[k];
-    if (k + 1 == k1 || keys[k + 1] != key) E[rp_slot(key - (uint32_t)R0)] = k + 1 - k0;
+  // (eight records in flight per thread: a crowded span is one block's work,
+  // and one at a time took 300 ns each round; keys from nrows on are slots
+  // without a record)
+  constexpr int U = 8;
+  for (uint32_t kk = k0 + tid; kk < k1; kk += U * TPB) {
+    uint32_t key[U], next[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint32_t k = kk + u * TPB;
+      key[u] = k < k1 ? keys[k] : 0u;
+      next[u] = k + 1 < k1 ? keys[k + 1] : 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint32_t k = kk + u * TPB;
+      if (k < k1 && next[u] != key[u] && key[u] < nrows)
+        E[rp_slot(key[u] - (uint32_t)R0)] = k + 1 - k0;
+    }
   }
   __syncthreads();
   // pass 1: the largest end in the thread's 32 rows (its last stored end)
@@ -400,6 +975,63 @@ __global__ void __launch_bounds__(TPB) k_rp_fill(const uint32_t *keys, uint64_t 
   if (lane == 0 && dmax) atomicMax(maxdeg, dmax);
 }
 
+// largest number of records in a bucket of 2^shift rows, reported to the host
+__global__ void __launch_bounds__(1024) k_bucket_load(const uint32_t *rp, uint64_t nrows,
+                                                      uint32_t shift, uint32_t nbuckets,
+                                                      uint32_t gen, RebuildReport *report) {
+  __shared__ unsigned top;
+  if (threadIdx.x == 0) top = 0;
+  __syncthreads();
+  for (uint32_t b = threadIdx.x; b < nbuckets; b += 1024) {
+    const uint64_t r0 = (uint64_t)b << shift, r1 = min((unsigned long long)nrows, (unsigned long long)(r0 + (1ull << shift)));
+    atomicMax(&top, rp[r1] - rp[r0]);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    *(volatile unsigned long long *)&report->load = (unsigned long long)gen << 32 | top;
+}
+
+// the sorted records into the container's columns (old edges stay ahead)
+__global__ void k_place_sorted(const uint32_t *keys, const uint32_t *vals, uint64_t n, BuildArgs a) {
+  const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n || keys[j] >= a.nrows) return;
+  uint64_t o = j;
+  if (a.old_rp) o += keys[j] < a.old_nrows ? a.old_rp[keys[j] + 1] : a.old_ne;
+  const uint32_t v = vals[j];
+  if (a.src) a.src[o] = a.slot_src ? a.slot_src[v] : v;
+  for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.pin[f], v, a.pout[f], o);
+}
+
+// row pointers of old and new edges together
+__global__ void k_merge_rows(const uint32_t *new_rp, BuildArgs a) {
+  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned deg = 0;
+  if (r <= a.nrows) {
+    const uint32_t o0 = r < a.old_nrows ? a.old_rp[r] : a.old_ne;
+    a.rp[r] = o0 + new_rp[r];
+    if (r < a.nrows) {
+      const uint32_t o1 = r < a.old_nrows ? a.old_rp[r + 1] : a.old_ne;
+      deg = o1 - o0 + new_rp[r + 1] - new_rp[r];
+    }
+  }
+  deg = __reduce_max_sync(0xffffffffu, deg);
+  if ((threadIdx.x & 31) == 0 && deg) atomicMax(a.p.maxdeg, deg);
+}
+
+__global__ void k_merge_old(const uint32_t *new_rp, BuildArgs a) {
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= a.old_ne) return;
+  uint64_t lo = 0, hi = a.old_nrows;  // old_rp[lo] <= k < old_rp[hi]
+  while (hi - lo > 1) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (a.old_rp[mid] <= k) lo = mid;
+    else hi = mid;
+  }
+  const uint64_t o = k + new_rp[lo];
+  if (a.src) a.src[o] = a.old_src[k];
+  for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.old_pay[f], k, a.pout[f], o);
+}
+
 }  // namespace
 
 uint32_t csr_max_degree(Sim &s, CSR &c) {
@@ -411,72 +1043,140 @@ uint32_t csr_max_degree(Sim &s, CSR &c) {
   return c.max_degree;
 }
 
-bool build_csr_typed(Sim &s, int e, const EdgeAppend &ap, uint64_t n) {
-  const EdgeTypeDesc &ed = s.model->et(e);
+static void ensure_buf(Sim &s, DevBuf &b, uint64_t bytes, bool slack = false) {
+  if (b.bytes < bytes || !b.p)
+    b.alloc(std::max<uint64_t>(slack ? bytes + bytes / 8 : bytes, 16), &s.footprint);
+}
+
+void forget_record_spread(Sim &s) {
+  for (auto &es : s.edges)
+    for (auto &c : es.csr)
+      if (c.rebuild) c.rebuild->forget();
+}
+
+// Buckets of about 512 records, 1024 rows or 1024 old edges carried over,
+// whichever asks for more of them, up to BK_MAX (the chip holds about 700
+// blocks at a time: fewer buckets leave it idle), each of at most BB_SPAN
+// rows.  The buckets take a rebuild when every bucket's records fit its
+// block's stage: a bucket that does not is placed at 5 ns per record by that
+// one block (10^6 records in one cell: 5.1 ms, the sort 0.33).  So the sort
+// takes rebuilds of more rows or records than that, and every rebuild until
+// one with the same sizes has reported its largest bucket; the buckets take
+// the following ones until a block reports that its bucket did not fit, or
+// the agents are written from outside.  The reports are read without waiting.
+// Measured, us per walker step, buckets and sort: 10^6 walkers on 4096^2
+// cells 49 and 94, on 1024^2 44 and 90, 10^5 on 1000 x 800 20 and 59, 10^4 on
+// 4096^2 32 and 64; 10^6 on 9000^2 476 and 164, 9*10^6 on 3000^2 661 and 438;
+// 10^6 on a tenth, a hundredth of 4096^2 148 and 98, 1060 and 143.
+BucketPlan plan_buckets(Sim &s, int e, int T, uint64_t n, bool vals) {
   EdgeStore &es = s.edges[e];
-  // the form the typed emitters produce: sources kept, no payload columns
-  if (!ap.ordered || ap.target_type <= 0 || !ed.stores_src() || ap.src_type <= 0 ||
-      ed.stores_payload() || ed.bool_only() || ed.singleedge() || es.add_existing ||
-      n >= (1ull << 31))
-    return false;
-  const int T = ap.target_type;
-  if (T > (int)s.model->atypes.size() || (ed.singletype() && T != ed.target)) return false;
-  s.csr_epoch++;
-  cudaStream_t st = s.stream;
   if (es.csr.size() < (size_t)MAX_AGENT_TYPES) es.csr.resize(MAX_AGENT_TYPES);
-  for (int U = 1; U < (int)es.csr.size(); U++)
-    if (U != T && es.csr[U].row_ptr.p) es.csr[U] = CSR();
   CSR &c = es.csr[T];
-  const uint64_t nrows = s.agents[T - 1].n;
-  // buffers of the previous container are reused when large enough (the
-  // stream orders every earlier reader before these writes)
-  auto ensure = [&](DevBuf &b, uint64_t bytes) {
-    if (b.bytes < bytes || !b.p) b.alloc(std::max<uint64_t>(bytes, 16), &s.footprint);
-  };
-  ensure(c.row_ptr, (nrows + 1) * 4);
-  ensure(c.src, std::max<uint64_t>(n, 1) * 4);
-  c.src_type.release();
-  c.payload.clear();
-  ensure(c.d_max_degree, 4);
   if (!c.rebuild) c.rebuild.reset(new RebuildCache());
   RebuildCache &rc = *c.rebuild;
-  const int bits = bits_for(nrows ? nrows - 1 : 0);
+  if (!s.reports_host) {
+    const size_t bytes = MAX_EDGE_TYPES * MAX_AGENT_TYPES * sizeof(RebuildReport);
+    void *h = nullptr, *d = nullptr;
+    VG_CUDA(cudaHostAlloc(&h, bytes, cudaHostAllocMapped));
+    std::memset(h, 0, bytes);
+    s.reports_host = (RebuildReport *)h;
+    VG_CUDA(cudaHostGetDevicePointer(&d, h, 0));
+    s.reports_dev = (RebuildReport *)d;
+  }
+  const uint64_t nrows = std::max<uint64_t>(s.agents[T - 1].n, 1);
+  auto buckets = [&](uint32_t shift) { return (nrows + (1ull << shift) - 1) >> shift; };
+  const uint64_t load = std::max<uint64_t>({n / 512, nrows / 1024,
+                                            es.add_existing ? c.nedges / 1024 : 0});
+  const uint64_t want = std::min<uint64_t>(BK_MAX, std::max<uint64_t>(1, load));
+  BucketPlan p;
+  while (buckets(p.shift) > want) p.shift++;
+  while (p.shift > 0 && (1u << p.shift) > BB_SPAN && buckets(p.shift - 1) <= BK_MAX) p.shift--;
+  p.n = n;
+  p.nbuckets = (uint32_t)buckets(p.shift);
+  p.ntiles = (uint32_t)((n + BK_TILE - 1) / BK_TILE);
+  p.pitch = (p.nbuckets + 4) & ~3u;
+  // (small spans stage 2048 records, large ones keep BB_U per thread)
+  p.limit = 1u << p.shift >= 2048 ? (es.add_existing ? 1024 : BB_U * BB_TPB) : 2048;
+  ensure_buf(s, c.d_max_degree, 4);
+  p.maxdeg = c.d_max_degree.as<unsigned>();
+  p.report = s.reports_dev + e * MAX_AGENT_TYPES + T;
+  volatile RebuildReport *rep = s.reports_host + e * MAX_AGENT_TYPES + T;
+  const bool same = rc.known_rows == nrows && rc.known_buckets == p.nbuckets &&
+                    n <= rc.known_n + rc.known_n / 16;
+  if (!same) {
+    rc.forget();
+  } else if (rc.known) {
+    if (rep->crowded) rc.forget();
+  } else {
+    const uint64_t load = rep->load;
+    const uint32_t gen = (uint32_t)(load >> 32);
+    if ((int32_t)(gen - rc.unknown_gen) > 0 && (int32_t)(rc.sort_gen - gen) >= 0 &&
+        (uint32_t)load <= p.limit - p.limit / 8) {
+      rc.known = true;
+      rep->crowded = 0;
+    }
+  }
+  p.fits = 1u << p.shift <= BB_SPAN && p.ntiles <= BB_TILES && n <= (uint64_t)p.nbuckets * p.limit;
+  p.sorted = !rc.known || !p.fits;
+  // (at most one bucket's records: nothing to be known)
+  if (n <= p.limit && 1u << p.shift <= BB_SPAN) p.sorted = false;
+  if (p.sorted) {
+    rc.known_n = n;
+    rc.known_rows = nrows;
+    rc.known_buckets = p.nbuckets;
+    return p;
+  }
+  ensure_buf(s, rc.recs, (uint64_t)p.ntiles * BK_TILE * 4, true);
+  if (vals) ensure_buf(s, rc.vals, (uint64_t)p.ntiles * BK_TILE * 4, true);
+  ensure_buf(s, rc.offs, (uint64_t)p.ntiles * p.pitch * 2, true);
+  p.recs = rc.recs.as<uint32_t>();
+  p.vals = vals ? rc.vals.as<uint32_t>() : nullptr;
+  p.offs = rc.offs.as<uint16_t>();
+  if (!p.ntiles) VG_CUDA(cudaMemsetAsync(p.maxdeg, 0, 4, s.stream));
+  return p;
+}
+
+// The rows of the records sorted, row pointers from the sorted rows, then the
+// records' columns; a plain container (sources only, nothing carried over)
+// has its source column carried through the sort, and its launch sequence
+// replayed from a recorded graph.
+static void build_sorted(Sim &s, CSR &c, const EdgeAppend &ap, BuildArgs &a, bool merge) {
+  cudaStream_t st = s.stream;
+  RebuildCache &rc = *c.rebuild;
+  const uint64_t n = a.p.n, nrows = a.nrows;
+  const bool plain = !merge && a.npay == 0 && a.src && !ap.holes;
+  const int bits = bits_for(ap.holes ? nrows : nrows ? nrows - 1 : 0);
   const uint64_t nbr = (nrows + 1 + RP_ROWS - 1) / RP_ROWS;
   const uint64_t sort_bytes = radix_sort_scratch_bytes(n, 4, bits);
-  ensure(rc.keys, std::max<uint64_t>(n, 1) * 4);
-  ensure(rc.bstart, (nbr + 1) * 4);
-  if (sort_bytes) ensure(rc.sort, sort_bytes);
-  const uint64_t *from = ap.from.as<uint64_t>();
-  // the sorted values are the source column itself
-  uint32_t *keys = rc.keys.as<uint32_t>(), *src = c.src.as<uint32_t>();
-  // the launch sequence, a function of these arguments only
-  const std::vector<uint64_t> args = {
-      (uint64_t)ap.to.p,  (uint64_t)from,          n,
-      nrows,              (uint64_t)T,             (uint64_t)ap.src_type,
-      (uint64_t)c.row_ptr.p, (uint64_t)src,        (uint64_t)c.d_max_degree.p,
-      (uint64_t)keys,     (uint64_t)rc.sort.p,     (uint64_t)rc.bstart.p,
-      (uint64_t)s.d_status.p};
+  ensure_buf(s, rc.keys, std::max<uint64_t>(n, 1) * 4, true);
+  if (!plain) ensure_buf(s, rc.vals, std::max<uint64_t>(n, 1) * 4, true);
+  ensure_buf(s, rc.bstart, (nbr + 1) * 4, true);
+  if (merge) ensure_buf(s, rc.new_rp, (nrows + 1) * 4, true);
+  if (sort_bytes) ensure_buf(s, rc.sort, sort_bytes, true);
+  uint32_t *keys = rc.keys.as<uint32_t>();
+  uint32_t *vals = plain ? a.src : rc.vals.as<uint32_t>();
+  uint32_t *rp = merge ? rc.new_rp.as<uint32_t>() : a.rp;
+  const uint32_t *rows = ap.to.as<uint32_t>(), *in = a.slot_src ? nullptr : ap.from.as<uint32_t>();
   auto enqueue = [&]() {
-    VG_CUDA(cudaMemsetAsync(c.d_max_degree.p, 0, 4, st));
+    VG_CUDA(cudaMemsetAsync(a.p.maxdeg, 0, 4, st));
     if (n) {
-      // the sort's digit counts come from the key kernel (one pass over the
-      // records fewer)
-      const bool counted = sort_bytes > 0;
-      const int passes = std::min((bits + 7) / 8, 4);
-      uint32_t *dc = counted ? radix_sort_digit_counts(rc.sort.p) : nullptr;
-      if (counted) VG_CUDA(cudaMemsetAsync(dc, 0, (size_t)passes * 256 * 4, st));
-      const unsigned kb = counted ? std::min<unsigned>(nblk(n), 152 * 4) : nblk(n);
-      k_typed_keys<<<kb, TPB, 0, st>>>(ap.to.as<uint64_t>(), from, n, (uint32_t)T,
-                                       (uint32_t)ap.src_type, nrows, keys, src,
-                                       s.d_status.as<int>(), dc, passes);
-      radix_sort_pairs_u32_in(keys, src, n, bits, st, s.d_status.as<int>(), rc.sort.p, counted);
+      const int passes = sort_bytes ? std::min((bits + 7) / 8, 4) : 0;
+      uint32_t *dc = radix_sort_digit_counts(rc.sort.p);
+      if (passes) VG_CUDA(cudaMemsetAsync(dc, 0, (size_t)passes * 256 * 4, st));
+      k_typed_keys<<<std::min<unsigned>(nblk(n), 152 * 4), TPB, 0, st>>>(rows, in, n, nrows, keys,
+                                                                        vals, dc, passes);
+      radix_sort_pairs_u32_in(keys, vals, n, bits, st, s.d_status.as<int>(), rc.sort.p, passes > 0);
     }
     k_rp_bounds<<<nblk(n + 1), TPB, 0, st>>>(keys, n, nbr, rc.bstart.as<uint32_t>());
-    k_rp_fill<<<(unsigned)nbr, TPB, 0, st>>>(keys, nrows, rc.bstart.as<uint32_t>(),
-                                             c.row_ptr.as<uint32_t>(),
-                                             c.d_max_degree.as<unsigned>());
+    k_rp_fill<<<(unsigned)nbr, TPB, 0, st>>>(keys, nrows, rc.bstart.as<uint32_t>(), rp,
+                                             a.p.maxdeg);
     VG_CUDA(cudaGetLastError());
   };
+  // the launch sequence, a function of these arguments only
+  const std::vector<uint64_t> args = {(uint64_t)rows, (uint64_t)in,   n,
+                                      nrows,          (uint64_t)rp,   (uint64_t)vals,
+                                      (uint64_t)keys, (uint64_t)rc.sort.p, (uint64_t)rc.bstart.p,
+                                      (uint64_t)a.p.maxdeg, (uint64_t)s.d_status.p, (uint64_t)bits};
   const bool graphable = st != nullptr && st != cudaStreamLegacy && st != cudaStreamPerThread;
   if (rc.exec && args == rc.graph_args) {
     VG_CUDA(cudaGraphLaunch(rc.exec, st));
@@ -506,15 +1206,129 @@ bool build_csr_typed(Sim &s, int e, const EdgeAppend &ap, uint64_t n) {
   } else {
     enqueue();
   }
-  rc.last = std::move(args);
+  rc.last = args;
+  rc.sort_gen++;
+  // (the first two rebuilds after what was known ended, then every eighth)
+  const uint32_t since = rc.sort_gen - rc.unknown_gen;
+  if (nrows && a.p.fits && (since <= 2 || since % 8 == 0))
+    k_bucket_load<<<1, 1024, 0, st>>>(rp, nrows, a.p.shift, a.p.nbuckets, rc.sort_gen, a.p.report);
+  if (merge) {
+    VG_CUDA(cudaMemsetAsync(a.p.maxdeg, 0, 4, st));
+    k_merge_rows<<<nblk(nrows + 1), TPB, 0, st>>>(rp, a);
+    if (a.old_ne) k_merge_old<<<nblk(a.old_ne), TPB, 0, st>>>(rp, a);
+  }
+  if (!plain && n) k_place_sorted<<<nblk(n), TPB, 0, st>>>(keys, vals, n, a);
   VG_CUDA(cudaGetLastError());
+}
+
+static void launch_buckets(const BuildArgs &a, bool merge, cudaStream_t st) {
+  // shared memory of bucket_build and of k_bucket_rows<rows / 2048>
+  auto general = [](uint64_t span, uint64_t chunk, bool big) {
+    return (size_t)((std::max<uint64_t>(span, 4) + 2 * chunk + BB_TILES + 2) * 4 +
+                    (BB_TILES + 2 * chunk) * 2 + (big ? 0 : BB_TPB / 32 * span * 2) + 16);
+  };
+  const bool big = a.span >= 2048;
+  size_t smem = general(a.span, a.chunk, big);
+  void (*k)(const BuildArgs);
+  if (merge) {
+    k = big ? k_bucket_build<true, 8> : k_bucket_build<true, 1>;
+  } else if (!big) {
+    k = k_bucket_build<false, 1>;
+  } else {
+    k = a.span == 2048 ? k_bucket_rows<1> : a.span == 4096 ? k_bucket_rows<2> : k_bucket_rows<4>;
+    smem = std::max<size_t>(general(a.span / 2, 512, true),
+                            a.span * 2 + (BB_TILES + 2) * 4 + BB_TILES * 2 + 2 * BB_U * BB_TPB * 2);
+  }
+  static const bool ok = [] {
+    bool r = true;
+    for (auto f : {k_bucket_build<true, 8>, k_bucket_build<true, 1>, k_bucket_build<false, 1>,
+                   k_bucket_rows<1>, k_bucket_rows<2>, k_bucket_rows<4>})
+      r = r && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024) ==
+                   cudaSuccess;
+    return r;
+  }();
+  if (!ok) fail(VG_ERR_CUDA, "cannot reserve the rebuild's shared memory");
+  k<<<a.p.nbuckets, BB_TPB, smem, st>>>(a);
+  VG_CUDA(cudaGetLastError());
+}
+
+void build_csr_typed(Sim &s, int e, EdgeAppend &ap) {
+  s.csr_epoch++;
+  const EdgeTypeDesc &ed = s.model->et(e);
+  EdgeStore &es = s.edges[e];
+  cudaStream_t st = s.stream;
+  const int T = ap.target_type;
+  const uint64_t n = ap.fixed_count, nrows = s.agents[T - 1].n;
+  const int nf = ed.stores_payload() ? (int)ed.fields.size() : 0;
+  BuildArgs a{};
+  const bool vals = nf == 0 && ed.stores_src();  // (else a record's slot says where to look)
+  a.p = ap.planned ? ap.plan : plan_buckets(s, e, T, n, vals);
+  if (!es.add_existing)
+    for (int U = 1; U < (int)es.csr.size(); U++)
+      if (U != T && es.csr[U].row_ptr.p) es.csr[U] = CSR();
+  CSR &c = es.csr[T];
+  RebuildCache &rc = *c.rebuild;
+  if (!ap.tiled) {
+    if (a.p.sorted) {
+      // (build_sorted)
+    } else if (vals) {
+      launch_bucket_tiles(SlotSource<true>{ap.to.as<uint32_t>(), ap.from.as<uint32_t>()}, a.p, st);
+    } else {
+      launch_bucket_tiles(SlotSource<false>{ap.to.as<uint32_t>(), nullptr}, a.p, st);
+    }
+    if (!vals) a.slot_src = ap.from.as<uint32_t>();
+  }
+  // without old edges to carry over, the previous container's buffers are
+  // written in place (the stream orders its readers before); otherwise the
+  // two containers take turns
+  const bool merge = es.add_existing && c.row_ptr.p;
+  const uint64_t old_ne = merge ? c.nedges : 0, ne_max = n + old_ne;
+  DevBuf &rp = merge ? rc.row_ptr : c.row_ptr, &src = merge ? rc.src : c.src;
+  std::vector<DevBuf> &pay = merge ? rc.payload : c.payload;
+  ensure_buf(s, rp, (nrows + 1) * 4, merge);
+  if (ed.stores_src()) ensure_buf(s, src, ne_max * 4, true);
+  pay.resize(nf);
+  for (int f = 0; f < nf; f++) ensure_buf(s, pay[f], ne_max * ed.fields[f].size, true);
+  c.src_type.release();
+  a.nrows = nrows;
+  a.span = std::min<uint32_t>(1u << std::min(a.p.shift, 13u), BB_SPAN);
+  a.chunk = a.span >= 2048 ? 1024 : 2048;
+  a.rp = rp.as<uint32_t>();
+  a.src = ed.stores_src() ? src.as<uint32_t>() : nullptr;
+  a.npay = nf;
+  for (int f = 0; f < nf; f++) {
+    a.psize[f] = ed.fields[f].size;
+    a.pin[f] = ap.payload[f].p;
+    a.pout[f] = pay[f].p;
+  }
+  if (merge) {
+    a.old_rp = c.row_ptr.as<uint32_t>();
+    a.old_src = c.src.as<uint32_t>();
+    a.old_nrows = c.nrows;
+    a.old_ne = (uint32_t)old_ne;
+    for (int f = 0; f < nf; f++) a.old_pay[f] = c.payload[f].p;
+  }
+  if (a.p.sorted) build_sorted(s, c, ap, a, merge);
+  else launch_buckets(a, merge, st);
+  uint64_t ne = ne_max;
+  if (ap.holes) {
+    uint32_t h = 0;
+    VG_CUDA(cudaMemcpyAsync(&h, rp.as<uint32_t>() + nrows, 4, cudaMemcpyDeviceToHost, st));
+    VG_CUDA(cudaStreamSynchronize(st));
+    ne = h;
+  }
+  if (merge) {
+    std::swap(c.row_ptr, rc.row_ptr);
+    std::swap(c.src, rc.src);
+    std::swap(c.payload, rc.payload);
+  }
+  if (!ed.stores_src()) c.src.release();
   c.nrows = nrows;
-  c.nedges = n;
+  c.nedges = ne;
   c.src_type_const = ed.stores_src() ? ap.src_type : 0;
   c.max_degree_pending = true;
   c.schedule_valid = false;
   c.unit_grid_weights = -1;
-  return true;
 }
 
 void build_csr_from_records(Sim &s, int e, const uint64_t *d_from,

@@ -141,20 +141,60 @@ struct AgentStore {
   bool readable = false, writeable = false;
 };
 
-// Persistent scratch of the typed rebuild (the per-step edge rebuild from
-// records whose types the emitting kernel declares) and a CUDA graph of its
-// launch sequence: recorded when the same arguments (sizes and buffers)
-// repeat on consecutive rebuilds, replayed while they stay the same.
+// Persistent workspace of the typed rebuild, in its two forms: by buckets
+// (vg_bucket.cuh) and by a radix sort of the rows, whose launch sequence is
+// recorded into a CUDA graph when the same sizes and buffers repeat and
+// replayed while they stay the same; and the previous container's buffers
+// when a rebuild cannot write in place (add_existing): the next one's output
+// goes there.
 struct RebuildCache {
-  DevBuf keys, sort, bstart;
+  DevBuf recs, vals, offs;             // buckets
+  DevBuf keys, sort, bstart, new_rp;   // sort (vals too)
+  DevBuf row_ptr, src;
+  std::vector<DevBuf> payload;
   std::vector<uint64_t> last, graph_args;
   cudaGraphExec_t exec = nullptr;
+  // whether the records are known to fit the buckets' blocks, and for which
+  // sizes; sorted rebuilds are numbered (sort_gen), and those after unknown_gen
+  // report what counts
+  bool known = false;
+  uint64_t known_n = 0, known_rows = 0;
+  uint32_t known_buckets = 0, sort_gen = 0, unknown_gen = 0;
+  void forget() {
+    known = false;
+    unknown_gen = sort_gen;
+  }
   RebuildCache() = default;
   RebuildCache(const RebuildCache &) = delete;
   RebuildCache &operator=(const RebuildCache &) = delete;
   ~RebuildCache() {
     if (exec) cudaGraphExecDestroy(exec);
   }
+};
+
+// Reports of the rebuilds' kernels, in mapped host memory, one per edge type
+// and target type (single stores; the host reads them without waiting).
+struct RebuildReport {
+  unsigned long long load;  // sorted rebuild: its number << 32 | largest bucket
+  unsigned crowded;         // bucket rebuild: some bucket did not fit its block
+  unsigned pad;
+};
+
+// buckets of a typed rebuild (vg_bucket.cuh).  recs: the tiles' records
+// sorted by bucket, a record's row in its bucket in the low `shift` bits and
+// its slot in the tile above; vals: their values in the same places (null: a
+// record's value is its slot); offs: [tile][pitch] number of the tile's
+// records in earlier buckets (entry nbuckets: all its records)
+struct BucketPlan {
+  uint64_t n = 0;
+  uint32_t ntiles = 0, nbuckets = 1, shift = 0, pitch = 4;
+  uint32_t *recs = nullptr, *vals = nullptr;
+  uint16_t *offs = nullptr;
+  unsigned *maxdeg = nullptr;  // the container's largest row length, set to 0 by the tile pass
+  RebuildReport *report = nullptr;
+  uint32_t limit = 0;   // records a bucket's block holds at once
+  bool fits = false;    // the buckets could hold this many records and rows
+  bool sorted = false;  // the sort takes the records instead
 };
 
 struct CSR {
@@ -331,6 +371,7 @@ struct Sim {
   // completion reports of a gather launch: per-range block counters on the
   // device, per-range flags in mapped pinned host memory (the last block of
   // a range writes the call's generation), created on first use
+  RebuildReport *reports_host = nullptr, *reports_dev = nullptr;  // created on first use
   DevBuf xchg_count;
   unsigned *xchg_flags_host = nullptr, *xchg_flags_dev = nullptr;
   unsigned xchg_gen = 0;
@@ -366,10 +407,16 @@ struct EdgeAppend {
   DevBuf counter;  // u64 device counter
   bool ordered = false;  // records already in order-key order
   uint64_t fixed_count = 0;  // when the count is known on the host
-  // declared by kernels whose records are typed by construction: every
-  // target of agent type target_type, every source of type src_type
-  // (0: unknown) -- allows the typed fast rebuild (build_csr_typed)
+  // typed: the records are slots 0 .. fixed_count - 1 in call order, every
+  // target of agent type target_type and every source of type src_type; `to`
+  // holds u32 rows (BK_HOLE: no record) and `from` u32 source indices, `key`
+  // is not used -- the rebuild of build_csr_typed
+  bool typed = false;
   int target_type = 0, src_type = 0;
+  bool holes = false;  // some slots may hold no record
+  bool tiled = false;  // the emitting kernel was the rebuild's tile pass itself (plan)
+  bool planned = false;
+  BucketPlan plan;
 };
 
 // remove_edges! calls recorded by a transition (src/EdgeMethods.jl:527-599):
@@ -407,6 +454,12 @@ struct ApplyCtx {
   // edge records appended by the launchers, per written edge type
   std::vector<std::unique_ptr<EdgeAppend>> appends;
   EdgeAppend *append_for(int edge_type, uint64_t capacity, bool ordered);
+  int ncalls = 0;  // agent types in `call`
+  bool may_die = false;  // the transition can return `nothing`
+  // whether records of `slots` slots into edge_type, all from agents of type
+  // S to agents of type T, may take the typed rebuild
+  bool typed_ok(int edge_type, int T, int S, uint64_t slots) const;
+  EdgeAppend *append_typed(int edge_type, int T, int S, uint64_t slots, bool holes, bool tiled);
   std::vector<std::unique_ptr<EdgeRemoval>> removals;
   EdgeRemoval *removal_for(int edge_type, uint64_t capacity);
 };
@@ -466,10 +519,6 @@ void radix_sort_pairs_u32(uint32_t *keys, uint32_t *vals, uint64_t n,
                           int bits, cudaStream_t st, Sim &s);
 void radix_sort_pairs_u64(uint64_t *keys, uint32_t *vals, uint64_t n,
                           int bits, cudaStream_t st, Sim &s);
-// caller-owned scratch of exclusive_scan_scratch_bytes(n) bytes: no allocation
-uint64_t exclusive_scan_scratch_bytes(uint64_t n);
-void exclusive_scan_u32_in(const uint32_t *in, uint32_t *out, uint64_t n, cudaStream_t st,
-                           int *err, void *scratch);
 // caller-owned scratch of radix_sort_scratch_bytes() bytes: no allocation
 uint64_t radix_sort_scratch_bytes(uint64_t n, int key_size, int bits);
 // counted: the caller has accumulated the digit counts of every pass (8-bit
@@ -494,9 +543,12 @@ void ensure_schedule(Sim &s, CSR &c, uint32_t hub_threshold, uint32_t block_thre
                      uint64_t n);
 // largest row length (synchronises when the value is still on the device)
 uint32_t csr_max_degree(Sim &s, CSR &c);
-// rebuild of an edge type's container from typed, ordered records without
-// host synchronisation; false when the generic build must run
-bool build_csr_typed(Sim &s, int edge_type, const EdgeAppend &ap, uint64_t n);
+// rebuild of an edge type's container from typed records (vg_bucket.cuh); the
+// host waits only to learn the number of edges when slots may be empty
+void build_csr_typed(Sim &s, int edge_type, EdgeAppend &ap);
+// the agents were moved from outside: where records fall is unknown again
+void forget_record_spread(Sim &s);
+BucketPlan plan_buckets(Sim &s, int edge_type, int target_type, uint64_t n, bool vals);
 uint64_t csr_edges_total(const EdgeStore &es);
 
 // agents (vg_api.cu)

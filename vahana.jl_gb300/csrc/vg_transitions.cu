@@ -14,6 +14,7 @@
 #include <map>
 #include <vector>
 
+#include "vg_bucket.cuh"
 #include "vg_internal.h"
 #include "vg_philox.cuh"
 
@@ -223,14 +224,28 @@ __global__ void k_keep(Sweep s) {
 
 // edge appends with an order key (call position, caller index, sequence):
 // the order in which the reference's sequential sweep calls add_edge!.
+// slots: the records' places are known instead (a prefix of the callers'
+// records: all callers' records lie in call order), rows and srcs take the
+// target row and the source, and nothing is counted or keyed.
 struct Append {
   uint64_t *to, *from, *key;
+  uint32_t *rows, *srcs;
   void *payload[MAX_FIELDS];
   int psize[MAX_FIELDS];
   int npayload;
   unsigned long long *counter;
   uint64_t cap;
 };
+
+__device__ __forceinline__ void copy_elem(int size, const void *in, uint64_t i, void *out,
+                                          uint64_t o) {
+  switch (size) {
+    case 1: ((uint8_t *)out)[o] = ((const uint8_t *)in)[i]; break;
+    case 2: ((uint16_t *)out)[o] = ((const uint16_t *)in)[i]; break;
+    case 4: ((uint32_t *)out)[o] = ((const uint32_t *)in)[i]; break;
+    case 8: ((uint64_t *)out)[o] = ((const uint64_t *)in)[i]; break;
+  }
+}
 
 __device__ __forceinline__ uint64_t order_key(int call_pos, uint64_t i,
                                               uint32_t seq) {
@@ -270,12 +285,21 @@ __global__ void k_self_edge(Sweep s, Append ap, int call_pos, const uint8_t *pl)
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = i < s.a.n && sw_begin(s, i);
   if (live && s.writes) sw_copy(s, i);
-  const int64_t k = warp_slot(ap.counter, ap.cap, live, s.status, 301);
-  if (k < 0) return;
-  uint64_t id = ((uint64_t)s.type_nr << SHIFT_TYPE) | (i + 1);
-  ap.to[k] = id;
-  ap.from[k] = id;
-  ap.key[k] = order_key(call_pos, i, 0);
+  int64_t k;
+  if (ap.rows) {
+    if (i >= s.a.n) return;
+    k = (int64_t)i;
+    ap.rows[k] = live ? (uint32_t)i : BK_HOLE;
+    if (!live) return;
+    ap.srcs[k] = (uint32_t)i;
+  } else {
+    k = warp_slot(ap.counter, ap.cap, live, s.status, 301);
+    if (k < 0) return;
+    uint64_t id = ((uint64_t)s.type_nr << SHIFT_TYPE) | (i + 1);
+    ap.to[k] = id;
+    ap.from[k] = id;
+    ap.key[k] = order_key(call_pos, i, 0);
+  }
   int off = 0;
   for (int f = 0; f < ap.npayload; f++) {
     for (int b = 0; b < ap.psize[f]; b++)
@@ -307,6 +331,60 @@ __global__ void k_readd_edges(Sweep s, DevCSRView c, Append ap, int call_pos) {
         ((uint8_t *)ap.payload[f])[k * sz + bb] = ((const uint8_t *)c.payload[f])[(uint64_t)e * sz + bb];
     }
   }
+}
+
+// The in-edges of a warp's 32 rows as one run, 32 consecutive edges at a
+// time: f(e, owner, has) with the edge's number and the lane whose row it is.
+// A lane per row would read and write its own short run, and the longest
+// row of the 32 would set the pace.
+template <class F>
+__device__ __forceinline__ void warp_edges(uint32_t b, uint32_t deg, F f) {
+  const unsigned lane = threadIdx.x & 31;
+  // (rows are consecutive: lane l's run starts where lane l - 1's ends; rows
+  // beyond the container are empty and start at the end)
+  const uint32_t begin = __shfl_sync(FULL_WARP, b, 0);
+  const uint32_t end = __shfl_sync(FULL_WARP, b + deg, 31);
+  for (uint32_t e0 = begin; e0 < end; e0 += 32) {
+    const uint32_t e = e0 + lane;
+    unsigned owner = 0;  // the last lane whose run starts at or before e
+#pragma unroll
+    for (unsigned o = 16; o; o >>= 1) {
+      const uint32_t bo = __shfl_sync(FULL_WARP, b, owner + o);
+      if (bo <= e) owner += o;
+    }
+    f(e, owner, e < end);
+  }
+}
+
+// start and length of row i, for warp_edges
+__device__ __forceinline__ uint32_t row_run(const DevCSRView &c, uint64_t i, uint32_t &deg) {
+  if (i >= c.nrows) {
+    deg = 0;
+    return (uint32_t)c.nedges;
+  }
+  const uint32_t b = c.row_ptr[i];
+  deg = c.row_ptr[i + 1] - b;
+  return b;
+}
+
+// k_readd_edges into slots: edge e of the read container is record e
+__global__ void k_readd_slots(Sweep s, DevCSRView c, Append ap) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = i < s.a.n && sw_begin(s, i);
+  if (live && s.writes) sw_copy(s, i);
+  uint32_t deg;
+  const uint32_t b = row_run(c, i, deg);
+  const unsigned alive = __ballot_sync(FULL_WARP, live);
+  const uint32_t r0 = (uint32_t)(i & ~31ull);
+  warp_edges(b, deg, [&](uint32_t e, unsigned owner, bool has) {
+    if (!has) return;
+    const bool swept = alive >> owner & 1u;
+    ap.rows[e] = swept ? r0 + owner : BK_HOLE;
+    if (!swept) return;
+    ap.srcs[e] = c.src[e];
+    for (int f = 0; f < ap.npayload; f++)
+      copy_elem(ap.psize[f], c.payload[f], e, ap.payload[f], e);
+  });
 }
 
 // remove_edges!: a swept agent keeps its state; mode 0: when its field 0
@@ -429,11 +507,19 @@ __global__ void k_spawn_new(Sweep s, uint64_t n_callers_scope, const uint32_t *f
     if (link_dt < 0) continue;
     const uint64_t nid = ((uint64_t)s.type_nr << SHIFT_TYPE) | nr;
     for (int d = 0; d < 2; d++) {
-      const int64_t k = warp_slot(ap.counter, ap.cap, caller, s.status, 301);
-      if (k < 0) continue;
-      ap.from[k] = d == 0 ? nid : id;
-      ap.to[k] = d == 0 ? id : nid;
-      ap.key[k] = order_key(call_pos, i, 2 * j + d);
+      int64_t k;
+      if (ap.rows) {
+        if (!caller) continue;
+        k = (int64_t)(2 * q + d);
+        ap.rows[k] = (uint32_t)(d == 0 ? i : t);
+        ap.srcs[k] = (uint32_t)(d == 0 ? t : i);
+      } else {
+        k = warp_slot(ap.counter, ap.cap, caller, s.status, 301);
+        if (k < 0) continue;
+        ap.from[k] = d == 0 ? nid : id;
+        ap.to[k] = d == 0 ? id : nid;
+        ap.key[k] = order_key(call_pos, i, 2 * j + d);
+      }
       if (ap.npayload > 0) st_i64(ap.payload[0], link_dt, k, (int64_t)nid);
     }
   }
@@ -479,6 +565,41 @@ __global__ void k_link_neighbors(Sweep s, DevCSRView c, Append ap, int pl_dt, in
   }
 }
 
+// k_link_neighbors into slots: in-edge e of E gives the records 2 e and 2 e + 1
+__global__ void k_link_slots(Sweep s, DevCSRView c, Append ap, int pl_dt, int has_die,
+                             double die_value) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  bool live = i < s.a.n && sw_begin(s, i);
+  const int dt0 = s.fdt[0];
+  const double v = live && s.nfields > 0 ? ld_f64(s.a.rd[0], dt0, i) : 0.0;
+  if (live && has_die && s.nfields > 0 && v == die_value) {
+    if (s.writes) sw_die(s, i);
+    live = false;
+  } else if (live && s.writes) {
+    sw_copy(s, i);
+  }
+  const long long vi = live && s.nfields > 0 ? (long long)ld_i64(s.a.rd[0], dt0, i) : 0;
+  uint32_t deg;
+  const uint32_t b = row_run(c, i, deg);
+  const unsigned alive = __ballot_sync(FULL_WARP, live);
+  const uint32_t r0 = (uint32_t)(i & ~31ull);
+  warp_edges(b, deg, [&](uint32_t e, unsigned owner, bool has) {
+    const double ov = __shfl_sync(FULL_WARP, v, owner);
+    const long long oi = __shfl_sync(FULL_WARP, vi, owner);
+    if (!has) return;
+    const bool swept = alive >> owner & 1u;
+    const uint32_t id = r0 + owner, nid = c.src[e];
+    ((uint2 *)ap.rows)[e] = swept ? make_uint2(id, nid) : make_uint2(BK_HOLE, BK_HOLE);
+    if (!swept) return;
+    ((uint2 *)ap.srcs)[e] = make_uint2(nid, id);
+    if (ap.npayload > 0)
+      for (int d = 0; d < 2; d++) {
+        if (is_float(pl_dt)) st_f64(ap.payload[0], pl_dt, 2ull * e + d, ov);
+        else st_i64(ap.payload[0], pl_dt, 2ull * e + d, oi);
+      }
+  });
+}
+
 // ----------------------------------------------- move_to! in a transition
 // move_to!(sim, raster, id, pos, edge_from_raster, edge_to_raster; distance,
 // metric, periodic, only_surrounding) -- src/Raster.jl:437-477 -- called by
@@ -508,8 +629,9 @@ struct MoveArgs {
   Append from, to;
 };
 
+// slot: the call's place among all agents' calls
 __device__ __forceinline__ void move_emit(const MoveArgs &m, bool want, const int64_t *p,
-                                          uint64_t id, uint64_t key, int *status) {
+                                          uint64_t id, uint64_t slot, uint64_t key, int *status) {
   uint64_t lin = 0, mul = 1;
   for (int d = 0; d < m.ndims; d++) {
     lin += (uint64_t)(p[d] - 1) * mul;
@@ -519,11 +641,24 @@ __device__ __forceinline__ void move_emit(const MoveArgs &m, bool want, const in
   for (int dir = 0; dir < 2; dir++) {
     if (dir == 0 ? !m.has_from : !m.has_to) continue;  // uniform over the launch
     const Append &ap = (dir == 1 && !m.same) ? m.to : m.from;
-    const int64_t k = warp_slot(ap.counter, ap.cap, want, status, 301);
-    if (k < 0) continue;
-    ap.to[k] = dir == 0 ? id : cell;
-    ap.from[k] = dir == 0 ? cell : id;
-    ap.key[k] = key + dir;
+    int64_t k;
+    if (ap.rows) {
+      if (slot == ~0ull) continue;  // no agent
+      k = (int64_t)slot;
+      if (!want) {
+        ap.rows[k] = BK_HOLE;
+        continue;
+      }
+      const uint32_t c32 = (uint32_t)(m.first_nr + lin - 1), a32 = (uint32_t)((id & NR_MASK) - 1);
+      ap.rows[k] = dir == 0 ? a32 : c32;
+      ap.srcs[k] = dir == 0 ? c32 : a32;
+    } else {
+      k = warp_slot(ap.counter, ap.cap, want, status, 301);
+      if (k < 0) continue;
+      ap.to[k] = dir == 0 ? id : cell;
+      ap.from[k] = dir == 0 ? cell : id;
+      ap.key[k] = key + dir;
+    }
     for (int f = 0; f < ap.npayload; f++)  // payload fields zero
       for (int b = 0; b < ap.psize[f]; b++) ((uint8_t *)ap.payload[f])[k * ap.psize[f] + b] = 0;
   }
@@ -561,7 +696,12 @@ __global__ void k_move_to(Sweep s, MoveArgs m, int call_pos) {
     }
   }
   const uint64_t id = ((uint64_t)s.type_nr << SHIFT_TYPE) | (i + 1);
-  if (!m.only_surrounding) move_emit(m, ok, pos, id, order_key(call_pos, i, 0), s.status);
+  const bool agent = i < s.a.n;
+  uint64_t slot = i * (uint64_t)(m.noff + (m.only_surrounding ? 0 : 1));
+  if (!m.only_surrounding) {
+    move_emit(m, ok, pos, id, agent ? slot : ~0ull, order_key(call_pos, i, 0), s.status);
+    slot++;
+  }
   for (int k = 0; k < m.noff; k++) {
     int64_t q[MAX_DIMS] = {1, 1, 1, 1};
     bool in = ok;
@@ -573,7 +713,9 @@ __global__ void k_move_to(Sweep s, MoveArgs m, int call_pos) {
       }
       q[d] = v;
     }
-    move_emit(m, in, q, id, order_key(call_pos, i, 2 * (uint32_t)(k + 1)), s.status);
+    move_emit(m, in, q, id, agent ? slot : ~0ull, order_key(call_pos, i, 2 * (uint32_t)(k + 1)),
+              s.status);
+    slot++;
   }
 }
 
@@ -1077,6 +1219,52 @@ __global__ void k_random_walk(const int32_t *__restrict__ x, const int32_t *__re
           (cell_first_nr + (uint64_t)(nx - 1) + (uint64_t)(ny - 1) * (uint64_t)W);
 }
 
+// The same walk as the rebuild's tile pass: slot i is walker i, whose record
+// goes from its registers into the tile's sort.
+struct WalkSource {
+  static constexpr bool VALS = false;  // the source is the walker, its slot
+  const int32_t *__restrict__ x, *__restrict__ y;
+  int32_t *__restrict__ xo, *__restrict__ yo;
+  int32_t W, H;
+  uint64_t seed;
+  uint32_t step, cell0;  // row of the raster's first cell
+  struct Raw {
+    int32_t x, y;
+  };
+  __device__ __forceinline__ Raw load(uint64_t i) const { return {x[i], y[i]}; }
+  __device__ __forceinline__ bool make(uint64_t i, const Raw &p, uint32_t &row,
+                                       uint32_t &) const {
+    const Philox4 r = philox_draw(seed, i + 1, step, TAG_MOVE);
+    const uint32_t k = bounded32(r.v[0], 8), m = k < 4 ? k : k + 1;
+    const int32_t nx = move1(p.x, (int)(m % 3) - 1, W), ny = move1(p.y, (int)(m / 3) - 1, H);
+    xo[i] = nx;
+    yo[i] = ny;
+    row = cell0 + (uint32_t)(nx - 1) + (uint32_t)(ny - 1) * (uint32_t)W;
+    return true;
+  }
+  // mod1(v + d, n); from a position inside without a division (out of line,
+  // so that the unrolled tile loop stays short)
+  static __device__ __noinline__ int32_t move_far(int32_t v, int d, int32_t n) {
+    const int64_t w = (int64_t)v + d;
+    return (int32_t)(((w - 1) % n + n) % n + 1);
+  }
+  static __device__ __forceinline__ int32_t move1(int32_t v, int d, int32_t n) {
+    if (__builtin_expect((uint32_t)(v - 1) >= (uint32_t)n, 0)) return move_far(v, d, n);
+    const uint32_t u = (uint32_t)(v + d);  // 0 .. n + 1
+    return u == 0 ? n : u > (uint32_t)n ? 1 : (int32_t)u;
+  }
+};
+
+__global__ void k_walk_slots(WalkSource w, uint64_t n, uint32_t *__restrict__ rows,
+                             uint32_t *__restrict__ srcs) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  uint32_t row = 0, unused = 0;
+  w.make(i, w.load(i), row, unused);
+  rows[i] = row;
+  srcs[i] = (uint32_t)i;
+}
+
 // ------------------------------------------------------------- launchers
 Sweep make_sweep(ApplyCtx &c) {
   Sim &s = *c.sim;
@@ -1208,6 +1396,7 @@ void tr_die_if(ApplyCtx &c) {
   }
   Sweep w = make_sweep(c);
   if (w.a.n == 0) return;
+  c.may_die = true;
   k_die_if<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, kind, field, arg, rp2, n2);
   VG_CUDA(cudaGetLastError());
 }
@@ -1231,16 +1420,24 @@ void tr_keep(ApplyCtx &c) {
   VG_CUDA(cudaGetLastError());
 }
 
-Append make_append(ApplyCtx &c, int e, uint64_t cap) {
+// T, S: target and source type of every record, when the call's records have
+// known slots (0 .. cap - 1 in call order; holes: some may stay empty)
+Append make_append(ApplyCtx &c, int e, uint64_t cap, int T = 0, int S = 0, bool holes = false) {
   Sim &s = *c.sim;
   const EdgeTypeDesc &ed = s.model->et(e);
   if (!c.in_write(VG_EDGE(e)) && s.check_readable)
     fail(VG_ERR_ASSERT, ed.name + " must be in the `write` argument of the transition function.");
-  EdgeAppend *a = c.append_for(e, cap, false);
+  const bool typed = T > 0 && S > 0 && c.typed_ok(e, T, S, cap);
+  EdgeAppend *a = typed ? c.append_typed(e, T, S, cap, holes, false) : c.append_for(e, cap, false);
   Append ap{};
-  ap.to = a->to.as<uint64_t>();
-  ap.from = a->from.as<uint64_t>();
-  ap.key = a->key.as<uint64_t>();
+  if (typed) {
+    ap.rows = a->to.as<uint32_t>();
+    ap.srcs = a->from.as<uint32_t>();
+  } else {
+    ap.to = a->to.as<uint64_t>();
+    ap.from = a->from.as<uint64_t>();
+    ap.key = a->key.as<uint64_t>();
+  }
   ap.npayload = (int)a->payload.size();
   for (int f = 0; f < ap.npayload; f++) {
     ap.payload[f] = a->payload[f].p;
@@ -1257,7 +1454,7 @@ void tr_self_edge(ApplyCtx &c) {
   const EdgeTypeDesc &ed = s.model->et(e);
   Sweep w = make_sweep(c);
   if (w.a.n == 0) return;
-  Append ap = make_append(c, e, w.a.n);
+  Append ap = make_append(c, e, w.a.n, c.call_type, c.call_type, w.mortal || w.with_rp);
   // constant payload from params[1..]: one value per field
   std::vector<uint8_t> pl;
   if (ed.stores_payload())
@@ -1288,8 +1485,12 @@ void tr_readd_edges(ApplyCtx &c) {
   Sweep w = make_sweep(c);
   DevCSRView v = csr_view(s, e, c.call_type);
   if (w.a.n == 0) return;
-  Append ap = make_append(c, e, std::max<uint64_t>(v.nedges, 1));
-  k_readd_edges<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap, c.call_pos);
+  // (a died agent has no in-edges: only with_edge leaves rows out)
+  Append ap = v.nedges && v.nrows <= w.a.n
+                  ? make_append(c, e, v.nedges, c.call_type, v.src_type_const, w.with_rp != nullptr)
+                  : make_append(c, e, std::max<uint64_t>(v.nedges, 1));
+  if (ap.rows) k_readd_slots<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap);
+  else k_readd_edges<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap, c.call_pos);
   VG_CUDA(cudaGetLastError());
 }
 
@@ -1370,7 +1571,7 @@ void tr_spawn(ApplyCtx &c) {
   agent_reserve(s, T, n_new);  // may move the columns: take the views after it
   Sweep w2 = make_sweep(c);
   Append ap{};
-  if (link >= 0 && total > 0) ap = make_append(c, link, 2 * total);
+  if (link >= 0 && total > 0) ap = make_append(c, link, 2 * total, T, T);
   if (total > 0)
     k_spawn_new<<<nblk(n), TPB, 0, s.stream>>>(w2, n, flag, pos, g, ap, link >= 0 ? link_dt : -1,
                                                c.call_pos);
@@ -1391,13 +1592,21 @@ void tr_link_neighbors(ApplyCtx &c) {
   Sweep w = make_sweep(c);
   if (w.nfields > 0) require_agent_read(c, c.call_type);
   const int has_die = c.nparams > 2;
+  c.may_die |= has_die != 0;
   const double die_value = c.param(2, 0);
   DevCSRView v = csr_view(s, E, c.call_type);
   if (w.a.n == 0) return;
-  Append ap = make_append(c, F, std::max<uint64_t>(2 * v.nedges, 1));
+  // (with neighbours of the called type every record links it with itself)
+  Append ap = v.nedges && v.nrows <= w.a.n && v.src && v.src_type_const == c.call_type
+                  ? make_append(c, F, 2 * v.nedges, c.call_type, c.call_type,
+                                has_die || w.with_rp != nullptr)
+                  : make_append(c, F, std::max<uint64_t>(2 * v.nedges, 1));
   const int pl_dt = fd.stores_payload() ? fd.fields[0].dtype : -1;
-  k_link_neighbors<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap, pl_dt, has_die, die_value,
-                                                      c.call_pos);
+  if (ap.rows)
+    k_link_slots<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap, pl_dt, has_die, die_value);
+  else
+    k_link_neighbors<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap, pl_dt, has_die, die_value,
+                                                        c.call_pos);
   VG_CUDA(cudaGetLastError());
 }
 
@@ -1613,10 +1822,25 @@ void tr_random_walk(ApplyCtx &c) {
   require_agent_read(c, c.call_type);
   DevAgentView a = agent_view(s, c.call_type);
   if (a.n == 0) return;
+  if (c.typed_ok(e, R.type_nr, c.call_type, a.n) && !s.edges[e].add_existing &&
+      R.dims[0] < (1ll << 31) && R.dims[1] < (1ll << 31)) {
+    const BucketPlan plan = plan_buckets(s, e, R.type_nr, a.n, false);
+    EdgeAppend *ap = c.append_typed(e, R.type_nr, c.call_type, a.n, false, !plan.sorted);
+    ap->plan = plan;
+    ap->planned = true;
+    WalkSource src{(const int32_t *)a.rd[0], (const int32_t *)a.rd[1], (int32_t *)a.wr[0],
+                   (int32_t *)a.wr[1], (int32_t)R.dims[0], (int32_t)R.dims[1], seed,
+                   (uint32_t)c.step, (uint32_t)(R.first_nr - 1)};
+    if (plan.sorted)
+      k_walk_slots<<<nblk(a.n), TPB, 0, s.stream>>>(src, a.n, ap->to.as<uint32_t>(),
+                                                    ap->from.as<uint32_t>());
+    else
+      launch_bucket_tiles(src, plan, s.stream);
+    VG_CUDA(cudaGetLastError());
+    return;
+  }
   EdgeAppend *ap = c.append_for(e, a.n, true);
   ap->fixed_count = a.n;
-  ap->target_type = R.type_nr;  // walker -> cell records, typed by construction
-  ap->src_type = c.call_type;
   k_random_walk<<<nblk(a.n), TPB, 0, s.stream>>>(
       (const int32_t *)a.rd[0], (const int32_t *)a.rd[1], (int32_t *)a.wr[0],
       (int32_t *)a.wr[1], a.n, R.dims[0], R.dims[1], seed, (uint32_t)c.step,
@@ -1679,8 +1903,15 @@ void tr_move_to(ApplyCtx &c) {
   m.has_from = ef >= 0;
   m.has_to = et >= 0;
   m.same = m.has_from && m.has_to && ef == et;
-  if (m.has_from) m.from = make_append(c, ef, std::max<uint64_t>(1, w.a.n * per * (m.same ? 2 : 1)));
-  if (m.has_to && !m.same) m.to = make_append(c, et, std::max<uint64_t>(1, w.a.n * per));
+  // (agents that died and positions beyond a bounded raster leave their slots
+  // empty; a position outside a periodic one is an error, status 204)
+  const bool typed = per > 0 && !m.same;
+  const bool holes = w.mortal || w.with_rp || !m.periodic || mode == 1;
+  const int T = typed ? c.call_type : 0, R_T = typed ? R.type_nr : 0;
+  if (m.has_from)
+    m.from = make_append(c, ef, std::max<uint64_t>(1, w.a.n * per * (m.same ? 2 : 1)), T, R_T, holes);
+  if (m.has_to && !m.same)
+    m.to = make_append(c, et, std::max<uint64_t>(1, w.a.n * per), R_T, T, holes);
   k_move_to<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, m, c.call_pos);
   VG_CUDA(cudaGetLastError());
 }
