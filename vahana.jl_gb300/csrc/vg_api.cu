@@ -96,6 +96,11 @@ void *Sim::scratch(size_t bytes) {
   return d_scratch.p;
 }
 
+void *Sim::work(Work w, size_t bytes) {
+  if (!works[w].p || works[w].bytes < bytes) works[w].alloc(bytes + bytes / 4 + 256, &footprint);
+  return works[w].p;
+}
+
 const void *Sim::const_table(const std::string &key, const void *host, size_t bytes) {
   ConstTable &t = const_tables[key];
   const uint8_t *h = (const uint8_t *)host;

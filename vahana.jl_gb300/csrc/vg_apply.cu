@@ -15,6 +15,7 @@
 #include <type_traits>
 
 #include "vg_internal.h"
+#include "vg_scan.cuh"
 
 namespace vg {
 
@@ -136,22 +137,21 @@ EdgeRemoval *ApplyCtx::removal_for(int e, uint64_t capacity) {
 namespace {
 
 constexpr int TPB = 256;
-inline unsigned nblk(uint64_t n, int tpb = TPB) {
-  uint64_t b = (n + tpb - 1) / tpb;
-  return (unsigned)std::max<uint64_t>(b, 1);
-}
-
-__global__ void k_new_deaths(const uint8_t *died_new, const uint8_t *died_old,
-                             uint64_t n, uint32_t *flag) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) flag[i] = (died_new[i] && !died_old[i]) ? 1u : 0u;
-}
-
-__global__ void k_push_reuse(const uint32_t *flag, const uint32_t *pos, uint64_t n,
-                             uint64_t *stack, uint64_t base) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && flag[i]) stack[base + pos[i]] = i + 1;  // agent numbers, in index order
-}
+// agents that died in this transition, their numbers in index order behind
+// the reuse stack's height (writereuseable, src/AgentMethods.jl:300-345):
+// flags, ranks and the push in one scan
+struct NewDeaths {
+  const uint8_t *now, *before;
+  __device__ __forceinline__ uint32_t operator()(uint64_t i) const {
+    return now[i] && !before[i] ? 1u : 0u;
+  }
+};
+struct PushReuse {
+  uint64_t *top;
+  __device__ __forceinline__ void operator()(uint64_t i, uint32_t rank, uint32_t died) const {
+    if (died) top[rank] = i + 1;
+  }
+};
 
 bool is_edge_ref(int r) { return (r & 0x10000) != 0; }
 int edge_of(int r) { return r & 0xFFFF; }
@@ -748,6 +748,37 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
     ctx.call_pos = pos;
     def->launch(ctx);
   }
+  // the agents that died are collected before the status is read, so that one
+  // wait serves both
+  std::vector<int> may_die_types;
+  std::vector<uint32_t> deaths;
+  if (ctx.may_die)
+    for (int T : C)
+      if (in(ctx.write, T) && !s.model->at(T).immortal() && s.agents[T - 1].n &&
+          std::find(may_die_types.begin(), may_die_types.end(), T) == may_die_types.end())
+        may_die_types.push_back(T);
+  if (!may_die_types.empty()) {
+    deaths.resize(may_die_types.size());
+    uint32_t *totals = (uint32_t *)s.work(Sim::WORK_TOTALS, 256);
+    for (size_t k = 0; k < may_die_types.size(); k++) {
+      AgentStore &a = s.agents[may_die_types[k] - 1];
+      // (no more numbers than agents are ever on the stack)
+      if (a.reuse_cap < a.n) {
+        DevBuf nb;
+        nb.alloc(a.cap * 8, &s.footprint);
+        if (a.nreuse)
+          VG_CUDA(cudaMemcpyAsync(nb.p, a.reuse.p, a.nreuse * 8, cudaMemcpyDeviceToDevice, s.stream));
+        VG_CUDA(cudaStreamSynchronize(s.stream));  // (the old stack is read until here)
+        a.reuse = std::move(nb);
+        a.reuse_cap = a.cap;
+      }
+      scan_map<8, uint32_t>(s, a.n, NewDeaths{a.died_wr.as<uint8_t>(), a.died_rd.as<uint8_t>()},
+                         PushReuse{a.reuse.as<uint64_t>() + a.nreuse}, totals + k);
+    }
+    VG_CUDA(cudaMemcpyAsync(deaths.data(), totals, deaths.size() * 4, cudaMemcpyDeviceToHost,
+                            s.stream));
+    if (s.async) VG_CUDA(cudaStreamSynchronize(s.stream));
+  }
   if (!s.async) check_device_status(s, tname);
 
   // finish_write! of the agent types (src/AgentMethods.jl:300-439)
@@ -759,36 +790,14 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
     std::swap(a.rd, a.wr);
     if (ad.immortal() || a.n == 0) continue;
     std::swap(a.died_rd, a.died_wr);
-    if (!ctx.may_die) continue;  // no agent can have died in this transition
-    // agents that died in this transition, in index order (writereuseable)
-    uint32_t *flag = nullptr, *pos = nullptr;
-    VG_CUDA(cudaMallocAsync((void **)&flag, (a.n + 1) * 4, s.stream));
-    VG_CUDA(cudaMallocAsync((void **)&pos, (a.n + 1) * 4, s.stream));
-    k_new_deaths<<<nblk(a.n), TPB, 0, s.stream>>>(a.died_rd.as<uint8_t>(),
-                                                   a.died_wr.as<uint8_t>(), a.n, flag);
-    VG_CUDA(cudaMemsetAsync(flag + a.n, 0, 4, s.stream));
-    exclusive_scan_u32(flag, pos, a.n + 1, s.stream, s);
-    uint32_t k = 0;
-    VG_CUDA(cudaMemcpyAsync(&k, pos + a.n, 4, cudaMemcpyDeviceToHost, s.stream));
-    VG_CUDA(cudaStreamSynchronize(s.stream));
-    if (k) {
-      if (a.nreuse + k > a.reuse_cap) {
-        uint64_t nc = std::max<uint64_t>(a.nreuse + k, 2 * a.reuse_cap);
-        DevBuf nb;
-        nb.alloc(nc * 8, &s.footprint);
-        if (a.nreuse)
-          VG_CUDA(cudaMemcpyAsync(nb.p, a.reuse.p, a.nreuse * 8, cudaMemcpyDeviceToDevice, s.stream));
-        a.reuse = std::move(nb);
-        a.reuse_cap = nc;
-      }
-      // readreuseable = [readreuseable; writereuseable]
-      k_push_reuse<<<nblk(a.n), TPB, 0, s.stream>>>(flag, pos, a.n, a.reuse.as<uint64_t>(), a.nreuse);
-      a.nreuse += k;
-      a.nliving -= std::min<uint64_t>(a.nliving, k);
-      died_types.push_back(T);
-    }
-    VG_CUDA(cudaFreeAsync(flag, s.stream));
-    VG_CUDA(cudaFreeAsync(pos, s.stream));
+    const auto it = std::find(may_die_types.begin(), may_die_types.end(), T);
+    if (it == may_die_types.end()) continue;  // no agent can have died
+    const uint32_t k = deaths[it - may_die_types.begin()];
+    if (!k) continue;
+    // readreuseable = [readreuseable; writereuseable]
+    a.nreuse += k;
+    a.nliving -= std::min<uint64_t>(a.nliving, k);
+    died_types.push_back(T);
   }
   // edges of the written edge types: new container from the appended
   // records (and the old edges with add_existing)
@@ -824,10 +833,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
                            merge);
   }
   // remove the edges of agents that died (src/AgentMethods.jl:314-345)
-  for (int T : died_types) {
-    AgentStore &a = s.agents[T - 1];
-    remove_died_edges(s, T, a.died_rd.as<uint8_t>(), a.n);
-  }
+  if (!died_types.empty()) remove_died_edges(s, died_types);
   for (auto &a : ctx.appends) s.append_spare[a->edge_type] = std::move(a);
   ctx.appends.clear();
   ctx.removals.clear();

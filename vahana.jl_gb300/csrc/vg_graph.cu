@@ -16,6 +16,8 @@
 
 #include "vg_bucket.cuh"
 #include "vg_internal.h"
+#include "vg_rows.cuh"
+#include "vg_scan.cuh"
 
 namespace vg {
 
@@ -206,24 +208,65 @@ template <class T> struct Tmp {
 };
 
 // ------------------------------------------------------ died-edge removal
-__global__ void k_keep_flags(const uint32_t *rp, uint64_t nrows,
-                             const uint32_t *src, const uint8_t *src_type,
-                             int src_type_const, const uint8_t *died,
-                             uint64_t died_n, int died_type, int target_is_died,
-                             int check_src, uint32_t *keep) {
-  uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrows) return;
-  uint32_t b = rp[r], e = rp[r + 1];
-  bool tdead = target_is_died && r < died_n && died[r];
-  for (uint32_t k = b; k < e; k++) {
-    bool kp = !tdead;
-    if (kp && check_src) {
-      int t = src_type ? src_type[k] : src_type_const;
-      uint32_t sidx = src[k];
-      if (t == died_type && sidx < died_n && died[sidx]) kp = false;
+// an edge stays unless its target or (where sources are kept) its source died
+struct DiedView {
+  const uint8_t *target, *source[MAX_AGENT_TYPES];  // died flags, null: none of them died
+  uint64_t target_n, source_n[MAX_AGENT_TYPES];
+};
+
+__device__ __forceinline__ bool edge_stays(const DevCSRView &c, const DiedView &d, uint32_t e) {
+  if (!c.src) return true;
+  const int t = c.src_type ? (int)c.src_type[e] : c.src_type_const;
+  if (t <= 0 || t >= MAX_AGENT_TYPES || !d.source[t]) return true;
+  const uint32_t s = c.src[e];
+  return s >= d.source_n[t] || !d.source[t][s];
+}
+
+// Edges kept in each row (counts; entry nrows: 0), or, with their exclusive
+// sums new_rp, the kept edges' columns packed.  A warp takes 32 rows' edges as
+// one run (warp_edges), and a group's kept edges by one ballot; they lie one
+// behind the other in the packed container too.
+struct KeptOut {
+  uint32_t *src;
+  uint8_t *src_type;
+  int npay, psize[MAX_FIELDS];
+  void *pay[MAX_FIELDS];
+};
+
+template <bool COPY>
+__global__ void __launch_bounds__(TPB) k_kept_edges(DevCSRView c, DiedView d, uint32_t *counts,
+                                                    const uint32_t *new_rp, KeptOut out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned lane = threadIdx.x & 31;
+  uint32_t deg;
+  const uint32_t b = row_run(c, i, deg);
+  const bool dead = d.target && i < d.target_n && d.target[i];
+  const unsigned live = __ballot_sync(0xffffffffu, !dead);
+  uint32_t kept = 0;
+  const uint64_t row0 = i - lane;
+  uint32_t at = COPY && row0 <= c.nrows ? new_rp[row0] : 0u;
+  warp_edges(b, deg, [&](uint32_t e, unsigned owner, bool has) {
+    const bool keep = has && (live >> owner & 1u) && edge_stays(c, d, e);
+    const unsigned mask = __ballot_sync(0xffffffffu, keep);
+    if (COPY) {
+      if (keep) {
+        const uint32_t o = at + __popc(mask & ((1u << lane) - 1u));
+        if (out.src) out.src[o] = c.src[e];
+        if (out.src_type) out.src_type[o] = c.src_type[e];
+        for (int f = 0; f < out.npay; f++) copy_elem(out.psize[f], c.payload[f], e, out.pay[f], o);
+      }
+      at += __popc(mask);
+    } else {
+      // this lane's row holds the lanes lo .. hi - 1 of the group
+      const uint32_t e0 = e - lane;
+      const uint32_t lo = b > e0 ? min(b - e0, 32u) : 0u;
+      const uint32_t hi = b + deg > e0 ? min(b + deg - e0, 32u) : 0u;
+      const unsigned below_hi = hi >= 32 ? 0xffffffffu : (1u << hi) - 1u;
+      const unsigned below_lo = lo >= 32 ? 0xffffffffu : (1u << lo) - 1u;
+      kept += __popc(mask & below_hi & ~below_lo);
     }
-    keep[k] = kp ? 1u : 0u;
-  }
+  });
+  if (!COPY && i <= c.nrows) counts[i] = i < c.nrows ? kept : 0u;
 }
 
 __global__ void k_new_rowptr(const uint32_t *rp, uint64_t nrows,
@@ -238,6 +281,24 @@ __global__ void k_compact_dest(const uint32_t *keep, const uint32_t *scan,
   if (k < n) dest[k] = keep[k] ? scan[k] : 0xffffffffu;
 }
 
+}  // namespace
+
+static void ensure_buf(Sim &s, DevBuf &b, uint64_t bytes, bool slack = false) {
+  if (b.bytes < bytes || !b.p)
+    b.alloc(std::max<uint64_t>(slack ? bytes + bytes / 8 : bytes, 16), &s.footprint);
+}
+
+namespace {
+struct RowsFrom {
+  const uint32_t *p;
+  __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return p[i]; }
+};
+struct RowsTo {
+  uint32_t *p;
+  __device__ __forceinline__ void operator()(uint64_t i, uint32_t before, uint32_t) const {
+    p[i] = before;
+  }
+};
 }  // namespace
 
 uint64_t csr_edges_total(const EdgeStore &es) {
@@ -315,16 +376,6 @@ __device__ __forceinline__ uint32_t bb_scan(uint32_t v, uint32_t *ws, uint32_t *
   }
   *total = all;
   return before + x - v;
-}
-
-__device__ __forceinline__ void bb_copy(int size, const void *in, uint64_t i, void *out,
-                                        uint64_t o) {
-  switch (size) {
-    case 1: ((uint8_t *)out)[o] = ((const uint8_t *)in)[i]; break;
-    case 2: ((uint16_t *)out)[o] = ((const uint16_t *)in)[i]; break;
-    case 4: ((uint32_t *)out)[o] = ((const uint32_t *)in)[i]; break;
-    case 8: ((uint64_t *)out)[o] = ((const uint64_t *)in)[i]; break;
-  }
 }
 
 // the value of the record q at place i
@@ -571,7 +622,7 @@ __device__ __forceinline__ void bucket_build(const BuildArgs &a, uint32_t span, 
         }
         const uint64_t o = (uint64_t)k + base + cnt[bb_slot<Q>(lo)];
         if (a.src) a.src[o] = a.old_src[k];
-        for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.old_pay[f], k, a.pout[f], o);
+        for (int f = 0; f < a.npay; f++) copy_elem(a.psize[f], a.old_pay[f], k, a.pout[f], o);
       }
     }
     // one record into the container
@@ -583,7 +634,7 @@ __device__ __forceinline__ void bucket_build(const BuildArgs &a, uint32_t span, 
       }
       const uint32_t u = val[j];
       if (a.src) a.src[o] = a.slot_src ? a.slot_src[u] : u;
-      for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.pin[f], u, a.pout[f], o);
+      for (int f = 0; f < a.npay; f++) copy_elem(a.psize[f], a.pin[f], u, a.pout[f], o);
     };
     if (by_warps) {
       // in place order, so that consecutive threads write consecutive edges
@@ -812,7 +863,7 @@ __global__ void __launch_bounds__(BB_TPB, 5) k_bucket_rows(const __grid_constant
     const uint64_t o = (uint64_t)base + k;
     const uint32_t v = byplace[k];
     if (a.src) a.src[o] = a.slot_src ? a.slot_src[v] : v;
-    for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.pin[f], v, a.pout[f], o);
+    for (int f = 0; f < a.npay; f++) copy_elem(a.psize[f], a.pin[f], v, a.pout[f], o);
   }
   unsigned d = dmax;
 #pragma unroll
@@ -999,7 +1050,7 @@ __global__ void k_place_sorted(const uint32_t *keys, const uint32_t *vals, uint6
   if (a.old_rp) o += keys[j] < a.old_nrows ? a.old_rp[keys[j] + 1] : a.old_ne;
   const uint32_t v = vals[j];
   if (a.src) a.src[o] = a.slot_src ? a.slot_src[v] : v;
-  for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.pin[f], v, a.pout[f], o);
+  for (int f = 0; f < a.npay; f++) copy_elem(a.psize[f], a.pin[f], v, a.pout[f], o);
 }
 
 // row pointers of old and new edges together
@@ -1029,7 +1080,7 @@ __global__ void k_merge_old(const uint32_t *new_rp, BuildArgs a) {
   }
   const uint64_t o = k + new_rp[lo];
   if (a.src) a.src[o] = a.old_src[k];
-  for (int f = 0; f < a.npay; f++) bb_copy(a.psize[f], a.old_pay[f], k, a.pout[f], o);
+  for (int f = 0; f < a.npay; f++) copy_elem(a.psize[f], a.old_pay[f], k, a.pout[f], o);
 }
 
 }  // namespace
@@ -1041,11 +1092,6 @@ uint32_t csr_max_degree(Sim &s, CSR &c) {
     c.max_degree_pending = false;
   }
   return c.max_degree;
-}
-
-static void ensure_buf(Sim &s, DevBuf &b, uint64_t bytes, bool slack = false) {
-  if (b.bytes < bytes || !b.p)
-    b.alloc(std::max<uint64_t>(slack ? bytes + bytes / 8 : bytes, 16), &s.footprint);
 }
 
 void forget_record_spread(Sim &s) {
@@ -1538,10 +1584,17 @@ static void compact_csr(Sim &s, const EdgeTypeDesc &ed, CSR &c, const uint32_t *
   c = std::move(n2);
 }
 
-void remove_died_edges(Sim &s, int died_type, const uint8_t *died,
-                       uint64_t died_n) {
+// The rows' kept edges are counted for every affected container before the
+// host learns any total (one wait); containers that lose edges are packed
+// into the buffers of their previous packing, which change places.
+void remove_died_edges(Sim &s, const std::vector<int> &died_types) {
   s.csr_epoch++;
   cudaStream_t st = s.stream;
+  struct Affected {
+    int e, T;
+    DiedView d;
+  };
+  std::vector<Affected> list;
   for (size_t e = 0; e < s.edges.size(); e++) {
     EdgeStore &es = s.edges[e];
     const EdgeTypeDesc &ed = s.model->et((int)e);
@@ -1549,24 +1602,85 @@ void remove_died_edges(Sim &s, int died_type, const uint8_t *died,
     for (int T = 1; T < (int)es.csr.size(); T++) {
       CSR &c = es.csr[T];
       if (c.nedges == 0) continue;
-      bool tgt = (T == died_type);
-      bool srcchk = ed.stores_src() &&
-                    (c.src_type_const == died_type || c.src_type_const < 0);
-      if (!tgt && !srcchk) continue;
-      uint64_t ne = c.nedges;
-      Tmp<uint32_t> keep(ne + 1, st), scan(ne + 1, st);
-      VG_CUDA(cudaMemsetAsync(keep.p + ne, 0, 4, st));
-      k_keep_flags<<<nblk(c.nrows), TPB, 0, st>>>(
-          c.row_ptr.as<uint32_t>(), c.nrows, c.src.as<uint32_t>(),
-          c.src_type.as<uint8_t>(), c.src_type_const, died, died_n, died_type,
-          tgt ? 1 : 0, srcchk ? 1 : 0, keep.p);
-      exclusive_scan_u32(keep.p, scan.p, ne + 1, st, s);
-      uint32_t newtotal = 0;
-      VG_CUDA(cudaMemcpyAsync(&newtotal, scan.p + ne, 4, cudaMemcpyDeviceToHost, st));
-      VG_CUDA(cudaStreamSynchronize(st));
-      if (newtotal == ne) continue;
-      compact_csr(s, ed, c, keep.p, scan.p, newtotal);
+      Affected x{(int)e, T, DiedView{}};
+      bool any = false;
+      for (int D : died_types) {
+        AgentStore &a = s.agents[D - 1];
+        if (T == D) {
+          x.d.target = a.died_rd.as<uint8_t>();
+          x.d.target_n = a.n;
+          any = true;
+        }
+        if (ed.stores_src() && D < MAX_AGENT_TYPES &&
+            (c.src_type_const == D || c.src_type_const < 0)) {
+          x.d.source[D] = a.died_rd.as<uint8_t>();
+          x.d.source_n[D] = a.n;
+          any = true;
+        }
+      }
+      if (any) list.push_back(x);
     }
+  }
+  if (list.empty()) return;
+  uint64_t rows = 0;
+  for (auto &x : list) rows += s.edges[x.e].csr[x.T].nrows + 1;
+  uint32_t *counts = (uint32_t *)s.work(Sim::WORK_ROWS, rows * 4);
+  uint32_t *totals = (uint32_t *)s.work(Sim::WORK_TOTALS, list.size() * 4);
+  uint64_t at = 0;
+  for (size_t k = 0; k < list.size(); k++) {
+    CSR &c = s.edges[list[k].e].csr[list[k].T];
+    k_kept_edges<false><<<nblk(c.nrows + 1), TPB, 0, st>>>(csr_view(s, list[k].e, list[k].T),
+                                                           list[k].d, counts + at, nullptr,
+                                                           KeptOut{});
+    VG_CUDA(cudaGetLastError());
+    scan_map<SCAN_IPT, uint32_t>(s, c.nrows + 1, RowsFrom{counts + at}, RowsTo{counts + at}, totals + k);
+    at += c.nrows + 1;
+  }
+  std::vector<uint32_t> kept(list.size());
+  VG_CUDA(cudaMemcpyAsync(kept.data(), totals, kept.size() * 4, cudaMemcpyDeviceToHost, st));
+  VG_CUDA(cudaStreamSynchronize(st));
+  at = 0;
+  for (size_t k = 0; k < list.size(); k++) {
+    CSR &c = s.edges[list[k].e].csr[list[k].T];
+    const EdgeTypeDesc &ed = s.model->et(list[k].e);
+    const uint32_t *new_rp = counts + at;
+    at += c.nrows + 1;
+    if (kept[k] == c.nedges) continue;
+    if (!c.rebuild) c.rebuild.reset(new RebuildCache());
+    RebuildCache &rc = *c.rebuild;
+    const uint64_t m = std::max<uint64_t>(kept[k], 1);
+    ensure_buf(s, rc.row_ptr, (c.nrows + 1) * 4, true);
+    VG_CUDA(cudaMemcpyAsync(rc.row_ptr.p, new_rp, (c.nrows + 1) * 4, cudaMemcpyDeviceToDevice, st));
+    KeptOut out{};
+    if (c.src.p) {
+      ensure_buf(s, rc.src, m * 4, true);
+      out.src = rc.src.as<uint32_t>();
+    }
+    DevBuf types;
+    if (c.src_type.p) {
+      types.alloc(m, &s.footprint);
+      out.src_type = types.as<uint8_t>();
+    }
+    out.npay = (int)c.payload.size();
+    rc.payload.resize(c.payload.size());
+    for (size_t f = 0; f < c.payload.size(); f++) {
+      out.psize[f] = ed.fields[f].size;
+      ensure_buf(s, rc.payload[f], m * ed.fields[f].size, true);
+      out.pay[f] = rc.payload[f].p;
+    }
+    k_kept_edges<true><<<nblk(c.nrows + 1), TPB, 0, st>>>(csr_view(s, list[k].e, list[k].T),
+                                                          list[k].d, nullptr, new_rp, out);
+    VG_CUDA(cudaGetLastError());
+    std::swap(c.row_ptr, rc.row_ptr);
+    if (c.src.p) std::swap(c.src, rc.src);
+    if (c.src_type.p) {
+      VG_CUDA(cudaStreamSynchronize(st));  // (the old column is freed here)
+      c.src_type = std::move(types);
+    }
+    std::swap(c.payload, rc.payload);
+    c.nedges = kept[k];
+    c.schedule_valid = false;  // (the largest row length stays a bound)
+    c.unit_grid_weights = -1;
   }
 }
 

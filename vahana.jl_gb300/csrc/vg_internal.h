@@ -327,6 +327,11 @@ struct Sim {
   DevBuf d_scratch;
   size_t scratch_bytes = 0;
   void *scratch(size_t bytes);
+  // workspaces of the transitions' passes over agents and rows, kept and
+  // grown: one use at a time each, in stream order
+  enum Work { WORK_SCAN, WORK_ROWS, WORK_TOTALS, WORK_PLACES, WORK_COUNT };
+  DevBuf works[WORK_COUNT];
+  void *work(Work w, size_t bytes);
   // constant tables of the transitions (e.g. infection probabilities per
   // infected-neighbour count), uploaded once per distinct content; the key
   // names the table, the bytes decide whether the copy is current
@@ -535,8 +540,8 @@ void build_csr_from_records(Sim &s, int edge_type, const uint64_t *d_from,
                             const std::vector<const void *> &d_payload,
                             uint64_t n, bool records_sorted_by_key,
                             const uint64_t *d_key, bool merge_existing);
-void remove_died_edges(Sim &s, int died_type, const uint8_t *died_now,
-                       uint64_t n_died);
+// the edges of the agents that died, of the given types
+void remove_died_edges(Sim &s, const std::vector<int> &died_types);
 // hub list and degree-sorted row order over n agent slots (n >= nrows)
 // block_threshold: hub rows above it take a whole block (UINT32_MAX: none)
 void ensure_schedule(Sim &s, CSR &c, uint32_t hub_threshold, uint32_t block_threshold,

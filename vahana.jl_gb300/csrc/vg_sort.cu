@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "vg_internal.h"
+#include "vg_scan.cuh"
 
 namespace vg {
 
@@ -19,39 +20,6 @@ int bits_for(uint64_t maxval) {
 }
 
 namespace {
-
-constexpr int SCAN_TPB = 256;
-constexpr int SCAN_IPT = 16;
-constexpr int SCAN_CHUNK = SCAN_TPB * SCAN_IPT;
-
-template <class T>
-__device__ T block_exclusive_scan(T v, T *warp_sums, T *block_total) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
-  T x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    T y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warp_sums[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    T s = lane < nw ? warp_sums[lane] : T(0);
-    T incl = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      T y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane < nw) warp_sums[lane] = incl - s;
-    if (lane == 31 && block_total) *block_total = incl;
-  }
-  __syncthreads();
-  T r = warp_sums[w] + x - v;
-  __syncthreads();
-  return r;
-}
 
 // The scan of at most one tile (SCAN_CHUNK items) in a single block, plus
 // an optional per-block prefix.  Each thread owns SCAN_IPT consecutive
@@ -79,130 +47,23 @@ __global__ void scan_apply(const T *in, T *out, uint64_t n, const T *prefix) {
   }
 }
 
-// Single-pass exclusive scan over tiles of SCAN_CHUNK items with decoupled
-// look-back (D. Merrill and M. Garland, NVR-2016-002): a tile publishes its
-// total, then warp 0 reads the flags of the 32 preceding tiles at once and
-// adds totals back to the nearest tile whose inclusive prefix is known.
-// Tiles take their index from a ticket counter in start order (a tile only
-// waits for running tiles); every wait is bounded and records an error in
-// *err when it gives up.  In place is allowed (a tile reads all its items
-// before it writes).
-constexpr uint32_t SCAN_SPIN_LIMIT = 1u << 21;
-constexpr int SCAN_ERR_LOOKBACK = 0x5e02;
-
-__device__ __forceinline__ void st_release_u32(uint32_t *a, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *a) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *a) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *a) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
-  return v;
-}
-
+// a column scanned into another or in place (a tile reads all its items
+// before it writes)
 template <class T>
-struct ScanState {
-  uint32_t *flag;  // per tile: 0 nothing, 1 total in agg, 2 inclusive prefix in pre
-  T *agg, *pre;
-  uint32_t *ticket;
+struct ScanFrom {
+  const T *p;
+  __device__ __forceinline__ T operator()(uint64_t i) const { return p[i]; }
+};
+template <class T>
+struct ScanTo {
+  T *p;
+  __device__ __forceinline__ void operator()(uint64_t i, T before, T) const { p[i] = before; }
 };
 
-template <class T>
-__global__ void __launch_bounds__(SCAN_TPB) scan_lookback(const T *in, T *out, uint64_t n,
-                                                          ScanState<T> S, int *err) {
-  __shared__ T ws[32];
-  __shared__ T s_tot, s_excl;
-  __shared__ uint32_t s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(S.ticket, 1u);
-  __syncthreads();
-  const uint32_t tile = s_tile;
-  const uint64_t base = (uint64_t)tile * SCAN_CHUNK + (uint64_t)threadIdx.x * SCAN_IPT;
-  T v[SCAN_IPT];
-  T sum = 0;
-#pragma unroll
-  for (int k = 0; k < SCAN_IPT; k++) {
-    const uint64_t i = base + k;
-    v[k] = i < n ? in[i] : T(0);
-    sum += v[k];
-  }
-  T run = block_exclusive_scan<T>(sum, ws, &s_tot);
-  if (threadIdx.x < 32) {
-    const uint32_t lane = threadIdx.x;
-    const T total = s_tot;
-    T excl = 0;
-    if (tile == 0) {
-      if (lane == 0) {
-        S.pre[0] = total;
-        st_release_u32(S.flag, 2u);
-      }
-    } else {
-      if (lane == 0) {
-        S.agg[tile] = total;
-        st_release_u32(S.flag + tile, 1u);
-      }
-      int64_t t = (int64_t)tile - 1;
-      uint32_t spins = 0;
-      for (;;) {
-        const int64_t tt = t - (int64_t)lane;
-        const uint32_t f = tt >= 0 ? ld_acquire_u32(S.flag + tt) : 2u;
-        const unsigned pm = __ballot_sync(0xffffffffu, f == 2u);
-        const unsigned zm = __ballot_sync(0xffffffffu, f == 0u);
-        const int P = pm ? __ffs(pm) - 1 : 32;  // nearest predecessor with a prefix
-        const unsigned need = P == 32 ? 0xffffffffu : (2u << P) - 1u;
-        if (zm & need) {  // a tile in between has published nothing yet
-          if (++spins > SCAN_SPIN_LIMIT) {
-            if (lane == 0) atomicCAS(err, 0, SCAN_ERR_LOOKBACK);
-            break;
-          }
-          if (spins > 16) __nanosleep(64);
-          continue;
-        }
-        T x = 0;
-        if ((int)lane < P) x = ld_relaxed(S.agg + tt);
-        else if ((int)lane == P && tt >= 0) x = ld_relaxed(S.pre + tt);
-#pragma unroll
-        for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        excl += x;
-        if (P < 32) break;
-        t -= 32;
-        spins = 0;
-      }
-      if (lane == 0) {
-        S.pre[tile] = excl + total;
-        st_release_u32(S.flag + tile, 2u);
-      }
-    }
-    if (lane == 0) s_excl = excl;
-  }
-  __syncthreads();
-  run += s_excl;
-#pragma unroll
-  for (int k = 0; k < SCAN_IPT; k++) {
-    const uint64_t i = base + k;
-    if (i < n) out[i] = run;
-    run += v[k];
-  }
-}
-
-template <class T>
-uint64_t scan_scratch_bytes(uint64_t n) {
-  const uint64_t nt = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-  return 64 + nt * 4 + 2 * nt * sizeof(T) + 64;
-}
-
-// scratch: null (allocated on the stream) or scan_scratch_bytes<T>(n) bytes
+// scratch: scan_scratch_bytes<T>(n) bytes (not read for one tile)
 template <class T>
 void exclusive_scan_impl(const T *in, T *out, uint64_t n, cudaStream_t st, int *err,
-                         void *scratch = nullptr) {
+                         void *scratch) {
   if (n == 0) return;
   const uint64_t nt = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
   if (nt == 1) {
@@ -210,20 +71,10 @@ void exclusive_scan_impl(const T *in, T *out, uint64_t n, cudaStream_t st, int *
     VG_CUDA(cudaGetLastError());
     return;
   }
-  if (nt >= (1ull << 31)) fail(VG_ERR_NOMEM, "scan: too many items");
-  char *buf = (char *)scratch;
-  const uint64_t bytes = scan_scratch_bytes<T>(n);
-  if (!buf) VG_CUDA(cudaMallocAsync((void **)&buf, bytes, st));
-  ScanState<T> S;
-  S.ticket = (uint32_t *)buf;
-  S.flag = (uint32_t *)(buf + 64);
-  const uint64_t aoff = (64 + nt * 4 + 15) & ~15ull;
-  S.agg = (T *)(buf + aoff);
-  S.pre = S.agg + nt;
-  VG_CUDA(cudaMemsetAsync(buf, 0, 64 + nt * 4, st));
-  scan_lookback<T><<<(unsigned)nt, SCAN_TPB, 0, st>>>(in, out, n, S, err);
+  const ScanState<T> S = scan_state<T>(scratch, n, st);
+  k_scan_map<SCAN_IPT, T><<<(unsigned)nt, SCAN_TPB, 0, st>>>(ScanFrom<T>{in}, ScanTo<T>{out}, n, (T *)nullptr,
+                                                   S, err);
   VG_CUDA(cudaGetLastError());
-  if (!scratch) VG_CUDA(cudaFreeAsync(buf, st));
 }
 
 // ------------------------------------------------------------ radix sort
@@ -554,20 +405,15 @@ void radix_sort_impl(K *keys, uint32_t *vals, uint64_t n, int bits, cudaStream_t
 
 void exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint64_t n,
                         cudaStream_t st, Sim &s) {
-  exclusive_scan_impl<uint32_t>(in, out, n, st, s.d_status.as<int>());
+  exclusive_scan_impl<uint32_t>(in, out, n, st, s.d_status.as<int>(),
+                                s.work(Sim::WORK_SCAN, scan_scratch_bytes<uint32_t>(n)));
 }
 void exclusive_scan_u64(const uint64_t *in, uint64_t *out, uint64_t n,
                         cudaStream_t st, Sim &s) {
   exclusive_scan_impl<unsigned long long>((const unsigned long long *)in,
-                                          (unsigned long long *)out, n, st,
-                                          s.d_status.as<int>());
-}
-uint64_t exclusive_scan_scratch_bytes(uint64_t n) {
-  return scan_scratch_bytes<uint32_t>(n);
-}
-void exclusive_scan_u32_in(const uint32_t *in, uint32_t *out, uint64_t n, cudaStream_t st,
-                           int *err, void *scratch) {
-  exclusive_scan_impl<uint32_t>(in, out, n, st, err, scratch);
+                                          (unsigned long long *)out, n, st, s.d_status.as<int>(),
+                                          s.work(Sim::WORK_SCAN,
+                                                 scan_scratch_bytes<unsigned long long>(n)));
 }
 void radix_sort_pairs_u32(uint32_t *keys, uint32_t *vals, uint64_t n, int bits,
                           cudaStream_t st, Sim &s) {
@@ -708,7 +554,8 @@ extern "C" int vg_selftest_scan_timeout(int *status_out, double *ms_out) {
     VG_CUDA(cudaEventCreate(&e0));
     VG_CUDA(cudaEventCreate(&e1));
     VG_CUDA(cudaEventRecord(e0, st));
-    scan_lookback<uint32_t><<<(unsigned)(nt - 1), SCAN_TPB, 0, st>>>(din, dout, n, S, derr);
+    k_scan_map<SCAN_IPT, uint32_t><<<(unsigned)(nt - 1), SCAN_TPB, 0, st>>>(
+        ScanFrom<uint32_t>{din}, ScanTo<uint32_t>{dout}, n, (uint32_t *)nullptr, S, derr);
     VG_CUDA(cudaGetLastError());
     VG_CUDA(cudaEventRecord(e1, st));
     VG_CUDA(cudaStreamSynchronize(st));
@@ -757,13 +604,15 @@ extern "C" int vg_selftest_scan(uint64_t n, int wide, int in_place, uint64_t see
                        cudaMemcpyHostToDevice));
     cudaStream_t st;
     VG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    void *o = in_place ? din : dout;
+    void *o = in_place ? din : dout, *scratch = nullptr;
+    VG_CUDA(cudaMalloc(&scratch, scan_scratch_bytes<unsigned long long>(n)));
     if (wide)
       exclusive_scan_impl<unsigned long long>((const unsigned long long *)din,
-                                              (unsigned long long *)o, n, st, derr);
+                                              (unsigned long long *)o, n, st, derr, scratch);
     else
-      exclusive_scan_impl<uint32_t>((const uint32_t *)din, (uint32_t *)o, n, st, derr);
+      exclusive_scan_impl<uint32_t>((const uint32_t *)din, (uint32_t *)o, n, st, derr, scratch);
     VG_CUDA(cudaStreamSynchronize(st));
+    VG_CUDA(cudaFree(scratch));
     std::vector<unsigned long long> r(n);
     std::vector<uint32_t> r32(wide ? 0 : n);
     int herr = 0;

@@ -17,6 +17,8 @@
 #include "vg_bucket.cuh"
 #include "vg_internal.h"
 #include "vg_philox.cuh"
+#include "vg_rows.cuh"
+#include "vg_scan.cuh"
 
 namespace vg {
 
@@ -237,16 +239,6 @@ struct Append {
   uint64_t cap;
 };
 
-__device__ __forceinline__ void copy_elem(int size, const void *in, uint64_t i, void *out,
-                                          uint64_t o) {
-  switch (size) {
-    case 1: ((uint8_t *)out)[o] = ((const uint8_t *)in)[i]; break;
-    case 2: ((uint16_t *)out)[o] = ((const uint16_t *)in)[i]; break;
-    case 4: ((uint32_t *)out)[o] = ((const uint32_t *)in)[i]; break;
-    case 8: ((uint64_t *)out)[o] = ((const uint64_t *)in)[i]; break;
-  }
-}
-
 __device__ __forceinline__ uint64_t order_key(int call_pos, uint64_t i,
                                               uint32_t seq) {
   return ((uint64_t)call_pos << 60) | ((i & ((1ull << 40) - 1)) << 20) | seq;
@@ -331,40 +323,6 @@ __global__ void k_readd_edges(Sweep s, DevCSRView c, Append ap, int call_pos) {
         ((uint8_t *)ap.payload[f])[k * sz + bb] = ((const uint8_t *)c.payload[f])[(uint64_t)e * sz + bb];
     }
   }
-}
-
-// The in-edges of a warp's 32 rows as one run, 32 consecutive edges at a
-// time: f(e, owner, has) with the edge's number and the lane whose row it is.
-// A lane per row would read and write its own short run, and the longest
-// row of the 32 would set the pace.
-template <class F>
-__device__ __forceinline__ void warp_edges(uint32_t b, uint32_t deg, F f) {
-  const unsigned lane = threadIdx.x & 31;
-  // (rows are consecutive: lane l's run starts where lane l - 1's ends; rows
-  // beyond the container are empty and start at the end)
-  const uint32_t begin = __shfl_sync(FULL_WARP, b, 0);
-  const uint32_t end = __shfl_sync(FULL_WARP, b + deg, 31);
-  for (uint32_t e0 = begin; e0 < end; e0 += 32) {
-    const uint32_t e = e0 + lane;
-    unsigned owner = 0;  // the last lane whose run starts at or before e
-#pragma unroll
-    for (unsigned o = 16; o; o >>= 1) {
-      const uint32_t bo = __shfl_sync(FULL_WARP, b, owner + o);
-      if (bo <= e) owner += o;
-    }
-    f(e, owner, e < end);
-  }
-}
-
-// start and length of row i, for warp_edges
-__device__ __forceinline__ uint32_t row_run(const DevCSRView &c, uint64_t i, uint32_t &deg) {
-  if (i >= c.nrows) {
-    deg = 0;
-    return (uint32_t)c.nedges;
-  }
-  const uint32_t b = c.row_ptr[i];
-  deg = c.row_ptr[i + 1] - b;
-  return b;
 }
 
 // k_readd_edges into slots: edge e of the read container is record e
@@ -469,22 +427,31 @@ struct SpawnArgs {
   uint64_t n_old;         // nextid - 1 before the transition
 };
 
-__global__ void k_spawn_flags(Sweep s, uint32_t *flag) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.a.n) return;
-  bool swept = sw_begin(s, i);
-  flag[i] = swept ? 1u : 0u;
-  if (swept && s.writes) sw_copy(s, i);
-}
+// item i: 1 for a caller, which keeps its state on the way; its rank is the
+// callers before it (BK_HOLE for the others)
+struct SpawnCallers {
+  Sweep s;
+  __device__ __forceinline__ uint32_t operator()(uint64_t i) const {
+    const bool swept = sw_begin(s, i);
+    if (swept && s.writes) sw_copy(s, i);
+    return swept ? 1u : 0u;
+  }
+};
+struct SpawnRanks {
+  uint32_t *rank;
+  __device__ __forceinline__ void operator()(uint64_t i, uint32_t before, uint32_t is) const {
+    rank[i] = is ? before : BK_HOLE;
+  }
+};
 
-__global__ void k_spawn_new(Sweep s, uint64_t n_callers_scope, const uint32_t *flag,
-                            const uint32_t *pos, SpawnArgs g, Append ap, int link_dt,
-                            int call_pos) {
+__global__ void k_spawn_new(Sweep s, uint64_t n_callers_scope, const uint32_t *rank, SpawnArgs g,
+                            Append ap, int link_dt, int call_pos) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool caller = i < n_callers_scope && flag[i];
+  const uint32_t mine = i < n_callers_scope ? rank[i] : BK_HOLE;
+  const bool caller = mine != BK_HOLE;
   const uint64_t id = ((uint64_t)s.type_nr << SHIFT_TYPE) | (i + 1);
   for (int j = 0; j < g.k; j++) {
-    const uint64_t q = caller ? (uint64_t)pos[i] * g.k + j : 0;
+    const uint64_t q = caller ? (uint64_t)mine * g.k + j : 0;
     const uint64_t nr = !caller ? 0
                         : q < g.take ? g.reuse[g.nreuse - 1 - q] : g.n_old + 1 + (q - g.take);
     const uint64_t t = nr - 1;
@@ -1551,15 +1518,11 @@ void tr_spawn(ApplyCtx &c) {
   Sweep w = make_sweep(c);
   const uint64_t n = w.a.n;
   if (n == 0) return;
-  uint32_t *flag = nullptr, *pos = nullptr;
-  VG_CUDA(cudaMallocAsync((void **)&flag, (n + 1) * 4, s.stream));
-  VG_CUDA(cudaMallocAsync((void **)&pos, (n + 1) * 4, s.stream));
-  k_spawn_flags<<<nblk(n), TPB, 0, s.stream>>>(w, flag);
-  VG_CUDA(cudaGetLastError());
-  VG_CUDA(cudaMemsetAsync(flag + n, 0, 4, s.stream));
-  exclusive_scan_u32(flag, pos, n + 1, s.stream, s);
+  uint32_t *rank = (uint32_t *)s.work(Sim::WORK_PLACES, n * 4);
+  uint32_t *callers = (uint32_t *)s.work(Sim::WORK_TOTALS, 256);
+  scan_map<4, uint32_t>(s, n, SpawnCallers{w}, SpawnRanks{rank}, callers);
   uint32_t m = 0;
-  VG_CUDA(cudaMemcpyAsync(&m, pos + n, 4, cudaMemcpyDeviceToHost, s.stream));
+  VG_CUDA(cudaMemcpyAsync(&m, callers, 4, cudaMemcpyDeviceToHost, s.stream));
   VG_CUDA(cudaStreamSynchronize(s.stream));
   AgentStore &a = s.agents[T - 1];
   const uint64_t total = (uint64_t)m * k;
@@ -1573,11 +1536,9 @@ void tr_spawn(ApplyCtx &c) {
   Append ap{};
   if (link >= 0 && total > 0) ap = make_append(c, link, 2 * total, T, T);
   if (total > 0)
-    k_spawn_new<<<nblk(n), TPB, 0, s.stream>>>(w2, n, flag, pos, g, ap, link >= 0 ? link_dt : -1,
+    k_spawn_new<<<nblk(n), TPB, 0, s.stream>>>(w2, n, rank, g, ap, link >= 0 ? link_dt : -1,
                                                c.call_pos);
   VG_CUDA(cudaGetLastError());
-  VG_CUDA(cudaFreeAsync(flag, s.stream));
-  VG_CUDA(cudaFreeAsync(pos, s.stream));
   a.nreuse = g.nreuse - g.take;
   a.n = n_new;
   a.nliving += total;
