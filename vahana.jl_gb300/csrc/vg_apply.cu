@@ -600,8 +600,7 @@ void run_reduce(Sim &s, RedArgs a, int out_dtype, bool ordered, void *out) {
     }
     VG_CUDA(cudaGetLastError());
     int64_t res[2];
-    VG_CUDA(cudaMemcpyAsync(res, d, 16, cudaMemcpyDeviceToHost, s.stream));
-    VG_CUDA(cudaStreamSynchronize(s.stream));
+    s.fetch(res, d, 16);
     ri = res[0];
     std::memcpy(&rf, &res[1], 8);
   }
@@ -775,9 +774,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
       scan_map<8, uint32_t>(s, a.n, NewDeaths{a.died_wr.as<uint8_t>(), a.died_rd.as<uint8_t>()},
                          PushReuse{a.reuse.as<uint64_t>() + a.nreuse}, totals + k);
     }
-    VG_CUDA(cudaMemcpyAsync(deaths.data(), totals, deaths.size() * 4, cudaMemcpyDeviceToHost,
-                            s.stream));
-    if (s.async) VG_CUDA(cudaStreamSynchronize(s.stream));
+    s.fetch(deaths.data(), totals, deaths.size() * 4);
   }
   if (!s.async) check_device_status(s, tname);
 
@@ -816,8 +813,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
       if (ap->ordered) {
         n = ap->fixed_count;
       } else {
-        VG_CUDA(cudaMemcpyAsync(&n, ap->counter.p, 8, cudaMemcpyDeviceToHost, s.stream));
-        VG_CUDA(cudaStreamSynchronize(s.stream));
+        s.fetch(&n, ap->counter.p, 8);
       }
       if (n > ap->cap) fail(VG_ERR_DEVICE, "edge append buffer overflow");
     }

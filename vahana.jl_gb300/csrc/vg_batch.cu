@@ -539,6 +539,8 @@ void sir_initial_state(uint64_t n, uint64_t seed, uint64_t n_inf, std::vector<ui
 
 using namespace vg;
 
+constexpr size_t READ_BOUNCE = 1 << 20;
+
 struct vg_batch {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -575,6 +577,7 @@ struct vg_batch {
   int c_ctas = 8, c_tpb = 512, c_ilp = 1;
   std::map<int, ClusterPlan> cplans;
   std::vector<uint64_t> host_base;  // first arena agent of each instance
+  char *bounce = nullptr;           // READ_BOUNCE pinned bytes that states are read through
   int form = 1;  // mode 3 runs: 1 graph replay, 2 persistent grid, 4 persistent clusters
   float tuned_graph_ms = 0, tuned_persistent_ms = 0, tuned_cluster_ms = 0;  // best trials
   std::vector<uint32_t> host_rp;       // arena row pointers (autotuner, buckets)
@@ -1332,14 +1335,33 @@ int vg_batch_read_states2(vg_batch *b, int i, int which, uint8_t *state_out,
   }
   if (which != 0) fail(VG_ERR_ARG, "batch: which 0 (the arena) or 1 (the instance's simulation)");
   need(n_out, "count pointer");
-  uint64_t a0 = 0;
-  for (int j = 0; j < i; j++) a0 += (uint64_t)b->N[j];
+  const uint64_t a0 = b->host_base[i];
   uint64_t Ni = (uint64_t)b->N[i];
   *n_out = Ni;
   uint64_t m = std::min(cap, Ni);
+  // through pinned memory where it fits: both copies queue behind the steps
+  // and one wait ends them; a copy to pageable memory waits by itself, twice
+  // an instance
+  if (!b->bounce && m * 5 <= READ_BOUNCE) {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, READ_BOUNCE, cudaHostAllocDefault) == cudaSuccess)
+      b->bounce = (char *)p;
+    else
+      cudaGetLastError();
+  }
+  char *via = m * 5 <= READ_BOUNCE ? b->bounce : nullptr;
+  void *days = via ? (void *)via : days_out, *states = via ? (void *)(via + m * 4) : state_out;
+  if (days_out)
+    VG_CUDA(cudaMemcpyAsync(days, b->dy[b->cur].as<int32_t>() + a0, m * 4, cudaMemcpyDeviceToHost,
+                            b->stream));
+  if (state_out)
+    VG_CUDA(cudaMemcpyAsync(states, b->st[b->cur].as<uint8_t>() + a0, m, cudaMemcpyDeviceToHost,
+                            b->stream));
   VG_CUDA(cudaStreamSynchronize(b->stream));
-  if (state_out) VG_CUDA(cudaMemcpy(state_out, b->st[b->cur].as<uint8_t>() + a0, m, cudaMemcpyDeviceToHost));
-  if (days_out) VG_CUDA(cudaMemcpy(days_out, b->dy[b->cur].as<int32_t>() + a0, m * 4, cudaMemcpyDeviceToHost));
+  if (via) {
+    if (days_out) std::memcpy(days_out, days, m * 4);
+    if (state_out) std::memcpy(state_out, states, m);
+  }
   API_END
 }
 
@@ -1513,6 +1535,7 @@ int vg_batch_destroy(vg_batch *b) {
       cudaGraphDestroy(b->graph_def[p]);
     }
   for (auto *s : b->sims) vg_sim_destroy(s);
+  if (b->bounce) cudaFreeHost(b->bounce);
   if (b->model) vg_model_destroy(b->model);
   cudaStream_t st = b->stream;
   bool own = b->own_stream;

@@ -1087,8 +1087,7 @@ __global__ void k_merge_old(const uint32_t *new_rp, BuildArgs a) {
 
 uint32_t csr_max_degree(Sim &s, CSR &c) {
   if (c.max_degree_pending) {
-    VG_CUDA(cudaMemcpyAsync(&c.max_degree, c.d_max_degree.p, 4, cudaMemcpyDeviceToHost, s.stream));
-    VG_CUDA(cudaStreamSynchronize(s.stream));
+    s.fetch(&c.max_degree, c.d_max_degree.p, 4);
     c.max_degree_pending = false;
   }
   return c.max_degree;
@@ -1359,8 +1358,7 @@ void build_csr_typed(Sim &s, int e, EdgeAppend &ap) {
   uint64_t ne = ne_max;
   if (ap.holes) {
     uint32_t h = 0;
-    VG_CUDA(cudaMemcpyAsync(&h, rp.as<uint32_t>() + nrows, 4, cudaMemcpyDeviceToHost, st));
-    VG_CUDA(cudaStreamSynchronize(st));
+    s.fetch(&h, rp.as<uint32_t>() + nrows, 4);
     ne = h;
   }
   if (merge) {
@@ -1637,8 +1635,7 @@ void remove_died_edges(Sim &s, const std::vector<int> &died_types) {
     at += c.nrows + 1;
   }
   std::vector<uint32_t> kept(list.size());
-  VG_CUDA(cudaMemcpyAsync(kept.data(), totals, kept.size() * 4, cudaMemcpyDeviceToHost, st));
-  VG_CUDA(cudaStreamSynchronize(st));
+  s.fetch(kept.data(), totals, kept.size() * 4);
   at = 0;
   for (size_t k = 0; k < list.size(); k++) {
     CSR &c = s.edges[list[k].e].csr[list[k].T];

@@ -323,13 +323,18 @@ struct Sim {
   std::map<std::string, double> params, globals;
   std::map<std::string, std::vector<double>> global_series;
   // scratch
-  DevBuf d_status;  // int32 device error word
+  DevBuf d_status;  // StatusWord: the kernels' first error
+  // a line of mapped pinned host memory (null: none was free): the status
+  // word's host copy, then PIN_BYTES - 64 bytes that fetch() reads through
+  char *pin = nullptr;
+  // a few bytes of device memory, after all work queued so far
+  void fetch(void *dst, const void *src, size_t bytes);
   DevBuf d_scratch;
   size_t scratch_bytes = 0;
   void *scratch(size_t bytes);
   // workspaces of the transitions' passes over agents and rows, kept and
   // grown: one use at a time each, in stream order
-  enum Work { WORK_SCAN, WORK_ROWS, WORK_TOTALS, WORK_PLACES, WORK_COUNT };
+  enum Work { WORK_SCAN, WORK_ROWS, WORK_TOTALS, WORK_PLACES, WORK_READ, WORK_COUNT };
   DevBuf works[WORK_COUNT];
   void *work(Work w, size_t bytes);
   // constant tables of the transitions (e.g. infection probabilities per
@@ -384,6 +389,26 @@ struct Sim {
 };
 
 // ---------------------------------------------------------------- kernels
+// A simulation's error word: kernels keep the first code that is reported and
+// store it in mapped host memory too, where the host reads it after a wait
+// for the stream -- a check costs no copy.
+struct StatusWord {
+  int code, pad;
+  int *host;  // may be null
+};
+constexpr size_t PIN_BYTES = 256;
+#ifdef __CUDACC__
+__device__ __forceinline__ void report_status(int *status, int code) {
+  if (atomicCAS(status, 0, code) == 0) {
+    int *host = ((StatusWord *)status)->host;
+    if (host) {
+      *(volatile int *)host = code;
+      __threadfence_system();
+    }
+  }
+}
+#endif
+
 // Views passed to kernels by value.
 struct DevAgentView {
   uint64_t n;

@@ -485,7 +485,7 @@ __device__ __noinline__ void hub_block(const OpinionArgs &p, uint32_t r) {
   uint32_t k = 0;
   for (; k < nch; k++) {
     if (!mbar_wait(&bar[k & 1], (k >> 1) & 1u)) {
-      atomicCAS(p.status, 0, HB_ERR_WAIT);
+      report_status(p.status, HB_ERR_WAIT);
       failed = 1;
     }
     __syncthreads();

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(SCAN_TPB) k_scan_map(In in, Out out, uint64_t 
         const unsigned need = P == 32 ? 0xffffffffu : (2u << P) - 1u;
         if (zm & need) {  // a tile in between has published nothing yet
           if (++spins > SCAN_SPIN_LIMIT) {
-            if (lane == 0) atomicCAS(err, 0, SCAN_ERR_LOOKBACK);
+            if (lane == 0) report_status(err, SCAN_ERR_LOOKBACK);
             break;
           }
           if (spins > 16) __nanosleep(64);

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(RS_TPB, 1) rs_pass(const K *kin, const uint32_
         spins = 0;
       } else {
         if (++spins > RS_SPIN_LIMIT) {
-          atomicCAS(err, 0, RS_ERR_LOOKBACK);
+          report_status(err, RS_ERR_LOOKBACK);
           break;
         }
         if (spins > 16) __nanosleep(64);
@@ -472,8 +472,8 @@ extern "C" int vg_selftest_sort(uint64_t n, int key_bits, int wide, int const_lo
     int *derr = nullptr;
     VG_CUDA(cudaMalloc(&dk, std::max<uint64_t>(n, 1) * 8));
     VG_CUDA(cudaMalloc(&dv, std::max<uint64_t>(n, 1) * 4));
-    VG_CUDA(cudaMalloc(&derr, 4));
-    VG_CUDA(cudaMemset(derr, 0, 4));
+    VG_CUDA(cudaMalloc(&derr, sizeof(StatusWord)));
+    VG_CUDA(cudaMemset(derr, 0, sizeof(StatusWord)));
     std::vector<uint32_t> k32(wide ? 0 : n);
     for (uint64_t i = 0; i < k32.size(); i++) k32[i] = (uint32_t)k[i];
     if (wide)
@@ -534,11 +534,11 @@ extern "C" int vg_selftest_scan_timeout(int *status_out, double *ms_out) {
     const uint64_t bytes = scan_scratch_bytes<uint32_t>(n);
     VG_CUDA(cudaMalloc(&din, n * 4));
     VG_CUDA(cudaMalloc(&dout, n * 4));
-    VG_CUDA(cudaMalloc(&derr, 4));
+    VG_CUDA(cudaMalloc(&derr, sizeof(StatusWord)));
     VG_CUDA(cudaMalloc(&buf, bytes));
     VG_CUDA(cudaMemset(din, 0, n * 4));
     VG_CUDA(cudaMemset(dout, 0, n * 4));
-    VG_CUDA(cudaMemset(derr, 0, 4));
+    VG_CUDA(cudaMemset(derr, 0, sizeof(StatusWord)));
     VG_CUDA(cudaMemset(buf, 0, bytes));
     const uint32_t first_ticket = 1;
     VG_CUDA(cudaMemcpy(buf, &first_ticket, 4, cudaMemcpyHostToDevice));
@@ -598,8 +598,8 @@ extern "C" int vg_selftest_scan(uint64_t n, int wide, int in_place, uint64_t see
     int *derr = nullptr;
     VG_CUDA(cudaMalloc(&din, std::max<uint64_t>(n, 1) * es));
     VG_CUDA(cudaMalloc(&dout, std::max<uint64_t>(n, 1) * es));
-    VG_CUDA(cudaMalloc(&derr, 4));
-    VG_CUDA(cudaMemset(derr, 0, 4));
+    VG_CUDA(cudaMalloc(&derr, sizeof(StatusWord)));
+    VG_CUDA(cudaMemset(derr, 0, sizeof(StatusWord)));
     VG_CUDA(cudaMemcpy(din, wide ? (const void *)h.data() : (const void *)h32.data(), n * es,
                        cudaMemcpyHostToDevice));
     cudaStream_t st;

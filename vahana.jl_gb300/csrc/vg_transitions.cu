@@ -31,7 +31,7 @@ inline unsigned nblk(uint64_t n, int tpb = TPB) {
 }
 
 __device__ __forceinline__ void set_status(int *st, int code) {
-  atomicCAS(st, 0, code);
+  report_status(st, code);
 }
 
 // ----------------------------------------------------------- field access
@@ -1522,8 +1522,7 @@ void tr_spawn(ApplyCtx &c) {
   uint32_t *callers = (uint32_t *)s.work(Sim::WORK_TOTALS, 256);
   scan_map<4, uint32_t>(s, n, SpawnCallers{w}, SpawnRanks{rank}, callers);
   uint32_t m = 0;
-  VG_CUDA(cudaMemcpyAsync(&m, callers, 4, cudaMemcpyDeviceToHost, s.stream));
-  VG_CUDA(cudaStreamSynchronize(s.stream));
+  s.fetch(&m, callers, 4);
   AgentStore &a = s.agents[T - 1];
   const uint64_t total = (uint64_t)m * k;
   g.nreuse = ad.immortal() ? 0 : a.nreuse;

@@ -348,8 +348,17 @@ def add_agent_per_process(sim, T, **fields):
     return np.uint64(out.value)
 
 
+def _zeros(n, dtype):
+    """Zeros the processor has touched: a device copy into pages that exist
+    only as promises (np.zeros) is served one page fault after the other,
+    5 ms for 16 MB against 0.4 ms for touching and copying."""
+    a = np.empty(n, dtype=dtype)
+    a.fill(0)
+    return a
+
+
 def _empty_cols(t, n):
-    cols = [np.zeros(n, dtype=NP_DTYPES[dt]) for _, dt in t.fields]
+    cols = [_zeros(n, NP_DTYPES[dt]) for _, dt in t.fields]
     ptrs = (C.c_void_p * max(len(cols), 1))(*[c.ctypes.data for c in cols])
     return cols, ptrs
 
@@ -391,7 +400,7 @@ def read_agents(sim, T):
     t = sim.T(T)
     n = agent_slots(sim, T)
     cols, ptrs = _empty_cols(t, n)
-    died = np.zeros(n, dtype=np.uint8)
+    died = _zeros(n, np.uint8)
     out = C.c_uint64()
     check(lib().vg_read_agents(sim._h, t.index, ptrs,
                                died.ctypes.data_as(C.POINTER(C.c_uint8)), n, C.byref(out)))
@@ -646,8 +655,8 @@ def read_edges(sim, E, T):
     nr, ne = C.c_uint64(), C.c_uint64()
     check(lib().vg_read_edges(sim._h, e.index, t.index, None, None, None, C.byref(nr),
                               C.byref(ne)))
-    rp = np.zeros(nr.value + 1, dtype=np.uint64)
-    frm = np.zeros(max(ne.value, 1), dtype=np.uint64)
+    rp = _zeros(nr.value + 1, np.uint64)
+    frm = _zeros(max(ne.value, 1), np.uint64)
     cols, ptrs = _empty_cols(e, max(ne.value, 1))
     check(lib().vg_read_edges(sim._h, e.index, t.index, rp.ctypes.data_as(C.POINTER(C.c_uint64)),
                               frm.ctypes.data_as(C.POINTER(C.c_uint64)),
@@ -898,7 +907,7 @@ def rastervalues(sim, name, field):
     ids = cellid(sim, name, [1] * len(dims))
     t = [x for x in sim.model.types.agent_types if x.index == type_nr(ids)][0]
     f = t.field_index(field)
-    out = np.zeros(int(np.prod(dims)), dtype=t.dtype(f))
+    out = _zeros(int(np.prod(dims)), t.dtype(f))
     check(lib().vg_rastervalues(sim._h, name.encode(), f, out.ctypes.data_as(C.c_void_p)))
     return out.reshape(dims, order="F")
 

@@ -171,8 +171,8 @@ class Batch:
 
     def states(self, i, which=0):
         n = int(self.N[i])
-        s = np.zeros(n, np.uint8)
-        d = np.zeros(n, np.int32)
+        s = api._zeros(n, np.uint8)
+        d = api._zeros(n, np.int32)
         out = C.c_uint64()
         check(lib().vg_batch_read_states2(self._h, int(i), int(which),
                                           s.ctypes.data_as(C.POINTER(C.c_uint8)),
