@@ -15,11 +15,14 @@
 //
 //   k_fold_sums   approximate sum of every tile of FOLD_TILE elements
 //   k_fold_frames their prefixes predict the binade ("frame") of each tile
-//   k_fold_tiles  the map of each tile in its predicted frame
-//   k_fold_chain  one block carries the exact sum through the tiles: 1024
-//                 maps are composed and checked per round; a tile that does
-//                 not pass (its sum crosses a power of two, or the
-//                 prediction was off) goes through fold_hard
+//   k_fold_tiles  the map of each tile in its predicted frame; for a tile
+//                 that is predicted to cross into another binade, the maps
+//                 of its chunks of 64 elements in both
+//   k_fold_chain  one block carries the exact sum through the tiles: up to
+//                 1024 maps are composed and checked per round; a predicted
+//                 crossing goes through fold_cross (one warp, its chunks'
+//                 maps up to the crossing and behind it), any other tile that
+//                 does not pass through fold_hard
 //
 // A wrong prediction costs time and nothing else: every map is applied only
 // after its frame and its prefixes were checked against the exact sum.  Sums
@@ -27,14 +30,16 @@
 // changing its binade falls back to the hardware additions, no slower than the
 // plain loop.
 //
-// Bound: for a few million elements the chain's rounds (about 25 crossings
-// of 6 us each), beyond that the two passes over the column (k_fold_sums 7 us
-// and k_fold_tiles 28 us for 5e6).  FOLD_TILE: tiles of 1024, 2048 and 4096
-// elements took 242, 242 and 270 us for 5e6 uniform values, and 15.3, 9.2 and
-// 6.4 ms for 2e6 values whose exponents spread over e^+-300 (there the chain
-// goes tile by tile); 2048 keeps both.  Measured at 5e6 Float64 agents:
-// 181 ms for the plain chain (36 ns per addition), 243 us here; a sum that
-// cancels to zero at every second addition (2e6): 72.6 and 73.5 ms.
+// Bound: for a few million elements the chain (a round 2 us, a crossing 3.5,
+// the first tile with its eleven crossings 30), beyond that the two passes over
+// the column (k_fold_sums 7 us and k_fold_tiles 19 us for 5e6).  FOLD_TILE:
+// tiles of 1024, 2048 and 4096 elements took 242, 242 and 270 us for 5e6
+// uniform values, and 15.3, 9.2 and 6.4 ms for 2e6 values whose exponents spread
+// over e^+-300 (there the chain goes tile by tile); 2048 keeps both.  Measured at
+// 5e6 Float64 agents: 181 ms for the plain chain (36 ns per addition), 253 us
+// with every crossing through fold_hard (two attempts of the whole block, 7.5
+// us) and all 1024 maps read and composed in each round (4.3 us), 145 us here;
+// a sum that cancels to zero at every second addition (2e6): 72.6 and 73.4 ms.
 #pragma once
 
 #include <cstdint>
@@ -52,6 +57,9 @@ constexpr int FOLD_FEW = 128;                       // hardware additions an att
 constexpr int FOLD_PLAIN_MAX = 63;                  // tiles added without an attempt
 constexpr int64_t FOLD_FAR = 1ll << 61;
 constexpr int FOLD_NO_FRAME = -1;
+constexpr int FOLD_CROSS = 1 << 24;                 // a tile's frame: FOLD_CROSS | first << 12 | last
+constexpr int FOLD_SLOTS = 64;                      // crossing tiles with chunk maps
+constexpr int FOLD_TURNS = 2;                       // attempts of fold_cross per tile and chunk
 
 // d0, d1: what an even and an odd m change by; lo, hi: bounds of every
 // prefix's change (lo > hi for the empty run); ok: no element too large for
@@ -59,6 +67,11 @@ constexpr int FOLD_NO_FRAME = -1;
 struct FoldMap {
   int64_t d0, d1, lo, hi;
   int ok;
+};
+
+// a predicted crossing's chunk maps in its first and its last frame
+struct FoldCross {
+  FoldMap m[2][32];
 };
 
 __device__ __forceinline__ FoldMap fold_identity() { return {0, 0, FOLD_FAR, -FOLD_FAR, 1}; }
@@ -202,10 +215,12 @@ __global__ void __launch_bounds__(FOLD_TPB) k_fold_sums(RedArgs a, float *tsum) 
 }
 
 // predicted frame of each tile: the binade of the approximate sum at its
-// start when its end has the same, none otherwise
+// start when its end has the same, else both of them, or none when either has none
 __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_frames(const float *tsum, uint64_t ntiles,
-                                                                double init, int *frame) {
+                                                                double init, int *frame,
+                                                                int *slots) {
   __shared__ float ws[32];
+  if (threadIdx.x == 0) *slots = 0;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float carry = fold_approx(init);
   for (uint64_t t0 = 0; t0 < ntiles; t0 += FOLD_CHAIN_TPB) {
@@ -229,23 +244,26 @@ __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_frames(const float *tsu
     const float total = __shfl_sync(0xffffffffu, s, 31);
     const float end = carry + (w ? before : 0.f) + x;
     const int f1 = fold_frame((double)end), f0 = fold_frame((double)(end - v));
-    if (t < ntiles) frame[t] = f0 == f1 ? f0 : FOLD_NO_FRAME;
+    if (t < ntiles)
+      frame[t] = f0 == f1 ? f0 : f0 < 0 || f1 < 0 ? FOLD_NO_FRAME : FOLD_CROSS | f0 << 12 | f1;
     carry += total;
     __syncthreads();
   }
 }
 
+// a tile without a map leaves NO_FRAME in its frame, a crossing with chunk maps
+// its slot in its map's d0
 template <bool F64>
-__global__ void __launch_bounds__(FOLD_TPB) k_fold_tiles(RedArgs a, const int *frame,
-                                                         FoldMap *maps) {
+__global__ void __launch_bounds__(FOLD_TPB) k_fold_tiles(RedArgs a, int *frame, FoldMap *maps,
+                                                         FoldCross *cross, int *slots,
+                                                         int nslots) {
   __shared__ double v[FOLD_TILE + FOLD_TPB];  // one pad per thread's elements
   __shared__ uint32_t live[FOLD_TILE / 32];
   __shared__ FoldMap ws[FOLD_TPB / 32];
+  __shared__ int slot;
   const int f = frame[blockIdx.x];
-  if (f == FOLD_NO_FRAME) {  // the chain cuts this tile finer
-    if (threadIdx.x == 0) maps[blockIdx.x].ok = 0;
-    return;
-  }
+  if (f == FOLD_NO_FRAME) return;  // the chain cuts this tile finer
+  if (f >= FOLD_CROSS && threadIdx.x == 0) slot = atomicAdd(slots, 1);
   const uint64_t base = (uint64_t)blockIdx.x * FOLD_TILE;
   const int lane = threadIdx.x & 31;
   double x[FOLD_PER];
@@ -261,19 +279,58 @@ __global__ void __launch_bounds__(FOLD_TPB) k_fold_tiles(RedArgs a, const int *f
     if (lane == 0) live[j / 32] = b;
   }
   __syncthreads();
-  FoldMap r = fold_identity();
   const unsigned mask = live[threadIdx.x * FOLD_PER / 32] >> (threadIdx.x * FOLD_PER & 31);
+  auto mine = [&](int in) {  // the map of this thread's elements
+    // all of the frame's sign and none halfway between two integers, as most
+    // are: their rounded values add up, and every prefix lies between the
+    // first and the last
+    int64_t sum = 0, first = 0;
+    bool plain = mask & ((1u << FOLD_PER) - 1), fit = true;
 #pragma unroll
-  for (int k = 0; k < FOLD_PER; k++)
-    if ((mask >> k) & 1u)
-      r = fold_then(r, fold_element(v[threadIdx.x * (FOLD_PER + 1) + k], f, 4));
-  r = fold_warp(r);
+    for (int k = FOLD_PER - 1; k >= 0; k--) {
+      if (!((mask >> k) & 1u)) continue;
+      const int64_t b = __double_as_longlong(v[threadIdx.x * (FOLD_PER + 1) + k]);
+      const int ex = (int)(b >> 52) & 0x7ff, sh = (in & 0x7ff) - (ex ? ex : 1);
+      const uint64_t mx = ((uint64_t)b & ((1ull << 52) - 1)) | (uint64_t)(ex ? 1 : 0) << 52;
+      const int s = min(max(sh, 1), 60);
+      first = (int64_t)((mx + (1ull << (s - 1))) >> s);
+      sum += first;
+      plain &= mx << (64 - s) != 1ull << 63 && (int)((uint64_t)b >> 63) == in >> 11;
+      fit &= sh >= 4;
+    }
+    if (plain) return FoldMap{sum, sum, first, sum, fit};
+    FoldMap r = fold_identity();
+#pragma unroll
+    for (int k = 0; k < FOLD_PER; k++)
+      if ((mask >> k) & 1u)
+        r = fold_then(r, fold_element(v[threadIdx.x * (FOLD_PER + 1) + k], in, 4));
+    return r;
+  };
+  if (f >= FOLD_CROSS) {
+    if (slot >= nslots) {
+      if (threadIdx.x == 0) frame[blockIdx.x] = FOLD_NO_FRAME;
+      return;
+    }
+    if (threadIdx.x == 0) maps[blockIdx.x].d0 = slot;
+    for (int q = 0; q < 2; q++) {
+      FoldMap r = mine((q ? f : f >> 12) & 0xfff);
+#pragma unroll
+      for (int o = 1; o < FOLD_CHUNK / FOLD_PER; o <<= 1) r = fold_then(r, fold_shfl_down(r, o));
+      if (threadIdx.x % (FOLD_CHUNK / FOLD_PER) == 0)
+        cross[slot].m[q][threadIdx.x / (FOLD_CHUNK / FOLD_PER)] = fold_clip(r);
+    }
+    return;
+  }
+  FoldMap r = fold_warp(mine(f));
   if (lane == 0) ws[threadIdx.x >> 5] = r;
   __syncthreads();
   if (threadIdx.x < 32) {
     r = lane < FOLD_TPB / 32 ? ws[lane] : fold_identity();
-    r = fold_warp(r);
-    if (lane == 0) maps[blockIdx.x] = fold_clip(r);
+    r = fold_clip(fold_warp(r));
+    if (lane == 0) {
+      maps[blockIdx.x] = r;
+      if (!r.ok) frame[blockIdx.x] = FOLD_NO_FRAME;
+    }
   }
 }
 
@@ -287,6 +344,9 @@ struct FoldShared {
   int step;       // groups of 32 the hardware adds after an attempt that failed early
   int plain, wait;  // tiles left to add without an attempt; how many after the next failure
   unsigned first;
+  int warps, slot;  // whole warps of a round that pass; chunk maps of the tile behind it
+  int64_t m;        // the sum behind those warps
+  bool stopped;     // a tile of the round did not pass
 };
 
 // the map of one lane's FOLD_LANE elements from j on, none before `from`
@@ -359,8 +419,11 @@ __device__ void fold_plain(const RedArgs &a, uint64_t tile, uint64_t run, FoldSh
 // 32, 64, 128, ... hardware additions before the next, and once that is a
 // whole tile, by whole tiles without an attempt (1, 3, 7, .. 63): a sum that
 // leaves its binade at every turn runs at the speed of the plain chain.
+// A sum that starts at zero doubles within every few elements at first: there
+// FOLD_FEW hardware additions precede the first attempt.
+// start: elements of the tile that are in the sum already
 template <bool F64>
-__device__ void fold_hard(const RedArgs &a, uint64_t tile, FoldShared &S) {
+__device__ void fold_hard(const RedArgs &a, uint64_t tile, int start, FoldShared &S) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint64_t base = tile * FOLD_TILE;
 #pragma unroll
@@ -372,8 +435,20 @@ __device__ void fold_hard(const RedArgs &a, uint64_t tile, FoldShared &S) {
     const unsigned b = __ballot_sync(0xffffffffu, on);
     if (lane == 0) S.live[j / 32] = b;
   }
-  if (threadIdx.x == 0) S.at = 0;
+  if (threadIdx.x == 0) S.at = start;
   __syncthreads();
+  if (tile == 0 && start == 0 && fold_frame(S.a) == FOLD_NO_FRAME) {  // block-uniform
+    double cur = S.a;
+    __syncthreads();
+    if (w == 0) {
+      for (int j = 0; j < FOLD_FEW; j += 32) cur = fold_plain_32(S.v[0], j, cur);
+      if (lane == 0) {
+        S.a = cur;
+        S.at = FOLD_FEW;
+      }
+    }
+    __syncthreads();
+  }
   const uint64_t left = a.n - base;
   const int end = left < (uint64_t)FOLD_TILE
                       ? (int)(left + FOLD_LANE - 1) / FOLD_LANE * FOLD_LANE : FOLD_TILE;
@@ -438,13 +513,76 @@ __device__ void fold_hard(const RedArgs &a, uint64_t tile, FoldShared &S) {
   }
 }
 
+// A predicted crossing, by warp 0: the maps of the chunks in the sum's frame,
+// one per lane, carry it to the chunk that leaves the binade; that chunk's
+// elements are mapped two per lane, those of the lane that crosses are added by
+// the hardware, and what is behind them goes on in the new frame.  Returns
+// the elements done, on all lanes, and the sum: all of the tile, or less when
+// the sum is in neither frame or crosses again (fold_hard does the rest).
+template <bool F64>
+__device__ int fold_cross(const RedArgs &a, uint64_t tile, int frames, const FoldCross *cross,
+                          double &acc) {
+  const int lane = threadIdx.x & 31;
+  const FoldMap m0 = cross->m[0][lane], m1 = cross->m[1][lane];
+  int c = 0;
+  for (int turn = 0; turn < FOLD_TURNS; turn++) {
+    int f = fold_frame(acc);
+    const bool second = f != (frames >> 12 & 0xfff);
+    if (f == FOLD_NO_FRAME || (second && f != (frames & 0xfff))) return c * FOLD_CHUNK;
+    int64_t m = fold_m(acc);
+    FoldMap r = fold_warp_scan(lane < c ? fold_identity() : second ? m1 : m0);
+    unsigned bad = __ballot_sync(0xffffffffu, !fold_fits(r, m));
+    const int b = bad ? __ffs(bad) - 1 : 32;
+    if (b > c) {
+      acc = fold_value(f, __shfl_sync(0xffffffffu, fold_apply(r, m), b - 1));
+      c = b;
+    }
+    if (c == 32) return FOLD_TILE;
+    double x[FOLD_LANE];
+    bool on[FOLD_LANE];
+    const int at = c * FOLD_CHUNK + FOLD_LANE * lane;
+#pragma unroll
+    for (int k = 0; k < FOLD_LANE; k++) {
+      on[k] = fold_load<F64>(a, tile * FOLD_TILE + at + k, &x[k]);
+      if (!on[k]) x[k] = -0.0;
+    }
+    int l = 0;  // lanes of the chunk that are in the sum
+    for (int in = 0; l < 32; in++) {
+      f = fold_frame(acc);
+      if (in == FOLD_TURNS || f == FOLD_NO_FRAME) return c * FOLD_CHUNK + FOLD_LANE * l;
+      m = fold_m(acc);
+      r = fold_identity();
+      if (lane >= l) {
+#pragma unroll
+        for (int k = 0; k < FOLD_LANE; k++)
+          if (on[k]) r = fold_then(r, fold_element(x[k], f, 1));
+      }
+      r = fold_warp_scan(r);
+      bad = __ballot_sync(0xffffffffu, !fold_fits(r, m));
+      const int e = bad ? __ffs(bad) - 1 : 32;
+      if (e > l) acc = fold_value(f, __shfl_sync(0xffffffffu, fold_apply(r, m), e - 1));
+      l = e;
+      if (l < 32) {
+#pragma unroll
+        for (int k = 0; k < FOLD_LANE; k++)
+          acc = __dadd_rn(__shfl_sync(0xffffffffu, x[k], l), acc);
+        l++;
+      }
+    }
+    c++;
+    if (c == 32) return FOLD_TILE;
+  }
+  return c * FOLD_CHUNK;
+}
+
 // the exact sum through all tiles; maps == null: every tile is cut finer
 // (short columns, where predicting costs more than it saves)
 template <bool F64>
 __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_chain(RedArgs a, uint64_t ntiles,
                                                                const int *frame,
-                                                               const FoldMap *maps, int64_t *oi,
-                                                               double *of) {
+                                                               const FoldMap *maps,
+                                                               const FoldCross *cross,
+                                                               int64_t *oi, double *of) {
   __shared__ FoldShared S;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
@@ -467,45 +605,93 @@ __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_chain(RedArgs a, uint64
       __syncthreads();
       continue;
     }
+    if (threadIdx.x == 0) {
+      S.first = FOLD_CHAIN_TPB;
+      S.slot = -1;
+      S.at = 0;
+    }
+    __syncthreads();
     bool hard = true;
     if (maps) {
-      // thread k: tile t0 + k; a tile beyond the end stops the round, one
-      // with another frame than the sum's fails
+      // thread k: tile t0 + k; the run ends at the first tile in another
+      // frame than the sum's, and only the warps of the run read and compose
+      // its maps
       const int f = fold_frame(acc);
       const uint64_t t = t0 + threadIdx.x;
+      const int tf = t < ntiles ? frame[t] : FOLD_NO_FRAME;
+      const unsigned other = __ballot_sync(0xffffffffu, tf != f || f == FOLD_NO_FRAME);
+      if (lane == 0 && other) atomicMin(&S.first, (unsigned)(w * 32 + __ffs(other) - 1));
+      __syncthreads();
+      const unsigned run = S.first, nw = (run + 31) / 32;
       FoldMap r = fold_identity();
-      if (t < ntiles) {
-        r.ok = frame[t] == f && f != FOLD_NO_FRAME && maps[t].ok;
-        if (r.ok) r = maps[t];
+      if (threadIdx.x == run && t < ntiles && tf >= FOLD_CROSS) S.slot = (int)maps[t].d0;
+      if ((unsigned)w < nw) {
+        if (threadIdx.x < run) r = maps[t];
+        r = fold_warp_scan(r);
+        if (lane == 31) S.wmap[w] = r;
       }
-      r = fold_warp_scan(r);
-      if (threadIdx.x == 0) S.first = FOLD_CHAIN_TPB;
-      if (lane == 31) S.wmap[w] = r;
       __syncthreads();
-      // maps of the warps before this one
-      FoldMap p = fold_warp_scan(S.wmap[lane]);
-      p = {__shfl_sync(0xffffffffu, p.d0, (w + 31) & 31), __shfl_sync(0xffffffffu, p.d1, (w + 31) & 31),
-           __shfl_sync(0xffffffffu, p.lo, (w + 31) & 31), __shfl_sync(0xffffffffu, p.hi, (w + 31) & 31),
-           __shfl_sync(0xffffffffu, p.ok, (w + 31) & 31)};
-      if (w) r = fold_then(p, r);
-      const int64_t m = fold_m(acc);
-      const bool pass = t < ntiles && f != FOLD_NO_FRAME && fold_fits(r, m);
-      const unsigned bad = __ballot_sync(0xffffffffu, !pass);
-      if (lane == 0 && bad) atomicMin(&S.first, (unsigned)(w * 32 + __ffs(bad) - 1));
+      if (w == 0) {
+        const FoldMap p = fold_warp_scan((unsigned)lane < nw ? S.wmap[lane] : fold_identity());
+        const int64_t m = fold_m(acc);
+        const unsigned bad = __ballot_sync(0xffffffffu, (unsigned)lane < nw && !fold_fits(p, m));
+        const int k = bad ? __ffs(bad) - 1 : (int)nw;
+        const int64_t to = __shfl_sync(0xffffffffu, fold_apply(p, m), (k + 31) & 31);
+        if (lane == 0) {
+          S.warps = k;
+          S.m = k ? to : m;
+          if (k == (int)nw) {
+            if (run) S.a = fold_value(f, to);
+            S.next = t0 + run;
+          }
+        }
+      }
       __syncthreads();
-      const unsigned first = S.first;  // tiles t0 .. t0 + first - 1 pass
-      if (first && threadIdx.x == first - 1) S.a = fold_value(f, fold_apply(r, m));
-      hard = first < FOLD_CHAIN_TPB && t0 + first < ntiles;
-      __syncthreads();
-      if (threadIdx.x == 0) S.next = t0 + first;
-      __syncthreads();
+      const int k = S.warps;
+      hard = t0 + run < ntiles && run < FOLD_CHAIN_TPB;
+      if (k < (int)nw) {  // block-uniform: warp k has the first tile that does not pass
+        if (w == k) {
+          // (none, when the warp's own bounds are met and only the bounds of
+          // all before it together, taken over both parities, were not)
+          const unsigned bad = __ballot_sync(0xffffffffu, !fold_fits(r, S.m));
+          const int l = bad ? __ffs(bad) - 1 : 32;
+          const int64_t to = __shfl_sync(0xffffffffu, fold_apply(r, S.m), (l + 31) & 31);
+          if (lane == 0) {
+            S.a = fold_value(f, l ? to : S.m);
+            S.next = min(t0 + k * 32 + l, t0 + run);
+            S.slot = -1;
+            S.stopped = bad != 0;
+          }
+        }
+        __syncthreads();
+        hard = S.stopped;
+      }
+      if (hard && S.slot >= 0) {  // block-uniform
+        const uint64_t tile = S.next;
+        __syncthreads();
+        if (w == 0) {
+          double cur = S.a;
+          const int done = fold_cross<F64>(a, tile, frame[tile], cross + S.slot, cur);
+          if (lane == 0) {
+            S.a = cur;
+            S.at = done;
+            if (done == FOLD_TILE) S.next = tile + 1;
+            if (done >= FOLD_FEW) {  // an attempt that was worth it
+              S.step = 0;
+              S.wait = 1;
+            }
+          }
+        }
+        __syncthreads();
+        hard = S.at < FOLD_TILE;
+      }
     }
     if (hard) {
-      fold_hard<F64>(a, S.next, S);
+      fold_hard<F64>(a, S.next, S.at, S);
       // NaN stays NaN whatever is added
       if (threadIdx.x == 0) S.next = isnan(S.a) ? ntiles : S.next + 1;
-      __syncthreads();
     }
+    __syncthreads();
   }
   if (threadIdx.x == 0) {
     *oi = a.init_i;
