@@ -995,9 +995,23 @@ uint64_t upload_staged(Sim &s, int e, DevBuf &from, DevBuf &to,
   uint64_t n = 0;
   for (auto &sg : es.staged) n += sg.n;
   int nf = ed.stores_payload() ? (int)ed.fields.size() : 0;
+  payload.resize(nf);
+  auto done = [&]() {
+    es.staged.clear();
+    es.nstaged = 0;
+    es.single_seen.clear();
+    return n;
+  };
+  if (n == 0) return done();
+  for (auto &sg : es.staged)
+    if (sg.device && sg.n == n) {  // all of them, on the device already
+      from = std::move(sg.d_from);
+      to = std::move(sg.d_to);
+      for (int f = 0; f < nf; f++) payload[f] = std::move(sg.d_payload[f]);
+      return done();
+    }
   from.alloc(std::max<uint64_t>(n, 1) * 8, &s.footprint);
   to.alloc(std::max<uint64_t>(n, 1) * 8, &s.footprint);
-  payload.resize(nf);
   for (int f = 0; f < nf; f++) payload[f].alloc(std::max<uint64_t>(n, 1) * ed.fields[f].size, &s.footprint);
   uint64_t off = 0;
   for (auto &sg : es.staged) {
@@ -1013,10 +1027,7 @@ uint64_t upload_staged(Sim &s, int e, DevBuf &from, DevBuf &to,
     off += sg.n;
   }
   VG_CUDA(cudaStreamSynchronize(s.stream));
-  es.staged.clear();
-  es.nstaged = 0;
-  es.single_seen.clear();
-  return n;
+  return done();
 }
 
 void flush_staged_edges(Sim &s, int e, bool merge) {
