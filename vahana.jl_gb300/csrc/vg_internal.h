@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstring>
 #include <map>
 #include <memory>
 #include <string>
@@ -398,6 +399,29 @@ struct StatusWord {
 };
 constexpr size_t PIN_BYTES = 256;
 #ifdef __CUDACC__
+// programmatic dependent launches: the next kernel of the stream may start
+// once every block has called let_next_start; the last block of a kernel that
+// started so waits for the preceding one, so that whatever follows it sees both
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void end_after_previous() {
+  if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// a launch that may start before the preceding one of the stream has ended
+template <class... A, class... B>
+void launch_dependent(void (*k)(A...), unsigned grid, unsigned block, cudaStream_t st, B... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  VG_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
+}
 __device__ __forceinline__ void report_status(int *status, int code) {
   if (atomicCAS(status, 0, code) == 0) {
     int *host = ((StatusWord *)status)->host;
@@ -533,8 +557,24 @@ struct OpinionJob {
   uint32_t hub_thr;
   uint32_t block_thr = 0xFFFFFFFFu;
 };
-void launch_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_t st, DevBuf &args_buf,
-                         DevBuf &tiles_buf, uint64_t *footprint);
+// Their steps in one launch: pack_opinion_jobs appends the launch's tables to
+// `bytes`, launch_opinion_jobs runs them from the device copy of `bytes`.
+// Returns whether a programmatic dependent launch may follow.
+struct OpinionTables {
+  size_t args_at, tiles_at;
+  unsigned ntiles, nlong;
+};
+OpinionTables pack_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_t st,
+                                std::vector<uint8_t> &bytes);
+bool launch_opinion_jobs(const OpinionTables &t, const uint8_t *dev, cudaStream_t st);
+// `a` behind what `bytes` holds, 16-byte aligned; returns where
+template <class T>
+size_t append_table(std::vector<uint8_t> &bytes, const std::vector<T> &a) {
+  const size_t at = (bytes.size() + 15) / 16 * 16;
+  bytes.resize(at + a.size() * sizeof(T));
+  if (!a.empty()) std::memcpy(bytes.data() + at, a.data(), a.size() * sizeof(T));
+  return at;
+}
 void prepare_opinion_job(const OpinionJob &job);
 // initial SIR state: the n_inf agents with the smallest Philox init draw
 void sir_initial_state(uint64_t n, uint64_t seed, uint64_t n_inf, std::vector<uint8_t> &state);

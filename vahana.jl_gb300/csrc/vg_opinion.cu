@@ -750,13 +750,6 @@ __device__ __forceinline__ void report_range(const Notify &nt, unsigned r) {
 // chains overlap everything else.  The two read the old opinions and write
 // disjoint rows; the second ends only after the first (its last block waits
 // for it), so whatever follows in the stream sees both.
-__device__ __forceinline__ void let_next_start() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void end_after_previous() {
-  if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 template <bool GRID, bool REPORT>
 __global__ void __launch_bounds__(LONG_TPB) k_opinion_long(OpinionArgs p, Notify nt) {
   __shared__ LongShared S;
@@ -808,6 +801,7 @@ struct JobTile {
 __global__ void __launch_bounds__(TPB, 9) k_opinion_jobs(const OpinionArgs *jobs,
                                                       const JobTile *tiles) {
   __shared__ OpinionArgs sp;
+  let_next_start();
   JobTile t = tiles[blockIdx.x];
   if (threadIdx.x == 0) sp = jobs[t.job];
   __syncthreads();
@@ -868,20 +862,6 @@ static unsigned split_long(OpinionArgs &p, uint64_t edges) {
   return (unsigned)p.nbig + p.hub_blocks + (unsigned)((p.nslices + (TPB / 32) - 1) / (TPB / 32));
 }
 
-// a launch that may start before the preceding one of the stream has ended
-template <class... A, class... B>
-static void launch_dependent(void (*k)(A...), unsigned grid, cudaStream_t st, B... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(TPB);
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  VG_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
-}
 // a gather launch whose finished row ranges are downloaded while it runs
 // (apply! with host exchange)
 static void launch_notified(Sim &s, OpinionArgs &p, unsigned grid, Sim::HostExchange &hx);
@@ -936,8 +916,8 @@ void tr_bounded_confidence(ApplyCtx &c) {
     if (p.grid) k_opinion_long<true, false><<<nl, LONG_TPB, 0, s.stream>>>(p, Notify{});
     else k_opinion_long<false, false><<<nl, LONG_TPB, 0, s.stream>>>(p, Notify{});
     VG_CUDA(cudaGetLastError());
-    launch_dependent(p.grid ? k_opinion<true, true> : k_opinion<false, true>, grid - nbig, s.stream,
-                     p);
+    launch_dependent(p.grid ? k_opinion<true, true> : k_opinion<false, true>, grid - nbig, TPB,
+                     s.stream, p);
   } else if (grid > nbig) {
     if (p.grid) k_opinion<true, false><<<grid - nbig, TPB, 0, s.stream>>>(p);
     else k_opinion<false, false><<<grid - nbig, TPB, 0, s.stream>>>(p);
@@ -1022,7 +1002,7 @@ static void launch_notified(Sim &s, OpinionArgs &p, unsigned grid, Sim::HostExch
     if (p.grid) k_opinion_long<true, true><<<nl, LONG_TPB, 0, s.stream>>>(p, nt);
     else k_opinion_long<false, true><<<nl, LONG_TPB, 0, s.stream>>>(p, nt);
     VG_CUDA(cudaGetLastError());
-    launch_dependent(p.grid ? k_opinion_notify<true, true> : k_opinion_notify<false, true>, grid,
+    launch_dependent(p.grid ? k_opinion_notify<true, true> : k_opinion_notify<false, true>, grid, TPB,
                      s.stream, p, nt);
   } else {
     if (p.grid) k_opinion_notify<true, false><<<grid, TPB, 0, s.stream>>>(p, nt);
@@ -1167,8 +1147,8 @@ void prepare_opinion_job(const OpinionJob &j) {
 // One launch for the bounded-confidence step of many simulations (the
 // serving loop's continuous batching).  Each job's blocks do exactly what
 // its own launch would; the caller finishes each job's transition.
-void launch_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_t st, DevBuf &args_buf,
-                         DevBuf &tiles_buf, uint64_t *fp) {
+OpinionTables pack_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_t st,
+                                std::vector<uint8_t> &bytes) {
   std::vector<OpinionArgs> args;
   std::vector<JobTile> tiles, longs;
   uint64_t edges = 0;  // of all jobs: they share the launch
@@ -1184,31 +1164,28 @@ void launch_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_t st, D
     for (unsigned k = 0; k < g; k++) tiles.push_back({(uint32_t)j, k});
     for (unsigned k = 0; k < p.long_hubs + p.nlong; k++) longs.push_back({(uint32_t)j, k});
   }
-  if (tiles.empty()) return;
-  // (one buffer: the long slices' tiles behind the others)
-  const size_t ntiles = tiles.size();
-  for (const JobTile &t : longs) tiles.push_back(t);
-  if (args_buf.bytes < args.size() * sizeof(OpinionArgs))
-    args_buf.alloc(args.size() * sizeof(OpinionArgs) * 2, fp);
-  if (tiles_buf.bytes < tiles.size() * sizeof(JobTile))
-    tiles_buf.alloc(tiles.size() * sizeof(JobTile) * 2, fp);
-  VG_CUDA(cudaMemcpyAsync(args_buf.p, args.data(), args.size() * sizeof(OpinionArgs),
-                          cudaMemcpyHostToDevice, st));
-  VG_CUDA(cudaMemcpyAsync(tiles_buf.p, tiles.data(), tiles.size() * sizeof(JobTile),
-                          cudaMemcpyHostToDevice, st));
-  const OpinionArgs *da = args_buf.as<OpinionArgs>();
-  const JobTile *dt = tiles_buf.as<JobTile>();
-  if (!longs.empty()) {
-    k_opinion_jobs_long<<<(unsigned)longs.size(), LONG_TPB, 0, st>>>(da, dt + ntiles);
+  OpinionTables t{0, 0, (unsigned)tiles.size(), (unsigned)longs.size()};
+  if (tiles.empty()) return t;
+  // (the long slices' tiles behind the others)
+  tiles.insert(tiles.end(), longs.begin(), longs.end());
+  t.args_at = append_table(bytes, args);
+  t.tiles_at = append_table(bytes, tiles);
+  return t;
+}
+
+bool launch_opinion_jobs(const OpinionTables &t, const uint8_t *dev, cudaStream_t st) {
+  if (!t.ntiles) return false;
+  const OpinionArgs *da = (const OpinionArgs *)(dev + t.args_at);
+  const JobTile *dt = (const JobTile *)(dev + t.tiles_at);
+  if (t.nlong) {
+    k_opinion_jobs_long<<<t.nlong, LONG_TPB, 0, st>>>(da, dt + t.ntiles);
     VG_CUDA(cudaGetLastError());
+    launch_dependent(k_opinion_jobs, t.ntiles, TPB, st, da, dt);
+  } else {
+    k_opinion_jobs<<<t.ntiles, TPB, 0, st>>>(da, dt);
   }
-  // (with no long block before it, its dependency is the copies above)
-  if (longs.empty()) k_opinion_jobs<<<(unsigned)ntiles, TPB, 0, st>>>(da, dt);
-  else launch_dependent(k_opinion_jobs, (unsigned)ntiles, st, da, dt);
   VG_CUDA(cudaGetLastError());
-  // no wait: a copy from pageable host memory is staged before the call
-  // returns, so the host vectors may go; the device buffers are rewritten by
-  // the next call's copies in stream order, after this launch
+  return true;
 }
 
 }  // namespace vg
