@@ -503,8 +503,9 @@ int vg_batch_set_launch(vg_batch *b, int persistent, int persistent_tpb,
 int vg_batch_set_cluster(vg_batch *b, int ctas, int tpb, int ilp);
 int vg_batch_cluster(vg_batch *b, int *ctas, int *tpb, int *ilp,
                      unsigned *clusters);
-/* Agents per lane of the per-step launch and of the persistent launch (1, 2
- * or 4: a lane walks the in-edge rows of its agents together).  The setter
+/* Agents per lane of the per-step launch (1, 2 or 4: a lane walks the in-edge
+ * rows of its agents together), and of the persistent launch, where 1, 2 or 4
+ * stand for 4, 8 or 16 edges of a lane's row per round.  The setter
  * overrides the autotuner's choice (0 keeps the current value); the getter
  * reads the values in use.  Both run the autotuner if it has not run. */
 int vg_batch_set_lanes(vg_batch *b, int per_step, int persistent);

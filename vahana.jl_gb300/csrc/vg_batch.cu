@@ -16,8 +16,8 @@
 // thread-block clusters that each step their own packs of
 // whole instances (masks in distributed shared memory, cluster barriers).
 // A small autotuner keyed on the arena's degree histogram picks the form and
-// its shape (block size, agents per lane, degree buckets, cluster size) by
-// timing them.
+// its shape (block size, agents or row loads per lane, degree buckets, cluster
+// size) by timing them.
 //
 // The plain path of the same instances (vg_batch_step_one) runs apply! on
 // the instance's own simulation; both paths produce bit-identical states.
@@ -95,22 +95,48 @@ __device__ __forceinline__ uint8_t sir_rule(const BatchArgs &a, uint64_t i, uint
   return s;
 }
 
+// The same rule on one buffer, which the agent alone reads and writes (its
+// neighbours read the mask): an agent that stays as it is writes nothing, and
+// only an infected one reads its days.
+__device__ __forceinline__ uint8_t sir_rule_in_place(const BatchArgs &a, uint64_t i, uint32_t k,
+                                                     uint8_t s, uint32_t step, uint8_t *st,
+                                                     int32_t *dy) {
+  if (s == 0 && k > 0) {
+    const uint32_t in = a.inst[i];
+    if (k >= a.kmax1) {
+      atomicCAS(a.status, 0, 402);
+    } else {
+      const uint64_t nr = i - a.base[in] + 1;
+      if (unit_below(philox_u64(philox_draw(a.seed[in], nr, step, TAG_INFECT)),
+                     a.ptab[(uint64_t)in * a.kmax1 + k])) {
+        st[i] = 1;
+        dy[i] = 0;
+        return 1;
+      }
+    }
+  } else if (s == 1) {
+    const int32_t d = dy[i] + 1;
+    dy[i] = d;
+    if (d >= a.rec[a.inst[i]]) {
+      st[i] = 2;
+      return 2;
+    }
+  }
+  return s;
+}
+
 // source loads of one row per round of a lane's row walk
 constexpr int ROW_UNROLL = 2;
 
 // One warp steps the ILP * 32 agents c0 .. c0 + 32 ILP - 1 (c0 a multiple of
 // 32): lane l takes agents c0 + 32 u + l, u < ILP, and walks their rows
 // together, ROW_UNROLL edges of each per round, so that ROW_UNROLL ILP
-// source loads (and then as many mask loads) are in flight at once.  Agents flagged in `skip`
-// are left to other warps (their bits too).  With `atomic_bits` the mask
-// words are updated bit by bit (other warps own some of their bits);
-// otherwise each word is stored whole.
+// source loads (and then as many mask loads) are in flight at once.
 template <int ILP>
 __device__ __forceinline__ void sir_chunk(const BatchArgs &a, const uint8_t *st_rd,
                                           const int32_t *d_rd, const uint32_t *inf_rd,
                                           uint8_t *st_wr, int32_t *d_wr, uint32_t *inf_wr,
-                                          uint64_t c0, uint32_t step, const uint8_t *skip,
-                                          bool atomic_bits) {
+                                          uint64_t c0, uint32_t step) {
   const unsigned lane = threadIdx.x & 31;
   uint8_t s[ILP];
   int32_t d[ILP];
@@ -119,7 +145,7 @@ __device__ __forceinline__ void sir_chunk(const BatchArgs &a, const uint8_t *st_
 #pragma unroll
   for (int u = 0; u < ILP; u++) {
     const uint64_t i = c0 + 32u * u + lane;
-    live[u] = i < a.n && !(skip && skip[i]);
+    live[u] = i < a.n;
     s[u] = live[u] ? st_rd[i] : (uint8_t)3;
     d[u] = live[u] ? d_rd[i] : 0;
     k[u] = 0;
@@ -159,15 +185,7 @@ __device__ __forceinline__ void sir_chunk(const BatchArgs &a, const uint8_t *st_
     uint8_t ns = 3;
     if (live[u]) ns = sir_rule(a, i0 + lane, k[u], s[u], d[u], step, st_wr, d_wr);
     const unsigned set = __ballot_sync(0xffffffffu, live[u] && ns == 1);
-    if (atomic_bits) {
-      const unsigned clr = __ballot_sync(0xffffffffu, live[u] && ns != 1);
-      if (lane == 0) {
-        if (set) atomicOr(inf_wr + (i0 >> 5), set);
-        if (clr) atomicAnd(inf_wr + (i0 >> 5), ~clr);
-      }
-    } else if (lane == 0) {
-      inf_wr[i0 >> 5] = set;
-    }
+    if (lane == 0) inf_wr[i0 >> 5] = set;
   }
 }
 
@@ -178,8 +196,7 @@ __global__ void k_batch_sir(BatchArgs a) {
   const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t c0 = warp * 32 * ILP;
   if (c0 >= a.n) return;
-  sir_chunk<ILP>(a, a.st_rd, a.d_rd, a.inf_rd, a.st_wr, a.d_wr, a.inf_wr, c0, a.step, nullptr,
-                 false);
+  sir_chunk<ILP>(a, a.st_rd, a.d_rd, a.inf_rd, a.st_wr, a.d_wr, a.inf_wr, c0, a.step);
 }
 
 // the infected-agent mask of a state array
@@ -209,22 +226,118 @@ __global__ void k_inf_bits(const uint8_t *st, uint64_t n, uint32_t *m) {
 // constant for the whole launch).  Agents above a degree threshold (listed
 // in `heavy`, sorted) are folded by a warp each, inside the ticket of their
 // range (the infected-neighbour count is an integer: any order gives the
-// same k); the others in warp chunks as in the per-step form.
+// same k); the others by warps of 32 rounds agents each (sir_warp).
+//
+// The states and days stay in one buffer and only the masks alternate; an odd
+// number of steps begins with a per-step launch into the other buffer.  An
+// instance without an infected agent never changes again: a range whose
+// instances have none (`active`) clears its mask words and goes on.
+// Bound: the rows of the susceptible agents while an epidemic runs, then the
+// tickets.  Measured, 512 instances, 1.1*10^7 agents, us per step with both
+// buffers read and written and every row walked by the lane of its agent, and
+// now: steps 0..10 269 and 282, 20..30 135 and 105, 40..80 110 and 57, 80..200
+// 103 and 39, 400 and later 102 and 23.  (Streaming the rows of a warp's 256
+// agents, an edge per lane, instead of walking them where most agents are
+// susceptible: 295 in the first ten steps.)
 struct PersistArgs {
   BatchArgs a;                 // graph, tables; state pointers unused
-  uint8_t *st[2];
-  int32_t *dy[2];
+  uint8_t *st;
+  int32_t *dy;
   uint32_t *inf[2];
-  int cur0;                    // buffer of the state before the first step
-  uint32_t steps, step0;       // steps to run, transition number of the first
+  int cur0;                    // mask of the state before the first step
+  uint32_t steps, step0;       // steps to run (an even number), transition number of the first
   const uint32_t *heavy;       // agents above the bucket threshold (nheavy, ascending)
   uint64_t nheavy;
   const uint8_t *is_heavy;     // per agent (null: no heavy agents)
   unsigned *ticket;            // next ticket (zero at launch)
   uint32_t *done;              // per instance: agent-steps finished in this launch (zero at launch)
   const uint32_t *inst_n;      // per instance: agents
-  unsigned rounds;             // chunk rounds per block ticket
+  // [t & 1][instance]: t when the instance has an infected agent before step t
+  // (two rows: ranges of an instance may be a step apart)
+  uint32_t *active;
+  uint32_t ninst;
+  int rounds;                  // mask words per warp and ticket, up to WARP_WORDS
 };
+
+constexpr int WARP_WORDS = 8;
+struct WarpShared {
+  uint32_t bits[WARP_WORDS];      // the new mask words
+  uint8_t list[WARP_WORDS * 32];  // susceptible agents
+};
+
+// One warp steps the 32 * words agents from c0 (a multiple of 32) up to a1 in
+// place.  Their states first, all in flight together: the infected ones count
+// their days, the susceptible ones are listed.  Then the listed rows, 32 at a
+// time and U edges of each per round: a lane whose agent is not susceptible
+// would wait for its neighbours' rows, and late in an epidemic nine of ten are
+// not.
+template <int U>
+__device__ __forceinline__ void sir_warp(const PersistArgs &p, const uint32_t *inf_rd,
+                                         uint32_t *inf_wr, uint64_t c0, uint64_t a1, uint32_t step,
+                                         uint32_t *active, uint32_t tag, WarpShared &S) {
+  const BatchArgs &a = p.a;
+  const unsigned lane = threadIdx.x & 31;
+  uint8_t s[WARP_WORDS];
+#pragma unroll
+  for (int u = 0; u < WARP_WORDS; u++) {
+    const uint64_t i = c0 + 32u * u + lane;
+    s[u] = u < p.rounds && i < a1 && !(p.is_heavy && p.is_heavy[i]) ? p.st[i] : (uint8_t)3;
+  }
+  uint32_t word = 0, live = 0, n = 0;  // of word `lane`; susceptible agents
+#pragma unroll
+  for (int u = 0; u < WARP_WORDS; u++) {
+    const uint64_t i = c0 + 32u * u + lane;
+    const unsigned sus = __ballot_sync(0xffffffffu, s[u] == 0);
+    if (s[u] == 0) S.list[n + __popc(sus & ((1u << lane) - 1u))] = (uint8_t)(32 * u + lane);
+    n += __popc(sus);
+    if (s[u] == 1) s[u] = sir_rule_in_place(a, i, 0, 1, step, p.st, p.dy);
+    const unsigned set = __ballot_sync(0xffffffffu, s[u] == 1);
+    const unsigned own = __ballot_sync(0xffffffffu, s[u] != 3);
+    if ((int)lane == u) {
+      word = set;
+      live = own;
+    }
+  }
+  if (lane < WARP_WORDS) S.bits[lane] = word;
+  __syncwarp();
+  for (uint32_t b = 0; b < n; b += 32) {
+    const bool on = b + lane < n;
+    const uint32_t o = on ? S.list[b + lane] : 0u;
+    const uint64_t i = c0 + o;
+    uint32_t q = on ? a.rp[i] : 0u, k = 0;
+    const uint32_t e = on ? a.rp[i + 1] : 0u;
+    while (__any_sync(0xffffffffu, q < e)) {
+      uint32_t j[U], w[U];
+#pragma unroll
+      for (int r = 0; r < U; r++) j[r] = q + r < e ? a.src[q + r] : 0u;
+#pragma unroll
+      for (int r = 0; r < U; r++) w[r] = q + r < e ? inf_rd[j[r] >> 5] : 0u;
+#pragma unroll
+      for (int r = 0; r < U; r++) k += (w[r] >> (j[r] & 31)) & 1u;
+      q = q + U < e ? q + U : e;
+    }
+    if (k > 0 && sir_rule_in_place(a, i, k, 0, step, p.st, p.dy) == 1)
+      atomicOr(&S.bits[o >> 5], 1u << (o & 31));
+  }
+  __syncwarp();
+  if (lane < WARP_WORDS && (int)lane < p.rounds && c0 + 32u * lane < a1) {
+    const uint64_t i0 = c0 + 32u * lane;
+    uint32_t set = S.bits[lane];
+    if (p.is_heavy) {  // other warps own some of the word's bits
+      if (set) atomicOr(inf_wr + (i0 >> 5), set);
+      if (live & ~set) atomicAnd(inf_wr + (i0 >> 5), ~(live & ~set));
+    } else {
+      inf_wr[i0 >> 5] = set;
+    }
+    while (set) {  // once per instance that has an infected agent in the word
+      const uint32_t in = a.inst[i0 + __ffs(set) - 1];
+      if (((volatile uint32_t *)active)[in] != tag) ((volatile uint32_t *)active)[in] = tag;
+      const uint64_t end = a.base[in] + p.inst_n[in];
+      set = end - i0 >= 32 ? 0u : set & ~((1u << (unsigned)(end - i0)) - 1u);
+    }
+  }
+  __syncwarp();  // (the shared words are used again)
+}
 
 constexpr uint32_t BAR_SPIN_LIMIT = 1u << 22;
 constexpr int BAR_ERR_WAIT = 0x5e04;
@@ -255,48 +368,65 @@ __global__ void k_barrier_probe(const uint32_t *counter, uint32_t target, int *s
   if (threadIdx.x == 0) wait_count(counter, target, status, limit);
 }
 
-template <int ILP>
+template <int U>
 __global__ void k_batch_persist(PersistArgs p) {
+  extern __shared__ WarpShared s_warp[];
   __shared__ unsigned s_ticket;
-  __shared__ int s_ok;
+  __shared__ int s_ok, s_quiet;
   const BatchArgs &a = p.a;
   const unsigned lane = threadIdx.x & 31;
   const unsigned wpb = blockDim.x / 32, wib = threadIdx.x / 32;
-  const bool atomic_bits = p.is_heavy != nullptr;
-  const uint64_t span = (uint64_t)wpb * 32 * ILP * p.rounds;
+  const uint64_t span = (uint64_t)wpb * 32 * p.rounds;
   const uint64_t tps = (a.n + span - 1) / span;  // tickets per step
   const uint64_t total = tps * p.steps;
+  // (a block takes its next ticket before it works on one: it still works on
+  // its tickets in order, so the lowest unfinished one is always worked on)
+  unsigned next = 0;
+  if (threadIdx.x == 0) next = atomicAdd(p.ticket, 1u);
   for (;;) {
-    if (threadIdx.x == 0) s_ticket = atomicAdd(p.ticket, 1u);
+    if (threadIdx.x == 0) {
+      s_ticket = next;
+      if (next < total) next = atomicAdd(p.ticket, 1u);
+    }
     __syncthreads();
     const uint64_t T = s_ticket;
-    __syncthreads();
     if (T >= total) break;
     const uint32_t t = (uint32_t)(T / tps);
     const uint64_t a0 = (T % tps) * span;
     const uint64_t a1 = a0 + span < a.n ? a0 + span : a.n;
     const uint32_t i0 = a.inst[a0], i1 = a.inst[a1 - 1];
     // the range's instances have finished step t - 1
-    if (threadIdx.x == 0) {
-      s_ok = !*(volatile int *)a.status;
-      for (uint32_t i = i0; t > 0 && s_ok && i <= i1; i++)
-        s_ok = wait_count(p.done + i, t * p.inst_n[i], a.status);
+    if (wib == 0) {
+      bool ok = true, live = t == 0;
+      const volatile uint32_t *before = p.active + (t & 1) * p.ninst;
+      for (uint32_t i = i0 + lane; t > 0 && ok && i <= i1; i += 32) {
+        ok = wait_count(p.done + i, t * p.inst_n[i], a.status);
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        live |= before[i] == t;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      live = __any_sync(0xffffffffu, live);
       asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      if (lane == 0) {
+        s_ok = ok;
+        s_quiet = !live;
+      }
     }
     __syncthreads();
     if (!s_ok) break;  // a wait gave up: the launch winds down
     const int cur = p.cur0 ^ (int)(t & 1);
-    const uint8_t *st_rd = p.st[cur];
-    const int32_t *d_rd = p.dy[cur];
     const uint32_t *inf_rd = p.inf[cur];
-    uint8_t *st_wr = p.st[1 - cur];
-    int32_t *d_wr = p.dy[1 - cur];
     uint32_t *inf_wr = p.inf[1 - cur];
     const uint32_t step = p.step0 + t;
-    for (uint64_t c0 = a0 + (uint64_t)wib * 32 * ILP; c0 < a1; c0 += (uint64_t)wpb * 32 * ILP)
-      sir_chunk<ILP>(a, st_rd, d_rd, inf_rd, st_wr, d_wr, inf_wr, c0, step, p.is_heavy,
-                     atomic_bits);
-    if (p.nheavy) {  // the range's heavy agents, a warp each
+    uint32_t *active = p.active + ((t + 1) & 1) * p.ninst;
+    const bool quiet = s_quiet;
+    if (quiet) {
+      for (uint64_t w = a0 / 32 + threadIdx.x; w * 32 < a1; w += blockDim.x) inf_wr[w] = 0;
+    } else {
+      const uint64_t c0 = a0 + (uint64_t)wib * 32 * p.rounds;
+      if (c0 < a1) sir_warp<U>(p, inf_rd, inf_wr, c0, a1, step, active, t + 1, s_warp[wib]);
+    }
+    if (p.nheavy && !quiet) {  // the range's heavy agents, a warp each
       uint64_t lo = 0, hi = p.nheavy;  // first heavy agent >= a0
       while (lo < hi) {
         const uint64_t mid = (lo + hi) / 2;
@@ -305,8 +435,7 @@ __global__ void k_batch_persist(PersistArgs p) {
       }
       for (uint64_t h = lo + wib; h < p.nheavy && p.heavy[h] < a1; h += wpb) {
         const uint64_t i = p.heavy[h];
-        const uint8_t s = st_rd[i];
-        const int32_t d = d_rd[i];
+        const uint8_t s = p.st[i];
         uint32_t k = 0;
         if (s == 0) {
           const uint32_t e = a.rp[i + 1];
@@ -314,12 +443,14 @@ __global__ void k_batch_persist(PersistArgs p) {
         }
         k = __reduce_add_sync(0xffffffffu, k);
         if (lane == 0) {
-          const uint8_t ns = sir_rule(a, i, k, s, d, step, st_wr, d_wr);
+          const uint8_t ns = sir_rule_in_place(a, i, k, s, step, p.st, p.dy);
           const unsigned bit = 1u << (i & 31);
-          if (ns == 1)
+          if (ns == 1) {
             atomicOr(inf_wr + (i >> 5), bit);
-          else
+            ((volatile uint32_t *)active)[a.inst[i]] = t + 1;
+          } else {
             atomicAnd(inf_wr + (i >> 5), ~bit);
+          }
         }
       }
     }
@@ -412,6 +543,9 @@ template <int ILP>
 __global__ void __launch_bounds__(512) k_batch_cluster(ClusterArgs p) {
   extern __shared__ uint32_t smask[];  // [2][wmax]
   __shared__ uint32_t s_pack;
+  // [t & 1]: t when an agent of the pack is infected before step t (every
+  // CTA's copy is stored by the warps that find one)
+  __shared__ uint32_t s_live[2];
   const BatchArgs &a = p.a;
   const unsigned csize = cluster_size(), crank = cluster_rank();
   const unsigned lane = threadIdx.x & 31;
@@ -441,13 +575,17 @@ __global__ void __launch_bounds__(512) k_batch_cluster(ClusterArgs p) {
         if (lane < csize) st_cluster(smask + D.word, lane, m);
       }
     }
+    if (threadIdx.x < 2) s_live[threadIdx.x] = 0;
     cluster_sync();
+    // one buffer, as in the persistent form; a pack without an infected agent
+    // is finished
+    uint8_t *st_wr = p.st[p.cur0 ^ (int)(p.steps & 1)];
+    int32_t *d_wr = p.dy[p.cur0 ^ (int)(p.steps & 1)];
     for (uint32_t t = 0; t < p.steps; t++) {
-      const int cur = p.cur0 ^ (int)(t & 1);
-      const uint8_t *st_rd = p.st[cur];
-      const int32_t *d_rd = p.dy[cur];
-      uint8_t *st_wr = p.st[1 - cur];
-      int32_t *d_wr = p.dy[1 - cur];
+      if (t > 0 && s_live[t & 1] != t) break;  // the whole cluster
+      const uint8_t *st_rd = t ? st_wr : p.st[p.cur0];
+      const int32_t *d_rd = t ? d_wr : p.dy[p.cur0];
+      const bool in_place = st_rd == st_wr;
       const uint32_t *m_rd = smask + (t & 1) * p.wmax;
       uint32_t *m_wr = smask + ((t + 1) & 1) * p.wmax;
       const uint32_t step = p.step0 + t;
@@ -464,7 +602,7 @@ __global__ void __launch_bounds__(512) k_batch_cluster(ClusterArgs p) {
           live[u] = lane < D[u].n;
           const uint32_t i = D[u].first + lane;
           s[u] = live[u] ? st_rd[i] : (uint8_t)3;
-          d[u] = live[u] ? d_rd[i] : 0;
+          d[u] = live[u] && !in_place ? d_rd[i] : 0;
           k[u] = 0;
           q[u] = e[u] = 0;
           if (s[u] == 0) {
@@ -495,9 +633,15 @@ __global__ void __launch_bounds__(512) k_batch_cluster(ClusterArgs p) {
         for (int u = 0; u < ILP; u++) {
           if (c0 + u >= c_hi) break;  // warp-uniform
           uint8_t ns = 3;
-          if (live[u]) ns = sir_rule(a, D[u].first + lane, k[u], s[u], d[u], step, st_wr, d_wr);
+          const uint32_t i = D[u].first + lane;
+          if (live[u])
+            ns = in_place ? sir_rule_in_place(a, i, k[u], s[u], step, st_wr, d_wr)
+                          : sir_rule(a, i, k[u], s[u], d[u], step, st_wr, d_wr);
           const unsigned m = __ballot_sync(0xffffffffu, live[u] && ns == 1);
-          if (lane < csize) st_cluster(m_wr + D[u].word, lane, m);
+          if (lane < csize) {
+            st_cluster(m_wr + D[u].word, lane, m);
+            if (m) st_cluster(s_live + ((t + 1) & 1), lane, t + 1);
+          }
         }
       }
       cluster_sync();
@@ -582,7 +726,7 @@ struct vg_batch {
   float tuned_graph_ms = 0, tuned_persistent_ms = 0, tuned_cluster_ms = 0;  // best trials
   std::vector<uint32_t> host_rp;       // arena row pointers (autotuner, buckets)
   uint32_t heavy_thr = 0xFFFFFFFFu;    // threshold the heavy list was built for
-  DevBuf heavy, is_heavy, bar;
+  DevBuf heavy, is_heavy, bar, active;
   DevBuf done, inst_n;  // persistent form: agent-steps finished per instance, agents per instance
   uint64_t nheavy = 0;
   DevBuf scratch_st[2], scratch_dy[2], scratch_inf[2];  // autotuner trials run on copies
@@ -668,14 +812,14 @@ void build_buckets(vg_batch *b, uint32_t thr) {
   VG_CUDA(cudaStreamSynchronize(b->stream));
 }
 
-// one cooperative launch of `steps` steps from buffer `cur` of `bufs`, the
-// first with transition number step0, ilp agents per lane (1, 2 or 4)
-template <int ILP>
-void launch_persistent_ilp(vg_batch *b, const PersistArgs &p, int tpb) {
+// one cooperative launch; U sources per lane and round
+template <int U>
+void launch_persistent_u(vg_batch *b, const PersistArgs &p, int tpb) {
   int dev = 0, sms = 0, per_sm = 0;
   VG_CUDA(cudaGetDevice(&dev));
   VG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_persist<ILP>, tpb, 0));
+  const size_t smem = (size_t)(tpb / 32) * sizeof(WarpShared);
+  VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_persist<U>, tpb, smem));
   if (per_sm < 1) fail(VG_ERR_CUDA, "persistent batch kernel: no block fits an SM");
   // every block resident: a ticket may wait for blocks holding earlier tickets
   unsigned grid = (unsigned)(sms * per_sm);
@@ -683,43 +827,61 @@ void launch_persistent_ilp(vg_batch *b, const PersistArgs &p, int tpb) {
   VG_CUDA(cudaMemsetAsync(b->done.p, 0, (uint64_t)b->n * 4, b->stream));
   PersistArgs q = p;
   void *args[] = {&q};
-  VG_CUDA(cudaLaunchCooperativeKernel((const void *)k_batch_persist<ILP>, dim3(grid), dim3(tpb),
-                                      args, 0, b->stream));
+  VG_CUDA(cudaLaunchCooperativeKernel((const void *)k_batch_persist<U>, dim3(grid), dim3(tpb),
+                                      args, smem, b->stream));
 }
 
+void launch_step(vg_batch *, const BatchArgs &a, int tpb, int ilp, cudaStream_t st);
+
+// `steps` steps from buffer `cur` of `bufs`, the first with transition number
+// step0; ilp (1, 2 or 4): 4 ilp sources per lane and round
 void launch_persistent(vg_batch *b, const StateBufs &bufs, int cur, uint32_t step0,
                        uint32_t steps, int tpb, uint32_t thr, int ilp, int rounds) {
   build_buckets(b, thr);
   if (!b->bar.p) b->bar.alloc(16, &b->footprint);
   if (!b->done.p) {
     b->done.alloc((uint64_t)b->n * 4, &b->footprint);
+    b->active.alloc((uint64_t)b->n * 8, &b->footprint);
+    VG_CUDA(cudaMemsetAsync(b->active.p, 0, (uint64_t)b->n * 8, b->stream));
     b->inst_n.alloc((uint64_t)b->n * 4, &b->footprint);
     std::vector<uint32_t> nn(b->N.begin(), b->N.end());
     VG_CUDA(cudaMemcpyAsync(b->inst_n.p, nn.data(), nn.size() * 4, cudaMemcpyHostToDevice,
                             b->stream));
     VG_CUDA(cudaStreamSynchronize(b->stream));
   }
+  if (steps & 1) {  // the state ends in the other buffer
+    BatchArgs a = batch_args(b, cur, step0, nullptr);
+    a.st_rd = bufs.st[cur];
+    a.d_rd = bufs.dy[cur];
+    a.inf_rd = bufs.inf[cur];
+    a.st_wr = bufs.st[1 - cur];
+    a.d_wr = bufs.dy[1 - cur];
+    a.inf_wr = bufs.inf[1 - cur];
+    launch_step(b, a, b->tpb, b->apt, b->stream);
+    VG_CUDA(cudaGetLastError());
+    cur = 1 - cur;
+    step0++;
+    steps--;
+  }
   // the tickets of a launch (tickets per step x steps) and an instance's
   // agent-steps (steps x N) are counted in 32 bits: longer runs take
   // several launches, each starting from the state the last one left
-  rounds = std::max(rounds, 1);
-  const uint64_t span = (uint64_t)tpb * (uint64_t)ilp * (uint64_t)rounds;
+  rounds = std::min(std::max(rounds, 1), WARP_WORDS);
+  const uint64_t span = (uint64_t)tpb * (uint64_t)rounds;
   const uint64_t tps = (b->total + span - 1) / span;
   const uint64_t maxn = (uint64_t)*std::max_element(b->N.begin(), b->N.end());
   const uint64_t lim = 0xFFFFFFFFull;
   const uint64_t tlim = lim - (1ull << 20);  // room for every block's last (unused) ticket
   const uint32_t chunk =
-      (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(lim / std::max<uint64_t>(maxn, 1),
-                                                         tlim / std::max<uint64_t>(tps, 1)));
+      (uint32_t)std::max<uint64_t>(2, std::min<uint64_t>(lim / std::max<uint64_t>(maxn, 1),
+                                                         tlim / std::max<uint64_t>(tps, 1)) & ~1ull);
   for (uint32_t done = 0; done < steps;) {
     const uint32_t c = std::min(steps - done, chunk);
     PersistArgs p{};
     p.a = batch_args(b, cur, step0 + done, nullptr);
-    for (int k = 0; k < 2; k++) {
-      p.st[k] = bufs.st[k];
-      p.dy[k] = bufs.dy[k];
-      p.inf[k] = bufs.inf[k];
-    }
+    p.st = bufs.st[cur];
+    p.dy = bufs.dy[cur];
+    for (int k = 0; k < 2; k++) p.inf[k] = bufs.inf[k];
     p.cur0 = cur;
     p.steps = c;
     p.step0 = step0 + done;
@@ -729,13 +891,14 @@ void launch_persistent(vg_batch *b, const StateBufs &bufs, int cur, uint32_t ste
     p.ticket = b->bar.as<unsigned>();
     p.done = b->done.as<uint32_t>();
     p.inst_n = b->inst_n.as<uint32_t>();
-    p.rounds = (unsigned)rounds;
+    p.active = b->active.as<uint32_t>();
+    p.ninst = (uint32_t)b->n;
+    p.rounds = rounds;
     switch (ilp) {
-      case 1: launch_persistent_ilp<1>(b, p, tpb); break;
-      case 2: launch_persistent_ilp<2>(b, p, tpb); break;
-      default: launch_persistent_ilp<4>(b, p, tpb); break;
+      case 1: launch_persistent_u<4>(b, p, tpb); break;
+      case 2: launch_persistent_u<8>(b, p, tpb); break;
+      default: launch_persistent_u<16>(b, p, tpb); break;
     }
-    if (c % 2) cur = 1 - cur;
     done += c;
   }
 }
@@ -911,10 +1074,11 @@ void launch_step(vg_batch *, const BatchArgs &a, int tpb, int ilp, cudaStream_t 
 // Choose the launch form by timing candidates on copies of the current
 // state (the simulation state is not touched): per-step launches (block
 // size 128/256/512 x agents per lane 1/2/4, replayed from a CUDA graph when
-// stepping) and the persistent launch (block size 256/512 x agents per lane
-// 1/2/4 x bucket threshold: none, or a warp for each agent above 64
-// in-edges).  Keyed on the arena's agents, edges and in-degree histogram
-// (log2 buckets).
+// stepping), the persistent launch (block size 256/512 x row loads per lane
+// 4/8/16 x mask words per warp 2/4/8 x bucket threshold: none, or a warp for
+// each agent above 64 in-edges) and the cluster launch; each form's best shape
+// over a few steps, then the forms over more.  Keyed on the arena's agents,
+// edges and in-degree histogram (log2 buckets).
 void autotune(vg_batch *b) {
   if (b->host_rp.empty()) {
     b->host_rp.resize(b->total + 1);
@@ -984,23 +1148,24 @@ void autotune(vg_batch *b) {
     VG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     return ms;
   };
+  auto per_step = [&](uint32_t steps, int tpb, int ilp) {
+    for (uint32_t t = 0; t < steps; t++) {
+      BatchArgs a = batch_args(b, 0, (uint32_t)b->step + t, nullptr);
+      const int c = (int)(t & 1);
+      a.st_rd = sb.st[c];
+      a.d_rd = sb.dy[c];
+      a.inf_rd = sb.inf[c];
+      a.st_wr = sb.st[1 - c];
+      a.d_wr = sb.dy[1 - c];
+      a.inf_wr = sb.inf[1 - c];
+      launch_step(b, a, tpb, ilp, b->stream);
+    }
+  };
   float best = 1e30f;
   int bt = 256, ba = 1;
   for (int tpb : {128, 256, 512})
     for (int ilp : {1, 2, 4}) {
-      const float ms = timed([&] {
-        for (uint32_t t = 0; t < TRIAL; t++) {
-          BatchArgs a = batch_args(b, 0, (uint32_t)b->step + t, nullptr);
-          const int c = (int)(t & 1);
-          a.st_rd = sb.st[c];
-          a.d_rd = sb.dy[c];
-          a.inf_rd = sb.inf[c];
-          a.st_wr = sb.st[1 - c];
-          a.d_wr = sb.dy[1 - c];
-          a.inf_wr = sb.inf[1 - c];
-          launch_step(b, a, tpb, ilp, b->stream);
-        }
-      });
+      const float ms = timed([&] { per_step(TRIAL, tpb, ilp); });
       if (ms < best) {
         best = ms;
         bt = tpb;
@@ -1048,6 +1213,18 @@ void autotune(vg_batch *b) {
           ci = ilp;
         }
       }
+  // The forms against each other over a longer run: the persistent ones pass
+  // over what no longer changes, the per-step launches do not (512 instances,
+  // us per step: steps 0..10 277 per step and 282 persistent, 30..40 107 and
+  // 82, 80..200 98 and 39).
+  constexpr uint32_t RACE = 96;
+  best = timed([&] { per_step(RACE, bt, ba); }) * TRIAL / RACE;
+  pbest = timed([&] {
+            launch_persistent(b, sb, 0, (uint32_t)b->step, RACE, pt, pthr, pi, pr);
+          }) * TRIAL / RACE;
+  if (cbest < 1e29f)
+    cbest = timed([&] { launch_cluster(b, sb, 0, (uint32_t)b->step, RACE, cc, ct, ci); }) *
+            TRIAL / RACE;
   VG_CUDA(cudaEventDestroy(e0));
   VG_CUDA(cudaEventDestroy(e1));
   check_batch_status(b);

@@ -205,8 +205,9 @@ class Batch:
         check(lib().vg_batch_set_launch(self._h, int(persistent), int(tpb), int(bucket_threshold)))
 
     def set_lanes(self, per_step=0, persistent=0):
-        """Agents per lane (1, 2, 4) of the per-step and persistent grid
-        launches; 0 keeps the autotuner's value."""
+        """Agents per lane (1, 2, 4) of the per-step launches, and lanes' row
+        loads in flight (4, 8, 16 for 1, 2, 4) of the persistent grid launch;
+        0 keeps the autotuner's value."""
         check(lib().vg_batch_set_lanes(self._h, int(per_step), int(persistent)))
 
     def lanes(self):
