@@ -276,7 +276,14 @@ using namespace vg;
 
 static Sim &S(vg_sim *s) {
   if (!s || !s->s) fail(VG_ERR_ARG, "null simulation handle");
+  s->s->calls++;
   return *s->s;
+}
+// for entries that leave every agent as it is
+static Sim &peek(vg_sim *s) {
+  Sim &r = S(s);
+  r.calls--;
+  return r;
 }
 
 static Model &MD(const vg_model *m) {
@@ -492,9 +499,10 @@ int vg_sim_set_stream(vg_sim *h, void *stream) {
 
 int vg_sim_synchronize(vg_sim *h) {
   API_BEGIN
-  S(h).ensure_device();
-  VG_CUDA(cudaStreamSynchronize(S(h).stream));
-  check_device_status(S(h), "asynchronous transition");
+  Sim &s = peek(h);
+  s.ensure_device();
+  VG_CUDA(cudaStreamSynchronize(s.stream));
+  check_device_status(s, "asynchronous transition");
   API_END
 }
 
@@ -681,7 +689,7 @@ int vg_unbind_params(vg_sim *h, const char *transition) {
 
 int vg_push_global(vg_sim *h, const char *name, double v) {
   API_BEGIN
-  S(h).global_series[name].push_back(v);
+  peek(h).global_series[name].push_back(v);
   API_END
 }
 int vg_global_series(vg_sim *h, const char *name, double *out, uint64_t cap,
@@ -907,6 +915,7 @@ int vg_agent_field_device_ptr(vg_sim *h, int nr, int field, void **out) {
   const AgentTypeDesc &ad = s.model->at(nr);
   if (field < 0 || field >= (int)ad.fields.size()) fail(VG_ERR_ARG, "bad field");
   if (!s.initialized) fail(VG_ERR_STATE, "device buffers exist after finish_init!");
+  s.columns_shared = true;  // the caller may write them at any time
   *out = s.agents[nr - 1].rd[field].p;
   API_END
 }

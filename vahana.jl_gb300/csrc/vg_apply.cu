@@ -677,6 +677,7 @@ void set_last_error(const std::string &m);
 
 static Sim &S(vg_sim *s) {
   if (!s || !s->s) fail(VG_ERR_ARG, "null simulation handle");
+  s->s->calls++;
   return *s->s;
 }
 
@@ -702,6 +703,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
   for (auto &t : transitions())
     if (std::strcmp(t.name, tname) == 0) def = &t;
   if (!def) fail(VG_ERR_ARG, std::string("unknown transition ") + tname);
+  s.infected.pending = false;
   validate_refs(s, call, ncall);
   validate_refs(s, read, nread);
   validate_refs(s, write, nwrite);
@@ -878,6 +880,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
   ctx.appends.clear();
   ctx.removals.clear();
   s.num_transitions++;
+  if (s.infected.pending) s.infected.call = s.calls;
   API_END
 }
 

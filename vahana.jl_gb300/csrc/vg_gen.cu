@@ -160,6 +160,7 @@ void set_last_error(const std::string &m);
 
 static Sim &S(vg_sim *s) {
   if (!s || !s->s) fail(VG_ERR_ARG, "null simulation handle");
+  s->s->calls++;
   return *s->s;
 }
 

@@ -317,6 +317,17 @@ struct Sim {
   // (sir_epoch: csr_epoch at that step), so the preceding kernel cannot be
   // writing them.
   uint64_t csr_epoch = 1, sir_epoch = 0;
+  // entries into the library with this simulation that may change agents
+  uint64_t calls = 0;
+  bool columns_shared = false;  // a column's device pointer was handed out
+  // one bit per agent of `type`, set where its state is 1, written by the SIR
+  // step beside the states; it holds for the step that is the very next call
+  struct InfectedMask {
+    DevBuf m[2];
+    int cur = 0, type = 0;
+    uint64_t call = ~1ull;  // the apply! that wrote m[cur]
+    bool pending = false;   // written by an apply! that has not succeeded yet
+  } infected;
   uint64_t footprint = 0;
   std::vector<AgentStore> agents;  // index = nr - 1
   std::vector<EdgeStore> edges;    // index = edge type index

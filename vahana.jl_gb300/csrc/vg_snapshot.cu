@@ -28,6 +28,7 @@ constexpr char MAGIC[8] = {'V', 'G', 'S', 'N', 'A', 'P', '0', '1'};
 
 Sim &S(vg_sim *h) {
   if (!h || !h->s) fail(VG_ERR_ARG, "null simulation");
+  h->s->calls++;
   return *h->s;
 }
 
