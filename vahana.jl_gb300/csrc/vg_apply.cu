@@ -587,25 +587,30 @@ constexpr uint64_t FOLD_SHORT = 2;
 
 int fold_slots(uint64_t nt) { return (int)std::min<uint64_t>(nt, FOLD_SLOTS); }
 size_t fold_bytes(uint64_t nt) {
-  return nt <= FOLD_SHORT ? 0 : fold_slots(nt) * sizeof(FoldCross) + nt * (sizeof(FoldMap) + 8) + 4;
+  return nt <= FOLD_SHORT ? 0
+                          : sizeof(FoldStart) + fold_slots(nt) * sizeof(FoldCross) +
+                                nt * (sizeof(FoldMap) + 8) + 4;
 }
 
 template <bool F64>
 void launch_fold(const RedArgs &a, void *ws, int64_t *oi, double *of, cudaStream_t st) {
   const uint64_t nt = (a.n + FOLD_TILE - 1) / FOLD_TILE;
   if (nt <= FOLD_SHORT) {
-    k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, nullptr, nullptr, nullptr, oi, of);
+    k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, nullptr, nullptr, nullptr, nullptr, oi, of);
     return;
   }
-  FoldCross *cross = (FoldCross *)ws;
+  FoldStart *start = (FoldStart *)ws;
+  FoldCross *cross = (FoldCross *)(start + 1);
   const int nslots = fold_slots(nt);
   FoldMap *maps = (FoldMap *)(cross + nslots);
   float *tsum = (float *)(maps + nt);
   int *frame = (int *)(tsum + nt), *slots = frame + nt;
   k_fold_sums<F64><<<(unsigned)nt, FOLD_TPB, 0, st>>>(a, tsum);
   k_fold_frames<<<1, FOLD_CHAIN_TPB, 0, st>>>(tsum, nt, a.init_f, frame, slots);
-  k_fold_tiles<F64><<<(unsigned)nt, FOLD_TPB, 0, st>>>(a, frame, maps, cross, slots, nslots);
-  k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, frame, maps, cross, oi, of);
+  k_fold_first<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, start);
+  launch_dependent(k_fold_tiles<F64>, (unsigned)nt, FOLD_TPB, st, a, frame, maps, cross, slots,
+                   nslots);
+  k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, frame, maps, cross, start, oi, of);
 }
 
 void run_reduce(Sim &s, RedArgs a, int out_dtype, bool ordered, void *out) {

@@ -18,7 +18,8 @@
 //   k_fold_tiles  the map of each tile in its predicted frame; for a tile
 //                 that is predicted to cross into another binade, the maps
 //                 of its chunks of 64 elements in both
-//   k_fold_chain  one block carries the exact sum through the tiles: up to
+//   k_fold_first  beside k_fold_tiles, the exact sum through the first tile
+//   k_fold_chain  one block carries it through the other tiles: up to
 //                 1024 maps are composed and checked per round; a predicted
 //                 crossing goes through fold_cross (one warp, its chunks'
 //                 maps up to the crossing and behind it), any other tile that
@@ -30,15 +31,16 @@
 // changing its binade falls back to the hardware additions, no slower than the
 // plain loop.
 //
-// Bound: for a few million elements the chain (a round 2 us, a crossing 3.5,
-// the first tile with its eleven crossings 30), beyond that the two passes over
-// the column (k_fold_sums 7 us and k_fold_tiles 19 us for 5e6).  FOLD_TILE:
+// Bound: for a few million elements the chain (a round 2 us, a crossing 3.5),
+// beyond that the two passes over the column (k_fold_sums 7 us and k_fold_tiles
+// 19 us for 5e6).  FOLD_TILE:
 // tiles of 1024, 2048 and 4096 elements took 242, 242 and 270 us for 5e6
 // uniform values, and 15.3, 9.2 and 6.4 ms for 2e6 values whose exponents spread
 // over e^+-300 (there the chain goes tile by tile); 2048 keeps both.  Measured at
 // 5e6 Float64 agents: 181 ms for the plain chain (36 ns per addition), 253 us
 // with every crossing through fold_hard (two attempts of the whole block, 7.5
-// us) and all 1024 maps read and composed in each round (4.3 us), 145 us here;
+// us) and all 1024 maps read and composed in each round (4.3 us), 145 us with the
+// first tile in the chain, 132 here;
 // a sum that cancels to zero at every second addition (2e6): 72.6 and 73.4 ms.
 #pragma once
 
@@ -254,9 +256,8 @@ __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_frames(const float *tsu
 // a tile without a map leaves NO_FRAME in its frame, a crossing with chunk maps
 // its slot in its map's d0
 template <bool F64>
-__global__ void __launch_bounds__(FOLD_TPB) k_fold_tiles(RedArgs a, int *frame, FoldMap *maps,
-                                                         FoldCross *cross, int *slots,
-                                                         int nslots) {
+__device__ __forceinline__ void fold_tile(const RedArgs &a, int *frame, FoldMap *maps,
+                                          FoldCross *cross, int *slots, int nslots) {
   __shared__ double v[FOLD_TILE + FOLD_TPB];  // one pad per thread's elements
   __shared__ uint32_t live[FOLD_TILE / 32];
   __shared__ FoldMap ws[FOLD_TPB / 32];
@@ -332,6 +333,15 @@ __global__ void __launch_bounds__(FOLD_TPB) k_fold_tiles(RedArgs a, int *frame, 
       if (!r.ok) frame[blockIdx.x] = FOLD_NO_FRAME;
     }
   }
+}
+
+// (started beside k_fold_first)
+template <bool F64>
+__global__ void __launch_bounds__(FOLD_TPB) k_fold_tiles(RedArgs a, int *frame, FoldMap *maps,
+                                                         FoldCross *cross, int *slots,
+                                                         int nslots) {
+  fold_tile<F64>(a, frame, maps, cross, slots, nslots);
+  end_after_previous();
 }
 
 struct FoldShared {
@@ -513,6 +523,27 @@ __device__ void fold_hard(const RedArgs &a, uint64_t tile, int start, FoldShared
   }
 }
 
+// The first tile, where a sum that starts at zero crosses a binade every few
+// elements: its sum needs no prediction, so it is taken while the other
+// tiles are mapped (30 us of one block beside 19 of the others).
+struct FoldStart {
+  double a;
+  int step, plain, wait;
+};
+template <bool F64>
+__global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_first(RedArgs a, FoldStart *start) {
+  __shared__ FoldShared S;
+  let_next_start();
+  if (threadIdx.x == 0) {
+    S.a = a.init_f;
+    S.step = S.plain = 0;
+    S.wait = 1;
+  }
+  __syncthreads();
+  fold_hard<F64>(a, 0, 0, S);
+  if (threadIdx.x == 0) *start = {S.a, S.step, S.plain, S.wait};
+}
+
 // A predicted crossing, by warp 0: the maps of the chunks in the sum's frame,
 // one per lane, carry it to the chunk that leaves the binade; that chunk's
 // elements are mapped two per lane, those of the lane that crosses are added by
@@ -582,14 +613,16 @@ __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_chain(RedArgs a, uint64
                                                                const int *frame,
                                                                const FoldMap *maps,
                                                                const FoldCross *cross,
+                                                               const FoldStart *start,
                                                                int64_t *oi, double *of) {
   __shared__ FoldShared S;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
-    S.a = a.init_f;
-    S.next = 0;
-    S.step = S.plain = 0;
-    S.wait = 1;
+    S.a = start ? start->a : a.init_f;
+    S.next = start ? (isnan(start->a) ? ntiles : 1) : 0;
+    S.step = start ? start->step : 0;
+    S.plain = start ? start->plain : 0;
+    S.wait = start ? start->wait : 1;
   }
   __syncthreads();
   while (S.next < ntiles) {
