@@ -608,7 +608,7 @@ void launch_fold(const RedArgs &a, void *ws, int64_t *oi, double *of, cudaStream
   k_fold_sums<F64><<<(unsigned)nt, FOLD_TPB, 0, st>>>(a, tsum);
   k_fold_frames<<<1, FOLD_CHAIN_TPB, 0, st>>>(tsum, nt, a.init_f, frame, slots);
   k_fold_first<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, start);
-  launch_dependent(k_fold_tiles<F64>, (unsigned)nt, FOLD_TPB, st, a, frame, maps, cross, slots,
+  launch_dependent(k_fold_tiles<F64>, (unsigned)nt, FOLD_TPB, 0, st, a, frame, maps, cross, slots,
                    nslots);
   k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, frame, maps, cross, start, oi, of);
 }

@@ -61,6 +61,7 @@ inline size_t bucket_tile_smem(const BucketPlan &p) {
 template <class Source>
 __global__ void __launch_bounds__(BK_TPB) k_bucket_tiles(Source source, BucketPlan p) {
   extern __shared__ __align__(16) unsigned char bk_smem[];
+  let_next_start();
   const uint32_t nb4 = (p.nbuckets + 3) & ~3u;
   uint32_t *srec = (uint32_t *)bk_smem;              // [BK_TILE]
   uint32_t *sval = srec + BK_TILE;                   // [BK_TILE] with VALS
@@ -70,6 +71,9 @@ __global__ void __launch_bounds__(BK_TPB) k_bucket_tiles(Source source, BucketPl
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint64_t t0 = (uint64_t)blockIdx.x * BK_TILE + (uint64_t)w * (32 * BK_IPT) + lane;
   uint32_t row[BK_IPT], val[BK_IPT], rank[BK_IPT];
+  uint2 *z = (uint2 *)wcnt;  // four 16-bit counters per word
+  for (uint32_t i = threadIdx.x; i < BK_WARPS * nb4 / 4; i += BK_TPB) z[i] = make_uint2(0, 0);
+  wait_for_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0) *p.maxdeg = 0;
   unsigned have = 0;
   typename Source::Raw raw[BK_IPT];
@@ -82,8 +86,6 @@ __global__ void __launch_bounds__(BK_TPB) k_bucket_tiles(Source source, BucketPl
     row[k] = val[k] = 0;
     if (i < p.n && source.make(i, raw[k], row[k], val[k])) have |= 1u << k;
   }
-  uint2 *z = (uint2 *)wcnt;  // four 16-bit counters per word
-  for (uint32_t i = threadIdx.x; i < BK_WARPS * nb4 / 4; i += BK_TPB) z[i] = make_uint2(0, 0);
   __syncthreads();
   // rank of each record among the warp's earlier records of its bucket: the
   // lanes with the same label (bucket, and whether there is a record) from
@@ -175,8 +177,7 @@ void launch_bucket_tiles(const Source &src, const BucketPlan &p, cudaStream_t st
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               128 * 1024) == cudaSuccess;
   if (!ok) fail(VG_ERR_CUDA, "cannot reserve the rebuild's shared memory");
-  k_bucket_tiles<Source><<<p.ntiles, BK_TPB, bucket_tile_smem(p), st>>>(src, p);
-  VG_CUDA(cudaGetLastError());
+  launch_dependent(k_bucket_tiles<Source>, p.ntiles, BK_TPB, bucket_tile_smem(p), st, src, p);
 }
 
 }  // namespace vg

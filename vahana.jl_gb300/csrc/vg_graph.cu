@@ -690,6 +690,8 @@ __device__ __forceinline__ void bucket_build(const BuildArgs &a, uint32_t span, 
 
 template <bool MERGE, int Q>
 __global__ void __launch_bounds__(BB_TPB, 6) k_bucket_build(const __grid_constant__ BuildArgs a) {
+  let_next_start();
+  wait_for_previous();
   bucket_build<MERGE, Q>(a, a.span, a.chunk);
 }
 
@@ -725,6 +727,10 @@ __global__ void __launch_bounds__(BB_TPB, 5) k_bucket_rows(const __grid_constant
   const uint32_t tid = threadIdx.x, lane = tid & 31, b = blockIdx.x;
   const BucketPlan &p = a.p;
   uint32_t base = 0, m = 0;
+  let_next_start();
+#pragma unroll
+  for (int q = 0; q < R; q++) cnt4[tid + BB_TPB * q] = make_uint4(0, 0, 0, 0);
+  wait_for_previous();  // (launched beside the end of k_bucket_tiles)
   if (p.ntiles && p.ntiles <= BB_TILES) m = bb_pieces(p, b, 0, pre, first, ws, &base);
   if (p.ntiles > BB_TILES || m > BB_U * BB_TPB || 1u << p.shift != SPAN) {
     __syncthreads();
@@ -732,8 +738,6 @@ __global__ void __launch_bounds__(BB_TPB, 5) k_bucket_rows(const __grid_constant
     bucket_build_apart(a, SPAN / 2, 512);
     return;
   }
-#pragma unroll
-  for (int q = 0; q < R; q++) cnt4[tid + BB_TPB * q] = make_uint4(0, 0, 0, 0);
   __syncthreads();
   const uint64_t R0 = (uint64_t)b << p.shift;
   uint32_t row[BB_U], val[BB_U], arr[BB_U];
@@ -1295,7 +1299,7 @@ static void launch_buckets(const BuildArgs &a, bool merge, cudaStream_t st) {
     return r;
   }();
   if (!ok) fail(VG_ERR_CUDA, "cannot reserve the rebuild's shared memory");
-  k<<<a.p.nbuckets, BB_TPB, smem, st>>>(a);
+  launch_dependent(k, a.p.nbuckets, BB_TPB, smem, st, a);
   VG_CUDA(cudaGetLastError());
 }
 

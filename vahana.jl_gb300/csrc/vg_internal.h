@@ -416,18 +416,23 @@ constexpr size_t PIN_BYTES = 256;
 __device__ __forceinline__ void let_next_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 __device__ __forceinline__ void end_after_previous() {
-  if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (blockIdx.x == gridDim.x - 1) wait_for_previous();
 }
 // a launch that may start before the preceding one of the stream has ended
 template <class... A, class... B>
-void launch_dependent(void (*k)(A...), unsigned grid, unsigned block, cudaStream_t st, B... args) {
+void launch_dependent(void (*k)(A...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      B... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;

@@ -917,7 +917,7 @@ void tr_bounded_confidence(ApplyCtx &c) {
     else k_opinion_long<false, false><<<nl, LONG_TPB, 0, s.stream>>>(p, Notify{});
     VG_CUDA(cudaGetLastError());
     launch_dependent(p.grid ? k_opinion<true, true> : k_opinion<false, true>, grid - nbig, TPB,
-                     s.stream, p);
+                     0, s.stream, p);
   } else if (grid > nbig) {
     if (p.grid) k_opinion<true, false><<<grid - nbig, TPB, 0, s.stream>>>(p);
     else k_opinion<false, false><<<grid - nbig, TPB, 0, s.stream>>>(p);
@@ -1002,7 +1002,7 @@ static void launch_notified(Sim &s, OpinionArgs &p, unsigned grid, Sim::HostExch
     if (p.grid) k_opinion_long<true, true><<<nl, LONG_TPB, 0, s.stream>>>(p, nt);
     else k_opinion_long<false, true><<<nl, LONG_TPB, 0, s.stream>>>(p, nt);
     VG_CUDA(cudaGetLastError());
-    launch_dependent(p.grid ? k_opinion_notify<true, true> : k_opinion_notify<false, true>, grid, TPB,
+    launch_dependent(p.grid ? k_opinion_notify<true, true> : k_opinion_notify<false, true>, grid, TPB, 0,
                      s.stream, p, nt);
   } else {
     if (p.grid) k_opinion_notify<true, false><<<grid, TPB, 0, s.stream>>>(p, nt);
@@ -1180,7 +1180,7 @@ bool launch_opinion_jobs(const OpinionTables &t, const uint8_t *dev, cudaStream_
   if (t.nlong) {
     k_opinion_jobs_long<<<t.nlong, LONG_TPB, 0, st>>>(da, dt + t.ntiles);
     VG_CUDA(cudaGetLastError());
-    launch_dependent(k_opinion_jobs, t.ntiles, TPB, st, da, dt);
+    launch_dependent(k_opinion_jobs, t.ntiles, TPB, 0, st, da, dt);
   } else {
     k_opinion_jobs<<<t.ntiles, TPB, 0, st>>>(da, dt);
   }

@@ -416,7 +416,8 @@ void tick(vg_server *S) {
       const auto *dj = (const SirJobDesc *)(dev + sir_at);
       const auto *dt = (const SirTile *)(dev + tiles_at);
       if (beside)
-        launch_dependent(k_sir_jobs, (unsigned)stiles.size(), 256, st, dj, dt, S->status.as<int>());
+        launch_dependent(k_sir_jobs, (unsigned)stiles.size(), 256, 0, st, dj, dt,
+                         S->status.as<int>());
       else
         k_sir_jobs<<<(unsigned)stiles.size(), 256, 0, st>>>(dj, dt, S->status.as<int>());
       VG_CUDA(cudaGetLastError());

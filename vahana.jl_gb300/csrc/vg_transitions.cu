@@ -855,9 +855,10 @@ __device__ __forceinline__ uint32_t life_rule(uint32_t cnt, uint32_t self) {
 // instructions).
 constexpr int LIFE_ROWS = 8;
 
-__global__ void __launch_bounds__(256) k_life2d_x4(const uint32_t *__restrict__ a,
-                                                   uint32_t *__restrict__ o, int Wq, int64_t H,
-                                                   int periodic) {
+__global__ void __launch_bounds__(256) k_life2d_x4(const uint32_t *a, uint32_t *o, int Wq,
+                                                   int64_t H, int periodic) {
+  let_next_start();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int qx = (int)blockIdx.x * 32 + lane;
   const int64_t y0 = ((int64_t)blockIdx.y * blockDim.y + threadIdx.y) * LIFE_ROWS;
@@ -1064,8 +1065,7 @@ __device__ __forceinline__ uint32_t row_rule(const RowStencil &s, uint32_t self,
 // CODE: the row code of a stencil of one plane (rasters of up to two
 // dimensions), -1: any planes
 template <int D, int CODE>
-__global__ void __launch_bounds__(256, 4) k_life_rows(const uint8_t *__restrict__ a,
-                                                   uint8_t *__restrict__ o,
+__global__ void __launch_bounds__(256, 4) k_life_rows(const uint8_t *a, uint8_t *o,
                                                    const __grid_constant__ RowStencil s) {
   constexpr int ROWS = ROW_TY + 2 * D, LOADS = (ROWS + 7) / 8;
   __shared__ uint32_t t[ROWS * ROW_WORDS];
@@ -1077,6 +1077,8 @@ __global__ void __launch_bounds__(256, 4) k_life_rows(const uint8_t *__restrict_
   const int y0 = (int)(blk % s.ty) * ROW_TY;
   blk /= s.ty;
   const int z = (int)(blk % (uint32_t)Z), v = (int)(blk / (uint32_t)Z);
+  let_next_start();
+  wait_for_previous();
   uint32_t acc[ROW_RY], self[ROW_RY];
 #pragma unroll
   for (int j = 0; j < ROW_RY; j++) acc[j] = self[j] = 0;
@@ -1848,8 +1850,8 @@ void tr_life(ApplyCtx &c) {
     dim3 blk(32, 8);
     dim3 grd((unsigned)((Wq + 31) / 32),
              (unsigned)((st.dims[1] + 8 * LIFE_ROWS - 1) / (8 * LIFE_ROWS)));
-    k_life2d_x4<<<grd, blk, 0, s.stream>>>((const uint32_t *)in, (uint32_t *)out, (int)Wq,
-                                          st.dims[1], st.periodic);
+    launch_dependent(k_life2d_x4, grd, blk, 0, s.stream, (const uint32_t *)in, (uint32_t *)out,
+                     (int)Wq, st.dims[1], st.periodic);
   } else if (ad.fields[0].dtype == VG_BOOL && rows_pay(st, R.ncells, moore2d) &&
              row_stencil(st, birth, survive, rs, reach)) {
     const uint64_t blocks = (uint64_t)rs.tx * rs.ty * rs.dims[2] * rs.dims[3];
@@ -1861,7 +1863,7 @@ void tr_life(ApplyCtx &c) {
     if (reach == 1 && code == row_code(1, 0, -1)) k = k_life_rows<1, row_code(1, 0, -1)>;
     if (reach == 2 && code == row_code(2, 2, 2)) k = k_life_rows<2, row_code(2, 2, 2)>;
     if (reach == 2 && code == row_code(2, 1, 0)) k = k_life_rows<2, row_code(2, 1, 0)>;
-    k<<<(unsigned)blocks, blk, 0, s.stream>>>(in, out, rs);
+    launch_dependent(k, (unsigned)blocks, blk, 0, s.stream, in, out, rs);
   } else if (moore2d) {
     dim3 blk(32, 8);
     dim3 grd((unsigned)((st.dims[0] + 31) / 32), (unsigned)((st.dims[1] + 7) / 8));
