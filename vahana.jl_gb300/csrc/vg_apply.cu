@@ -342,6 +342,7 @@ template <class E>
 __global__ void __launch_bounds__(TPB) k_reduce_partial(RedArgs a, int64_t *pi, double *pf) {
   __shared__ int64_t si[TPB / 32];
   __shared__ double sf[TPB / 32];
+  let_next_start();
   const bool keys = a.float_acc && (a.op == VG_OP_MAX || a.op == VG_OP_MIN);
   const bool sums = a.float_acc && !keys;
   const int64_t neut_i = keys ? red_key(a.neut_f) : a.neut_i;
@@ -440,6 +441,7 @@ __global__ void __launch_bounds__(RED_BLOCKS) k_reduce_final(const int64_t *pi, 
   __shared__ int64_t si[32];
   __shared__ double sf[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  wait_for_previous();
   const double fill = a.op == VG_OP_ADD ? -0.0 : a.neut_f;
   const bool keys = a.float_acc && (a.op == VG_OP_MAX || a.op == VG_OP_MIN);
   const bool sums = a.float_acc && !keys;
@@ -606,11 +608,12 @@ void launch_fold(const RedArgs &a, void *ws, int64_t *oi, double *of, cudaStream
   float *tsum = (float *)(maps + nt);
   int *frame = (int *)(tsum + nt), *slots = frame + nt;
   k_fold_sums<F64><<<(unsigned)nt, FOLD_TPB, 0, st>>>(a, tsum);
-  k_fold_frames<<<1, FOLD_CHAIN_TPB, 0, st>>>(tsum, nt, a.init_f, frame, slots);
-  k_fold_first<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, start);
+  launch_dependent(k_fold_frames, 1, FOLD_CHAIN_TPB, 0, st, tsum, nt, a.init_f, frame, slots);
+  launch_dependent(k_fold_first<F64>, 1, FOLD_CHAIN_TPB, 0, st, a, start);
   launch_dependent(k_fold_tiles<F64>, (unsigned)nt, FOLD_TPB, 0, st, a, frame, maps, cross, slots,
                    nslots);
-  k_fold_chain<F64><<<1, FOLD_CHAIN_TPB, 0, st>>>(a, nt, frame, maps, cross, start, oi, of);
+  launch_dependent(k_fold_chain<F64>, 1, FOLD_CHAIN_TPB, 0, st, a, nt, frame, maps, cross, start,
+                   oi, of);
 }
 
 void run_reduce(Sim &s, RedArgs a, int out_dtype, bool ordered, void *out) {
@@ -645,7 +648,7 @@ void run_reduce(Sim &s, RedArgs a, int out_dtype, bool ordered, void *out) {
         case VG_F64: k_reduce_partial<double><<<nb, TPB, 0, s.stream>>>(a, pi, pf); break;
         default: k_reduce_partial<int64_t><<<nb, TPB, 0, s.stream>>>(a, pi, pf);
       }
-      k_reduce_final<<<1, RED_BLOCKS, 0, s.stream>>>(pi, pf, nb, a, oi, of);
+      launch_dependent(k_reduce_final, 1, RED_BLOCKS, 0, s.stream, pi, pf, nb, a, oi, of);
     }
     VG_CUDA(cudaGetLastError());
     int64_t res[2];

@@ -198,6 +198,7 @@ __device__ __forceinline__ bool fold_load(const RedArgs &a, uint64_t i, double *
 template <bool F64>
 __global__ void __launch_bounds__(FOLD_TPB) k_fold_sums(RedArgs a, float *tsum) {
   __shared__ float ws[FOLD_TPB / 32];
+  let_next_start();
   const uint64_t base = (uint64_t)blockIdx.x * FOLD_TILE;
   double v[FOLD_PER];
 #pragma unroll
@@ -222,6 +223,8 @@ __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_frames(const float *tsu
                                                                 double init, int *frame,
                                                                 int *slots) {
   __shared__ float ws[32];
+  let_next_start();
+  wait_for_previous();
   if (threadIdx.x == 0) *slots = 0;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float carry = fold_approx(init);
@@ -340,6 +343,7 @@ template <bool F64>
 __global__ void __launch_bounds__(FOLD_TPB) k_fold_tiles(RedArgs a, int *frame, FoldMap *maps,
                                                          FoldCross *cross, int *slots,
                                                          int nslots) {
+  let_next_start();
   fold_tile<F64>(a, frame, maps, cross, slots, nslots);
   end_after_previous();
 }
@@ -533,6 +537,7 @@ struct FoldStart {
 template <bool F64>
 __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_first(RedArgs a, FoldStart *start) {
   __shared__ FoldShared S;
+  wait_for_previous();  // (before the mapping may start: it reads the frames)
   let_next_start();
   if (threadIdx.x == 0) {
     S.a = a.init_f;
@@ -617,6 +622,7 @@ __global__ void __launch_bounds__(FOLD_CHAIN_TPB) k_fold_chain(RedArgs a, uint64
                                                                int64_t *oi, double *of) {
   __shared__ FoldShared S;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  wait_for_previous();
   if (threadIdx.x == 0) {
     S.a = start ? start->a : a.init_f;
     S.next = start ? (isnan(start->a) ? ntiles : 1) : 0;
