@@ -79,3 +79,37 @@ def test_mask(vh, n, degree, queued):
                                                 vh.read_agents(c, "Person")[0].values())))
     steps(2)
     same(vh, a, b)
+
+
+def test_recorded_steps(vh):
+    """Two steps recorded in a CUDA graph and replayed after the states were
+    written, then steps again: as the same steps made directly."""
+    import torch
+    n = 40_000
+    rng = np.random.default_rng(5)
+    a, b = build(vh, n, 12, 9), build(vh, n, 12, 9)
+    stream = torch.cuda.Stream()
+    vh.set_stream(a.sim, stream.cuda_stream)
+    for r in (a, b):
+        vh.set_async(r.sim, True)
+        for _ in range(4):
+            r.step()
+        vh.synchronize(r.sim)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        a.step()
+        a.step()
+    new = {"state": rng.choice([0, 0, 0, 1, 2], n).astype(np.uint8),
+           "days": rng.integers(0, 3, n).astype(np.int32)}
+    for r in (a, b):
+        vh.write_agents(r.sim, "Person", **new)
+        vh.synchronize(r.sim)
+    graph.replay()
+    torch.cuda.synchronize()
+    b.step()
+    b.step()
+    same(vh, a, b)
+    for r in (a, b):
+        r.step()
+        r.step()
+    same(vh, a, b)

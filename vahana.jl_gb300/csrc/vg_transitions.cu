@@ -1716,7 +1716,12 @@ void tr_sir(ApplyCtx &c) {
   cfg.numAttrs = s.sir_epoch == s.csr_epoch ? 1 : 0;
   Sim::InfectedMask &inf = s.infected;
   const size_t words = (a.n + 31) / 32 * 4;
-  const bool mask = inf.call + 1 == s.calls && inf.type == c.call_type && !s.columns_shared &&
+  // (a recorded step may be replayed after anything: it reads the states, and
+  // what follows the recording does not take its mask for done)
+  cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+  VG_CUDA(cudaStreamIsCapturing(s.stream, &recording));
+  const bool direct = recording == cudaStreamCaptureStatusNone && !s.columns_shared;
+  const bool mask = direct && inf.call + 1 == s.calls && inf.type == c.call_type &&
                     inf.m[inf.cur].bytes >= words;
   const bool early = v.nedges < SIR_EARLY_EDGES;
   auto kernel = mask ? (early ? k_sir<true, true> : k_sir<true, false>)
@@ -1732,7 +1737,7 @@ void tr_sir(ApplyCtx &c) {
                              inf.m[1 - inf.cur].as<uint32_t>()));
   inf.cur = 1 - inf.cur;
   inf.type = c.call_type;
-  inf.pending = true;
+  inf.pending = direct;
   s.sir_epoch = s.csr_epoch;
 }
 
