@@ -78,6 +78,9 @@ struct OpinionArgs {
   uint32_t long_slots;
   uint32_t hub_thr;
   unsigned hub_blocks;   // blocks of the other hub rows, 4 per block
+  // order of the slice blocks (slice_block): blocks of a window, full windows,
+  // first blocks of each that run ahead of all others (0: none do), all blocks
+  unsigned wblocks, nwindows, ahead, slice_blocks;
   double eps, a, b;
   int a_pow2, b_pow2, a_k, b_k;  // a = 2^a_k, b = 2^b_k (positive normal powers of two)
   float eps_lo, eps_hi;  // float filter: certainly inside / certainly outside
@@ -567,6 +570,21 @@ __device__ __noinline__ void hub_block(const OpinionArgs &p, uint32_t r) {
 // The work of one block of the gather grid: hub warps, then slices (one
 // per warp).  Shared by the single-simulation kernel and the multi-job
 // kernel of the serving loop.
+// The slice block that launch block b takes.  The first blocks of a window hold
+// its longest slices; in the windows' order those of the last windows would
+// start last and end the launch alone, so the first `ahead` blocks of every
+// window run before all others (and those of the last window, not full).
+__device__ __forceinline__ unsigned slice_block(const OpinionArgs &p, unsigned b) {
+  if (!p.ahead) return b;
+  const unsigned W = p.wblocks, h = p.ahead, nw = p.nwindows;
+  const unsigned rest = p.slice_blocks - nw * W;
+  if (b < rest) return nw * W + b;
+  b -= rest;
+  if (b < nw * h) return b % nw * W + b / nw;
+  b -= nw * h;
+  return b / (W - h) * W + h + b % (W - h);
+}
+
 // BIG: the block range starts with the block-wide hub rows; otherwise they
 // are run by their own launch (k_opinion_big) and the range starts at the
 // warp hubs, so that this kernel needs no shared memory (its L1 keeps the
@@ -587,7 +605,9 @@ __device__ __forceinline__ void opinion_block(const OpinionArgs &p, unsigned blk
     if (h < p.nhub) hub_warp<GRID>(p, p.hub_rows[h]);
     return;
   }
-  const uint64_t sl = warp - (uint64_t)p.hub_blocks * (TPB / 32);
+  const uint64_t sl = LONG ? (uint64_t)slice_block(p, blk - p.hub_blocks) * (TPB / 32) +
+                                 (threadIdx.x >> 5)
+                           : warp - (uint64_t)p.hub_blocks * (TPB / 32);
   if (sl < p.nslices && !(LONG && p.slice_deg[sl] >= p.long_slots)) sell_slice<GRID>(p, sl);
 }
 
@@ -772,9 +792,10 @@ __global__ void __launch_bounds__(TPB, 9) k_opinion_notify(OpinionArgs p, Notify
   opinion_block<GRID, false, LONG>(p, blockIdx.x);
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned b = blockIdx.x;
+    unsigned b = blockIdx.x;
     unsigned r = nt.nranges;  // the hub warps
     if (b >= nt.hub_blocks) {
+      if (LONG) b = nt.hub_blocks + slice_block(p, b - nt.hub_blocks);
       r = 0;
       while (r + 1 < nt.nranges && b >= nt.end[r]) r++;
     }
@@ -846,6 +867,16 @@ static unsigned opinion_args(Sim &s, int e, int T, double eps, double a, double 
                              uint32_t thr, uint32_t big_thr, OpinionArgs &p,
                              cudaStream_t launch_stream);
 
+// Where the first blocks of the windows run ahead: launches whose last slices
+// are a good part of them and whose opinions stay in L2 in any order.  Measured,
+// us per step in the windows' order and so: host-made graphs (degrees of a
+// narrow distribution with a heavy end) 10^6 agents with 2*10^7 edges 167 and
+// 133, with 8*10^6 84 and 66, 3*10^5 with 6*10^6 75 and 76; power-law graphs
+// 10^6 with 2*10^7 118 and 119, 1.5*10^6 with 3*10^7 159 and 165, 3*10^6 with
+// 6*10^7 298 and 302.  3 or 12 blocks: 139 and 129 for the first, 160 and 176 for
+// the last but one.
+constexpr unsigned AHEAD_BLOCKS = 6;
+constexpr uint64_t AHEAD_EDGES = 24000000;
 // which slices and hub rows take a block each, in a launch over `edges`
 // edges; returns the grid of the other blocks
 static unsigned split_long(OpinionArgs &p, uint64_t edges) {
@@ -859,6 +890,10 @@ static unsigned split_long(OpinionArgs &p, uint64_t edges) {
   const uint64_t hubs = at_least(p.csr->long_hubs, 32 * p.long_slots);
   p.long_hubs = hubs > p.nbig ? (unsigned)(hubs - p.nbig) : 0;
   p.hub_blocks = (unsigned)((p.nhub - p.nbig - p.long_hubs + (TPB / 32) - 1) / (TPB / 32));
+  p.slice_blocks = (unsigned)((p.nslices + (TPB / 32) - 1) / (TPB / 32));
+  p.wblocks = (1u << p.csr->wshift) / TPB;
+  p.nwindows = p.wblocks ? p.slice_blocks / p.wblocks : 0;
+  p.ahead = edges < AHEAD_EDGES && p.wblocks > AHEAD_BLOCKS && p.nwindows ? AHEAD_BLOCKS : 0;
   return (unsigned)p.nbig + p.hub_blocks + (unsigned)((p.nslices + (TPB / 32) - 1) / (TPB / 32));
 }
 
