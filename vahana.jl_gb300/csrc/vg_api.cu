@@ -155,10 +155,19 @@ PinPool &pins() {
 }  // namespace
 
 void Sim::fetch(void *dst, const void *src, size_t bytes) {
-  void *to = pin && bytes <= PIN_BYTES - 64 ? pin + 64 : dst;
+  void *to = pin && bytes <= PIN_FETCH ? pin + 64 : dst;
   VG_CUDA(cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, stream));
   VG_CUDA(cudaStreamSynchronize(stream));
   if (to != dst) std::memcpy(dst, to, bytes);
+}
+
+void *Sim::results(size_t bytes) {
+  return pin && bytes <= PIN_RESULTS ? pin_dev + 64 + PIN_FETCH : work(WORK_TOTALS, bytes);
+}
+void Sim::read_results(void *dst, const void *res, size_t bytes) {
+  if (!pin || res != pin_dev + 64 + PIN_FETCH) return fetch(dst, res, bytes);
+  VG_CUDA(cudaStreamSynchronize(stream));
+  std::memcpy(dst, pin + 64 + PIN_FETCH, bytes);
 }
 
 void Sim::ensure_device() {
@@ -173,6 +182,7 @@ void Sim::ensure_device() {
   if (pin) {
     void *d = nullptr;
     VG_CUDA(cudaHostGetDevicePointer(&d, pin, 0));
+    pin_dev = (char *)d;
     w.host = (int *)d;
   }
   VG_CUDA(cudaMemcpyAsync(d_status.p, &w, sizeof(w), cudaMemcpyHostToDevice, stream));

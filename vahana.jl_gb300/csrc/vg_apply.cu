@@ -309,11 +309,12 @@ __device__ __forceinline__ bool key_is_nan(int64_t k) {
 // loads in flight per thread, and one loop per operator: the operator, the
 // comparison and the accumulator's type are chosen once per RED_U elements.
 // The elements of a thread are folded in index order.  Bound: memory latency
-// (a thread has two or three batches of loads; 5e6 elements occupy every SM
-// once).  Measured at 5e6 mortal agents, operator looked up per element and
-// Float max by three binary64 operations each before, now: Float64 max 50
-// and 13 us, a comparison of UInt8 counted 22 and 14, Int32 sum 21 and 14.
-constexpr int RED_U = 8;
+// (5e6 elements occupy every SM once).  Measured at 5e6 agents, operator looked
+// up per element and Float max by three binary64 operations each before, now:
+// Float64 max 50 and 13 us, a comparison of UInt8 counted 22 and 11, Int32 sum
+// 21 and 9; with 2, 8 and 16 loads in flight the last takes 11, 14.5 and 19
+// (registers).
+constexpr int RED_U = 4;
 
 // a comparison with the reduction's threshold: below, equal, above, unordered
 struct RedCmp {
@@ -625,8 +626,8 @@ void run_reduce(Sim &s, RedArgs a, int out_dtype, bool ordered, void *out) {
     // the simulation's workspace: the result, then partials or tile maps
     char *d = (char *)s.scratch(64 + std::max<uint64_t>(2 * 8 * RED_BLOCKS,
                                                         fold_bytes(tiles)));
-    int64_t *oi = (int64_t *)d;
-    double *of = (double *)(d + 8);
+    int64_t *oi = (int64_t *)s.results(16);
+    double *of = (double *)(oi + 1);
     if (ordered && a.float_acc && a.op == VG_OP_ADD) {
       if (a.dt == VG_F64 && a.kind == VG_MAP_FIELD) launch_fold<true>(a, d + 64, oi, of, s.stream);
       else launch_fold<false>(a, d + 64, oi, of, s.stream);
@@ -652,7 +653,7 @@ void run_reduce(Sim &s, RedArgs a, int out_dtype, bool ordered, void *out) {
     }
     VG_CUDA(cudaGetLastError());
     int64_t res[2];
-    s.fetch(res, d, 16);
+    s.read_results(res, oi, 16);
     ri = res[0];
     std::memcpy(&rf, &res[1], 8);
   }
@@ -812,7 +813,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
         may_die_types.push_back(T);
   if (!may_die_types.empty()) {
     deaths.resize(may_die_types.size());
-    uint32_t *totals = (uint32_t *)s.work(Sim::WORK_TOTALS, 256);
+    uint32_t *totals = (uint32_t *)s.results(deaths.size() * 4);
     for (size_t k = 0; k < may_die_types.size(); k++) {
       AgentStore &a = s.agents[may_die_types[k] - 1];
       // (no more numbers than agents are ever on the stack)
@@ -828,7 +829,7 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
       scan_map<8, uint32_t>(s, a.n, NewDeaths{a.died_wr.as<uint8_t>(), a.died_rd.as<uint8_t>()},
                          PushReuse{a.reuse.as<uint64_t>() + a.nreuse}, totals + k);
     }
-    s.fetch(deaths.data(), totals, deaths.size() * 4);
+    s.read_results(deaths.data(), totals, deaths.size() * 4);
   }
   if (!s.async) check_device_status(s, tname);
 

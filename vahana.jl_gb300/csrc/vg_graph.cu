@@ -1670,7 +1670,7 @@ void remove_died_edges(Sim &s, const std::vector<int> &died_types) {
   uint64_t rows = 0;
   for (auto &x : list) rows += s.edges[x.e].csr[x.T].nrows + 1;
   uint32_t *counts = (uint32_t *)s.work(Sim::WORK_ROWS, rows * 4);
-  uint32_t *totals = (uint32_t *)s.work(Sim::WORK_TOTALS, list.size() * 4);
+  uint32_t *totals = (uint32_t *)s.results(list.size() * 4);
   uint64_t at = 0;
   for (size_t k = 0; k < list.size(); k++) {
     CSR &c = s.edges[list[k].e].csr[list[k].T];
@@ -1682,7 +1682,7 @@ void remove_died_edges(Sim &s, const std::vector<int> &died_types) {
     at += c.nrows + 1;
   }
   std::vector<uint32_t> kept(list.size());
-  s.fetch(kept.data(), totals, kept.size() * 4);
+  s.read_results(kept.data(), totals, kept.size() * 4);
   at = 0;
   for (size_t k = 0; k < list.size(); k++) {
     CSR &c = s.edges[list[k].e].csr[list[k].T];

@@ -336,11 +336,16 @@ struct Sim {
   std::map<std::string, std::vector<double>> global_series;
   // scratch
   DevBuf d_status;  // StatusWord: the kernels' first error
-  // a line of mapped pinned host memory (null: none was free): the status
-  // word's host copy, then PIN_BYTES - 64 bytes that fetch() reads through
-  char *pin = nullptr;
+  // a line of mapped pinned host memory (null: none was free) and its device
+  // address: the status word's host copy, PIN_FETCH bytes that fetch() reads
+  // through, PIN_RESULTS bytes that kernels store small results in
+  char *pin = nullptr, *pin_dev = nullptr;
   // a few bytes of device memory, after all work queued so far
   void fetch(void *dst, const void *src, size_t bytes);
+  // where kernels store up to a few words for the host: mapped memory if there
+  // is some (read_results then takes a wait and no copy); until the next call
+  void *results(size_t bytes);
+  void read_results(void *dst, const void *res, size_t bytes);
   DevBuf d_scratch;
   size_t scratch_bytes = 0;
   void *scratch(size_t bytes);
@@ -408,7 +413,7 @@ struct StatusWord {
   int code, pad;
   int *host;  // may be null
 };
-constexpr size_t PIN_BYTES = 256;
+constexpr size_t PIN_FETCH = 192, PIN_RESULTS = 256, PIN_BYTES = 64 + PIN_FETCH + PIN_RESULTS;
 #ifdef __CUDACC__
 // programmatic dependent launches: the next kernel of the stream may start
 // once every block has called let_next_start; the last block of a kernel that

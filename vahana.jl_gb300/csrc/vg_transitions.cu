@@ -1623,10 +1623,10 @@ void tr_spawn(ApplyCtx &c) {
   const uint64_t n = w.a.n;
   if (n == 0) return;
   uint32_t *rank = (uint32_t *)s.work(Sim::WORK_PLACES, n * 4);
-  uint32_t *callers = (uint32_t *)s.work(Sim::WORK_TOTALS, 256);
+  uint32_t *callers = (uint32_t *)s.results(4);
   scan_map<4, uint32_t>(s, n, SpawnCallers{w}, SpawnRanks{rank}, callers);
   uint32_t m = 0;
-  s.fetch(&m, callers, 4);
+  s.read_results(&m, callers, 4);
   AgentStore &a = s.agents[T - 1];
   const uint64_t total = (uint64_t)m * k;
   g.nreuse = ad.immortal() ? 0 : a.nreuse;
