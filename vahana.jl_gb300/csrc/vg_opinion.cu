@@ -951,6 +951,9 @@ void tr_bounded_confidence(ApplyCtx &c) {
     if (p.grid) k_opinion_long<true, false><<<nl, LONG_TPB, 0, s.stream>>>(p, Notify{});
     else k_opinion_long<false, false><<<nl, LONG_TPB, 0, s.stream>>>(p, Notify{});
     VG_CUDA(cudaGetLastError());
+  }
+  // (no other blocks when every row is long: a complete graph of 3073 agents)
+  if (grid > nbig && nl) {
     launch_dependent(p.grid ? k_opinion<true, true> : k_opinion<false, true>, grid - nbig, TPB,
                      0, s.stream, p);
   } else if (grid > nbig) {
@@ -1200,7 +1203,7 @@ OpinionTables pack_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_
     for (unsigned k = 0; k < p.long_hubs + p.nlong; k++) longs.push_back({(uint32_t)j, k});
   }
   OpinionTables t{0, 0, (unsigned)tiles.size(), (unsigned)longs.size()};
-  if (tiles.empty()) return t;
+  if (tiles.empty() && longs.empty()) return t;
   // (the long slices' tiles behind the others)
   tiles.insert(tiles.end(), longs.begin(), longs.end());
   t.args_at = append_table(bytes, args);
@@ -1209,16 +1212,15 @@ OpinionTables pack_opinion_jobs(const std::vector<OpinionJob> &jobs, cudaStream_
 }
 
 bool launch_opinion_jobs(const OpinionTables &t, const uint8_t *dev, cudaStream_t st) {
-  if (!t.ntiles) return false;
+  if (!t.ntiles && !t.nlong) return false;
   const OpinionArgs *da = (const OpinionArgs *)(dev + t.args_at);
   const JobTile *dt = (const JobTile *)(dev + t.tiles_at);
   if (t.nlong) {
     k_opinion_jobs_long<<<t.nlong, LONG_TPB, 0, st>>>(da, dt + t.ntiles);
     VG_CUDA(cudaGetLastError());
-    launch_dependent(k_opinion_jobs, t.ntiles, TPB, 0, st, da, dt);
-  } else {
-    k_opinion_jobs<<<t.ntiles, TPB, 0, st>>>(da, dt);
   }
+  if (t.ntiles && t.nlong) launch_dependent(k_opinion_jobs, t.ntiles, TPB, 0, st, da, dt);
+  else if (t.ntiles) k_opinion_jobs<<<t.ntiles, TPB, 0, st>>>(da, dt);
   VG_CUDA(cudaGetLastError());
   return true;
 }
