@@ -829,20 +829,28 @@ __global__ void k_sir(const uint32_t *__restrict__ rp, const uint32_t *__restric
 // ------------------------------------------------ Life B3/S23 (cfg 2)
 // Cells of a 2-D raster, implicit Moore stencil (chebyshev, distance 1).
 // The count of alive neighbours does not depend on edge order.
-// Four cells are the bytes of a 32-bit word (byte i = cell x + i, 0 or 1): the
+// Four cells are the bytes of a 32-bit word (byte i = cell x + i): the
 // sum of a row's three horizontally adjacent cells for all four bytes at
-// once, three rows added and the centre subtracted; no byte exceeds 8, so
-// none carries into the next.  A warp holds 32 consecutive words of a row;
+// once, three rows added and the centre subtracted; with cells of 0 and 1 no
+// byte exceeds 8, so none carries into the next.  A warp holds 32 consecutive words of a row;
 // the neighbouring words come from the adjacent lanes, and only the warp's
 // edge lanes load them.
 __device__ __forceinline__ uint32_t life_hsum(uint32_t c, uint32_t lw, uint32_t rw) {
   return __funnelshift_l(lw, c, 8) + c + __funnelshift_r(c, rw, 8);
 }
-// alive next: three neighbours, or two around a living cell -- exactly when
-// count | cell is 3; bytes below 16 are zero when adding 15 leaves bit 4 clear
+// alive next: a count of three, or of two around a living cell.  For cells of
+// 0 and 1 (UNIT) exactly when count | cell is 3: bytes below 16 are zero when
+// adding 15 leaves bit 4 clear.  UInt8 cells may hold more, and three byte-wise
+// comparisons stay: a cell of 2 beside one neighbour of 1 is not born.
+template <bool UNIT>
 __device__ __forceinline__ uint32_t life_rule(uint32_t cnt, uint32_t self) {
-  const uint32_t t = (cnt | self) ^ 0x03030303u;
-  return ~((t + 0x0f0f0f0fu) >> 4) & 0x01010101u;
+  if (UNIT) {
+    const uint32_t t = (cnt | self) ^ 0x03030303u;
+    return ~((t + 0x0f0f0f0fu) >> 4) & 0x01010101u;
+  }
+  const uint32_t born = __vcmpeq4(cnt, 0x03030303u);
+  const uint32_t stay = __vcmpeq4(cnt, 0x02020202u) & __vcmpne4(self, 0u);
+  return (born | stay) & 0x01010101u;
 }
 
 // blocks of 32 x 8 threads; each thread LIFE_ROWS consecutive rows of one
@@ -855,6 +863,7 @@ __device__ __forceinline__ uint32_t life_rule(uint32_t cnt, uint32_t self) {
 // instructions).
 constexpr int LIFE_ROWS = 8;
 
+template <bool UNIT>
 __global__ void __launch_bounds__(256) k_life2d_x4(const uint32_t *a, uint32_t *o, int Wq,
                                                    int64_t H, int periodic) {
   let_next_start();
@@ -906,12 +915,12 @@ __global__ void __launch_bounds__(256) k_life2d_x4(const uint32_t *a, uint32_t *
   if (y0 + LIFE_ROWS <= H) {
 #pragma unroll
     for (int j = 0; j < LIFE_ROWS; j++)
-      out[(int64_t)j * Wq] = life_rule(e[j] + e[j + 1] + e[j + 2] - c[j + 1], c[j + 1]);
+      out[(int64_t)j * Wq] = life_rule<UNIT>(e[j] + e[j + 1] + e[j + 2] - c[j + 1], c[j + 1]);
   } else {
 #pragma unroll
     for (int j = 0; j < LIFE_ROWS; j++)
       if (y0 + j < H)
-        out[(int64_t)j * Wq] = life_rule(e[j] + e[j + 1] + e[j + 2] - c[j + 1], c[j + 1]);
+        out[(int64_t)j * Wq] = life_rule<UNIT>(e[j] + e[j + 1] + e[j + 2] - c[j + 1], c[j + 1]);
   }
 }
 
@@ -1855,8 +1864,9 @@ void tr_life(ApplyCtx &c) {
     dim3 blk(32, 8);
     dim3 grd((unsigned)((Wq + 31) / 32),
              (unsigned)((st.dims[1] + 8 * LIFE_ROWS - 1) / (8 * LIFE_ROWS)));
-    launch_dependent(k_life2d_x4, grd, blk, 0, s.stream, (const uint32_t *)in, (uint32_t *)out,
-                     (int)Wq, st.dims[1], st.periodic);
+    launch_dependent(ad.fields[0].dtype == VG_BOOL ? k_life2d_x4<true> : k_life2d_x4<false>, grd,
+                     blk, 0, s.stream, (const uint32_t *)in, (uint32_t *)out, (int)Wq, st.dims[1],
+                     st.periodic);
   } else if (ad.fields[0].dtype == VG_BOOL && rows_pay(st, R.ncells, moore2d) &&
              row_stencil(st, birth, survive, rs, reach)) {
     const uint64_t blocks = (uint64_t)rs.tx * rs.ty * rs.dims[2] * rs.dims[3];
