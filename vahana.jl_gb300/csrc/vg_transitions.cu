@@ -1092,6 +1092,9 @@ __global__ void __launch_bounds__(256, 4) k_life_rows(const uint8_t *a, uint8_t 
 #pragma unroll
   for (int j = 0; j < ROW_RY; j++) acc[j] = self[j] = 0;
   const int nplanes = CODE >= 0 ? 1 : s.nplanes;
+  // a raster of one dimension has one row, which a position D rows away does
+  // not reach by wrapping once (and no row of its stencil lies there)
+  const bool wrap_y = s.periodic && H > D;
   for (int p = 0; p < nplanes; p++) {
     int pz = z + (CODE >= 0 ? 0 : s.plane[p].z), pv = v + (CODE >= 0 ? 0 : s.plane[p].v);
     if (pz < 0 || pz >= Z || pv < 0 || pv >= V) {
@@ -1112,7 +1115,7 @@ __global__ void __launch_bounds__(256, 4) k_life_rows(const uint8_t *a, uint8_t 
     for (int u = 0; u < LOADS; u++) {
       const int r = u * 8 + (int)threadIdx.y;  // warp-uniform
       int y = y0 - D + r;
-      const bool use = r < ROWS && ((y >= 0 && y < H) || (s.periodic && y < H + D));
+      const bool use = r < ROWS && ((y >= 0 && y < H) || (wrap_y && y < H + D));
       y += y < 0 ? H : y >= H ? -H : 0;
       const uint8_t *row = base + (uint64_t)(use ? y : 0) * W;
       sh[u] = 8 * ((uint32_t)(uint64_t)(row + x0) & 3u);
@@ -1142,7 +1145,7 @@ __global__ void __launch_bounds__(256, 4) k_life_rows(const uint8_t *a, uint8_t 
         const int r = i / 8, k = i % 8, j = k < 2 ? k : jr + k - 4;
         const int x = x0 - 8 + 4 * j;
         int y = y0 - D + r;
-        if (j >= ROW_WORDS || (k >= 2 && j < 2) || !((y >= 0 && y < H) || (s.periodic && y < H + D)))
+        if (j >= ROW_WORDS || (k >= 2 && j < 2) || !((y >= 0 && y < H) || (wrap_y && y < H + D)))
           continue;
         y += y < 0 ? H : y >= H ? -H : 0;
         const uint8_t *row = base + (uint64_t)y * W;
