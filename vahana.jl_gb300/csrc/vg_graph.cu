@@ -963,8 +963,9 @@ __global__ void __launch_bounds__(TPB) k_rp_fill(const uint32_t *keys, uint64_t 
   __syncthreads();
   // (eight records in flight per thread: a crowded span is one block's work,
   // and one at a time took 300 ns each round; keys from nrows on are slots
-  // without a record)
+  // without a record, and no key of another span is stored whatever the order)
   constexpr int U = 8;
+  const uint32_t rows = (uint32_t)(min((unsigned long long)R1, (unsigned long long)nrows) - R0);
   for (uint32_t kk = k0 + tid; kk < k1; kk += U * TPB) {
     uint32_t key[U], next[U];
 #pragma unroll
@@ -976,8 +977,8 @@ __global__ void __launch_bounds__(TPB) k_rp_fill(const uint32_t *keys, uint64_t 
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint32_t k = kk + u * TPB;
-      if (k < k1 && next[u] != key[u] && key[u] < nrows)
-        E[rp_slot(key[u] - (uint32_t)R0)] = k + 1 - k0;
+      const uint32_t row = key[u] - (uint32_t)R0;
+      if (k < k1 && next[u] != key[u] && row < rows) E[rp_slot(row)] = k + 1 - k0;
     }
   }
   __syncthreads();

@@ -1503,6 +1503,12 @@ void tr_keep(ApplyCtx &c) {
   VG_CUDA(cudaGetLastError());
 }
 
+// Whether a caller's slots may stay empty: agents that died and agents without
+// a with_edge edge are not swept, and their rows may hold edges all the same (a
+// dead agent loses its edges when it dies, but walkers move onto dead cells and
+// add_edges! takes any target).
+bool slots_may_be_empty(const Sweep &w) { return w.mortal || w.with_rp; }
+
 // T, S: target and source type of every record, when the call's records have
 // known slots (0 .. cap - 1 in call order; holes: some may stay empty)
 Append make_append(ApplyCtx &c, int e, uint64_t cap, int T = 0, int S = 0, bool holes = false) {
@@ -1537,7 +1543,7 @@ void tr_self_edge(ApplyCtx &c) {
   const EdgeTypeDesc &ed = s.model->et(e);
   Sweep w = make_sweep(c);
   if (w.a.n == 0) return;
-  Append ap = make_append(c, e, w.a.n, c.call_type, c.call_type, w.mortal || w.with_rp);
+  Append ap = make_append(c, e, w.a.n, c.call_type, c.call_type, slots_may_be_empty(w));
   // constant payload from params[1..]: one value per field
   std::vector<uint8_t> pl;
   if (ed.stores_payload())
@@ -1568,9 +1574,9 @@ void tr_readd_edges(ApplyCtx &c) {
   Sweep w = make_sweep(c);
   DevCSRView v = csr_view(s, e, c.call_type);
   if (w.a.n == 0) return;
-  // (a died agent has no in-edges: only with_edge leaves rows out)
   Append ap = v.nedges && v.nrows <= w.a.n
-                  ? make_append(c, e, v.nedges, c.call_type, v.src_type_const, w.with_rp != nullptr)
+                  ? make_append(c, e, v.nedges, c.call_type, v.src_type_const,
+                                slots_may_be_empty(w))
                   : make_append(c, e, std::max<uint64_t>(v.nedges, 1));
   if (ap.rows) k_readd_slots<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap);
   else k_readd_edges<<<nblk(w.a.n), TPB, 0, s.stream>>>(w, v, ap, c.call_pos);
@@ -1675,7 +1681,7 @@ void tr_link_neighbors(ApplyCtx &c) {
   // (with neighbours of the called type every record links it with itself)
   Append ap = v.nedges && v.nrows <= w.a.n && v.src && v.src_type_const == c.call_type
                   ? make_append(c, F, 2 * v.nedges, c.call_type, c.call_type,
-                                has_die || w.with_rp != nullptr)
+                                has_die || slots_may_be_empty(w))
                   : make_append(c, F, std::max<uint64_t>(2 * v.nedges, 1));
   const int pl_dt = fd.stores_payload() ? fd.fields[0].dtype : -1;
   if (ap.rows)
@@ -2000,10 +2006,11 @@ void tr_move_to(ApplyCtx &c) {
   m.has_from = ef >= 0;
   m.has_to = et >= 0;
   m.same = m.has_from && m.has_to && ef == et;
-  // (agents that died and positions beyond a bounded raster leave their slots
-  // empty; a position outside a periodic one is an error, status 204)
+  // (positions beyond a bounded raster leave their slots empty; one outside a
+  // periodic raster is an error, status 204, which is read before the rebuild
+  // unless transitions are queued)
   const bool typed = per > 0 && !m.same;
-  const bool holes = w.mortal || w.with_rp || !m.periodic || mode == 1;
+  const bool holes = slots_may_be_empty(w) || !m.periodic || mode == 1 || s.async;
   const int T = typed ? c.call_type : 0, R_T = typed ? R.type_nr : 0;
   if (m.has_from)
     m.from = make_append(c, ef, std::max<uint64_t>(1, w.a.n * per * (m.same ? 2 : 1)), T, R_T, holes);
