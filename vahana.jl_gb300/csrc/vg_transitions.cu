@@ -612,7 +612,12 @@ __global__ void k_link_slots(Sweep s, DevCSRView c, Append ap, int pl_dt, int ha
     const long long oi = __shfl_sync(FULL_WARP, vi, owner);
     if (!has) return;
     const bool swept = alive >> owner & 1u;
-    const uint32_t id = r0 + owner, nid = c.src[e];
+    const uint32_t id = r0 + owner;
+    uint32_t nid = c.src[e];
+    if (swept && nid >= s.a.n) {  // an edge from an agent that does not exist
+      set_status(s.status, 501);
+      nid = id;
+    }
     ((uint2 *)ap.rows)[e] = swept ? make_uint2(id, nid) : make_uint2(BK_HOLE, BK_HOLE);
     if (!swept) return;
     ((uint2 *)ap.srcs)[e] = make_uint2(nid, id);
@@ -1509,6 +1514,13 @@ void tr_keep(ApplyCtx &c) {
 // add_edges! takes any target).
 bool slots_may_be_empty(const Sweep &w) { return w.mortal || w.with_rp; }
 
+// Whether every cell of a raster is an agent: cells of a mortal type are gone
+// after a transition that writes their type anew (no add_existing).  Records onto
+// such cells take the general build, which refuses them.
+bool cells_exist(const Sim &s, const Raster &R) {
+  return R.first_nr - 1 + R.ncells <= s.agents[R.type_nr - 1].n;
+}
+
 // T, S: target and source type of every record, when the call's records have
 // known slots (0 .. cap - 1 in call order; holes: some may stay empty)
 Append make_append(ApplyCtx &c, int e, uint64_t cap, int T = 0, int S = 0, bool holes = false) {
@@ -1925,8 +1937,8 @@ void tr_random_walk(ApplyCtx &c) {
   require_agent_read(c, c.call_type);
   DevAgentView a = agent_view(s, c.call_type);
   if (a.n == 0) return;
-  if (c.typed_ok(e, R.type_nr, c.call_type, a.n) && !s.edges[e].add_existing &&
-      R.dims[0] < (1ll << 31) && R.dims[1] < (1ll << 31)) {
+  if (cells_exist(s, R) && c.typed_ok(e, R.type_nr, c.call_type, a.n) &&
+      !s.edges[e].add_existing && R.dims[0] < (1ll << 31) && R.dims[1] < (1ll << 31)) {
     const BucketPlan plan = plan_buckets(s, e, R.type_nr, a.n, false);
     EdgeAppend *ap = c.append_typed(e, R.type_nr, c.call_type, a.n, false, !plan.sorted);
     ap->plan = plan;
@@ -2009,7 +2021,7 @@ void tr_move_to(ApplyCtx &c) {
   // (positions beyond a bounded raster leave their slots empty; one outside a
   // periodic raster is an error, status 204, which is read before the rebuild
   // unless transitions are queued)
-  const bool typed = per > 0 && !m.same;
+  const bool typed = per > 0 && !m.same && cells_exist(s, R);
   const bool holes = slots_may_be_empty(w) || !m.periodic || mode == 1 || s.async;
   const int T = typed ? c.call_type : 0, R_T = typed ? R.type_nr : 0;
   if (m.has_from)
