@@ -13,6 +13,7 @@
 #include <cstring>
 #include <limits>
 #include <type_traits>
+#include <utility>
 
 #include "vg_internal.h"
 #include "vg_scan.cuh"
@@ -844,7 +845,8 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
     std::swap(a.died_rd, a.died_wr);
     const auto it = std::find(may_die_types.begin(), may_die_types.end(), T);
     if (it == may_die_types.end()) continue;  // no agent can have died
-    const uint32_t k = deaths[it - may_die_types.begin()];
+    // (counted once, also for a type that `call` names twice)
+    const uint32_t k = std::exchange(deaths[it - may_die_types.begin()], 0u);
     if (!k) continue;
     // readreuseable = [readreuseable; writereuseable]
     a.nreuse += k;
