@@ -284,17 +284,7 @@ using namespace vg;
     return VG_ERR_ARG;                    \
   }
 
-static Sim &S(vg_sim *s) {
-  if (!s || !s->s) fail(VG_ERR_ARG, "null simulation handle");
-  s->s->calls++;
-  return *s->s;
-}
-// for entries that leave every agent as it is
-static Sim &peek(vg_sim *s) {
-  Sim &r = S(s);
-  r.calls--;
-  return r;
-}
+static Sim &S(vg_sim *h) { return enter(h); }
 
 static Model &MD(const vg_model *m) {
   if (!m || !m->m) fail(VG_ERR_ARG, "null model handle");

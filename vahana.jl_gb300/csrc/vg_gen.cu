@@ -158,11 +158,7 @@ void set_last_error(const std::string &m);
     return VG_ERR_ARG;              \
   }
 
-static Sim &S(vg_sim *s) {
-  if (!s || !s->s) fail(VG_ERR_ARG, "null simulation handle");
-  s->s->calls++;
-  return *s->s;
-}
+static Sim &S(vg_sim *h) { return enter(h); }
 
 extern "C" {
 

@@ -319,7 +319,9 @@ struct Sim {
   uint64_t csr_epoch = 1, sir_epoch = 0;
   // entries into the library with this simulation that may change agents
   uint64_t calls = 0;
-  bool columns_shared = false;  // a column's device pointer was handed out
+  // the columns may change without a call: a device pointer was handed out, or a
+  // call was recorded into a CUDA graph
+  bool columns_shared = false;
   // one bit per agent of `type`, set where its state is 1, written by the SIR
   // step beside the states; it holds for the step that is the very next call
   struct InfectedMask {
@@ -657,3 +659,24 @@ struct vg_model {
 struct vg_sim {
   std::unique_ptr<vg::Sim> s;
 };
+
+namespace vg {
+// the simulation behind a handle, for entry points that leave every agent as it is
+inline Sim &peek(vg_sim *h) {
+  if (!h || !h->s) fail(VG_ERR_ARG, "null simulation handle");
+  return *h->s;
+}
+// and for all others.  What a step left for the very next one (Sim::infected)
+// holds only while no call came between; a call that is being recorded into a
+// CUDA graph may run again, unseen, at any time after.
+inline Sim &enter(vg_sim *h) {
+  Sim &s = peek(h);
+  s.calls++;
+  if (s.device_ready && !s.columns_shared) {
+    cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s.stream, &recording) != cudaSuccess) cudaGetLastError();
+    else s.columns_shared = recording != cudaStreamCaptureStatusNone;
+  }
+  return s;
+}
+}  // namespace vg

@@ -26,11 +26,7 @@ namespace {
 
 constexpr char MAGIC[8] = {'V', 'G', 'S', 'N', 'A', 'P', '0', '1'};
 
-Sim &S(vg_sim *h) {
-  if (!h || !h->s) fail(VG_ERR_ARG, "null simulation");
-  h->s->calls++;
-  return *h->s;
-}
+Sim &S(vg_sim *h) { return enter(h); }
 
 struct File {
   FILE *f = nullptr;

@@ -1746,11 +1746,9 @@ void tr_sir(ApplyCtx &c) {
   cfg.numAttrs = s.sir_epoch == s.csr_epoch ? 1 : 0;
   Sim::InfectedMask &inf = s.infected;
   const size_t words = (a.n + 31) / 32 * 4;
-  // (a recorded step may be replayed after anything: it reads the states, and
-  // what follows the recording does not take its mask for done)
-  cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
-  VG_CUDA(cudaStreamIsCapturing(s.stream, &recording));
-  const bool direct = recording == cudaStreamCaptureStatusNone && !s.columns_shared;
+  // (columns that may change without a call: the step reads the states, and
+  // leaves no mask for the next)
+  const bool direct = !s.columns_shared;
   const bool mask = direct && inf.call + 1 == s.calls && inf.type == c.call_type &&
                     inf.m[inf.cur].bytes >= words;
   const bool early = v.nedges < SIR_EARLY_EDGES;
