@@ -25,3 +25,21 @@ def test_type_called_twice(vh, n, share):
     np.testing.assert_array_equal(np.sort(cols["die"][:n] >= 100)[::-1],
                                   np.arange(n) < reused)
     sim.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 5000, 70_000])
+def test_more_numbers_than_agents(vh, n):
+    """Agents whose numbers are on the stack already die again and again: the
+    stack grows with them."""
+    m = (vh.ModelTypes().register_agenttype("P", [("die", "i64")]).create_model("Again"))
+    sim = vh.create_simulation(m)
+    vh.add_agents(sim, "P", n, die=1)
+    vh.finish_init(sim)
+    for _ in range(3):
+        vh.apply_(sim, "die_if", ["P", "P"], ["P"], ["P"], params=[1, 0, 1.0])
+        assert not vh.read_agents(sim, "P")[1].any()
+    # 3 n numbers are on the stack: n callers with 4 newcomers each take them all
+    vh.apply_(sim, "spawn", ["P"], ["P"], ["P"], params=[4, 1, 1, 1, 1])
+    cols, died = vh.read_agents(sim, "P")
+    assert cols["die"].size == 2 * n and not died.any()
+    sim.close()

@@ -149,8 +149,9 @@ struct NewDeaths {
 };
 struct PushReuse {
   uint64_t *top;
+  uint64_t room;
   __device__ __forceinline__ void operator()(uint64_t i, uint32_t rank, uint32_t died) const {
-    if (died) top[rank] = i + 1;
+    if (died && rank < room) top[rank] = i + 1;
   }
 };
 
@@ -811,22 +812,34 @@ int vg_apply(vg_sim *h, const char *tname, const int *call, int ncall, const int
   if (!may_die_types.empty()) {
     deaths.resize(may_die_types.size());
     uint32_t *totals = (uint32_t *)s.results(deaths.size() * 4);
-    for (size_t k = 0; k < may_die_types.size(); k++) {
+    auto collect = [&](size_t k, uint64_t room) {
       AgentStore &a = s.agents[may_die_types[k] - 1];
-      // (no more numbers than agents are ever on the stack)
-      if (a.reuse_cap < a.n) {
+      if (a.reuse_cap < a.nreuse + room) {
         DevBuf nb;
-        nb.alloc(a.cap * 8, &s.footprint);
+        const uint64_t cap = std::max(a.cap, a.nreuse + room);
+        nb.alloc(cap * 8, &s.footprint);
         if (a.nreuse)
           VG_CUDA(cudaMemcpyAsync(nb.p, a.reuse.p, a.nreuse * 8, cudaMemcpyDeviceToDevice, s.stream));
         VG_CUDA(cudaStreamSynchronize(s.stream));  // (the old stack is read until here)
         a.reuse = std::move(nb);
-        a.reuse_cap = a.cap;
+        a.reuse_cap = cap;
       }
       scan_map<8, uint32_t>(s, a.n, NewDeaths{a.died_wr.as<uint8_t>(), a.died_rd.as<uint8_t>()},
-                         PushReuse{a.reuse.as<uint64_t>() + a.nreuse}, totals + k);
+                            PushReuse{a.reuse.as<uint64_t>() + a.nreuse, a.reuse_cap - a.nreuse},
+                            totals + k);
+    };
+    // room for the agents that are not on the stack yet: those that can die,
+    // unless numbers of living agents are on it (a type that `call` names twice
+    // has its deaths collected and its state swapped back)
+    for (size_t k = 0; k < may_die_types.size(); k++) {
+      const AgentStore &a = s.agents[may_die_types[k] - 1];
+      collect(k, a.n > a.nreuse ? a.n - a.nreuse : 0);
     }
     s.read_results(deaths.data(), totals, deaths.size() * 4);
+    for (size_t k = 0; k < may_die_types.size(); k++) {
+      const AgentStore &a = s.agents[may_die_types[k] - 1];
+      if (deaths[k] > a.reuse_cap - a.nreuse) collect(k, deaths[k]);
+    }
   }
   if (!s.async) check_device_status(s, tname);
 
