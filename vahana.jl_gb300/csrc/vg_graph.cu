@@ -1920,10 +1920,15 @@ __global__ void k_slice_deg(const uint32_t *rp, uint64_t nrows, const uint32_t *
   slots[sl] = 32ull * dm;
 }
 
-// flag the slices of at least thr slots
-__global__ void k_flag_long(const uint32_t *sdeg, uint64_t nslices, uint32_t thr, uint32_t *flag) {
+// flag the slices of at least thr slots; *tail: the longest of the others from
+// slice `from` on
+__global__ void k_flag_long(const uint32_t *sdeg, uint64_t nslices, uint32_t thr, uint64_t from,
+                            uint32_t *flag, uint32_t *tail) {
   uint64_t sl = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (sl < nslices) flag[sl] = sdeg[sl] >= thr ? 1u : 0u;
+  const uint32_t d = sl < nslices ? sdeg[sl] : 0u;
+  if (sl < nslices) flag[sl] = d >= thr ? 1u : 0u;
+  const uint32_t m = __reduce_max_sync(0xffffffffu, sl >= from && d < thr ? d : 0u);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(tail, m);
 }
 
 // sort key of a listed slice: descending length
@@ -2004,6 +2009,7 @@ void ensure_schedule(Sim &s, CSR &c, uint32_t thr, uint32_t big_thr, uint64_t n)
   c.long_slices.release();
   c.long_slots.clear();
   c.long_hubs.clear();
+  c.tail_slots = 0;
   c.nhub = c.norder = c.nslices = c.nbig = 0;
   c.range_block.clear();
   c.range_rows.clear();
@@ -2066,13 +2072,19 @@ void ensure_schedule(Sim &s, CSR &c, uint32_t thr, uint32_t big_thr, uint64_t n)
                               st));
       // the long slices, listed longest first (no slice has more than thr slots)
       if (thr >= long_min) {
-        Tmp<uint32_t> flag(ns + 1, st), pos(ns + 1, st);
+        Tmp<uint32_t> flag(ns + 1, st), pos(ns + 2, st);
         VG_CUDA(cudaMemsetAsync(flag.p + ns, 0, 4, st));
-        k_flag_long<<<nblk(ns), TPB, 0, st>>>(c.slice_deg.as<uint32_t>(), ns, long_min, flag.p);
+        VG_CUDA(cudaMemsetAsync(pos.p + ns + 1, 0, 4, st));
+        // (two windows at least: the last full one's first slices among them)
+        const uint64_t last = std::min(ns, std::max<uint64_t>(ns / 8, 2ull << (wshift - 5)));
+        k_flag_long<<<nblk(ns), TPB, 0, st>>>(c.slice_deg.as<uint32_t>(), ns, long_min,
+                                              ns - last, flag.p, pos.p + ns + 1);
         exclusive_scan_u32(flag.p, pos.p, ns + 1, st, s);
-        uint32_t nlong = 0;
-        VG_CUDA(cudaMemcpyAsync(&nlong, pos.p + ns, 4, cudaMemcpyDeviceToHost, st));
+        uint32_t found[2] = {0, 0};
+        VG_CUDA(cudaMemcpyAsync(found, pos.p + ns, 8, cudaMemcpyDeviceToHost, st));
         VG_CUDA(cudaStreamSynchronize(st));
+        const uint32_t nlong = found[0];
+        c.tail_slots = found[1];
         if (nlong) {
           Tmp<uint32_t> lkeys(nlong, st);
           c.long_slices.alloc((uint64_t)nlong * 4, &s.footprint);

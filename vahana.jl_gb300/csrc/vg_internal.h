@@ -233,6 +233,7 @@ struct CSR {
   // their slots
   DevBuf long_slices;  // u32
   std::vector<uint32_t> long_slots;
+  uint32_t tail_slots = 0;  // the longest other slice of the last windows (an eighth, two at least)
   // in-degrees of the leading hub rows with 32 times as many edges or more
   std::vector<uint32_t> long_hubs;
   DevBuf sell_src;  // u32 [slots]

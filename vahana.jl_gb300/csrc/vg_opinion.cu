@@ -867,16 +867,23 @@ static unsigned opinion_args(Sim &s, int e, int T, double eps, double a, double 
                              uint32_t thr, uint32_t big_thr, OpinionArgs &p,
                              cudaStream_t launch_stream);
 
-// Where the first blocks of the windows run ahead: launches whose last slices
-// are a good part of them and whose opinions stay in L2 in any order.  Measured,
-// us per step in the windows' order and so: host-made graphs (degrees of a
-// narrow distribution with a heavy end) 10^6 agents with 2*10^7 edges 167 and
-// 133, with 8*10^6 84 and 66, 3*10^5 with 6*10^6 75 and 76; power-law graphs
-// 10^6 with 2*10^7 118 and 119, 1.5*10^6 with 3*10^7 159 and 165, 3*10^6 with
-// 6*10^7 298 and 302.  3 or 12 blocks: 139 and 129 for the first, 160 and 176 for
-// the last but one.
+// Where the first blocks of the windows run ahead: in the windows' order the
+// last windows' longest slices start when the launch is nearly done, 340 ns per
+// slot.  They do where the last windows hold a slice of a third of the long
+// slices' length, a fifth of the launch (tail_slots): graphs whose heavy rows are
+// spread over the agents.  Generated power-law graphs have theirs in the first
+// windows; there the windows' order keeps the gathers local and is the better one.
+// Measured, us per step in the windows' order and with the first blocks ahead.
+// Heavy rows spread: 10^6 agents with 8*10^6 edges 84 and 66, with 2*10^7 167 and
+// 132; 1.5*10^6 with 3*10^7 250 and 185; 3*10^6 with 6*10^7 445 and 346; 5*10^6
+// with 10^8 673 and 577; 7*10^6 with 1.4*10^8 1196 and 817; 3*10^5 with 6*10^6 75
+// and 76; with hub rows, whose place in the order is missing so that the windows
+// begin a few blocks early, 10^6 with 3*10^7 242 and 243, 5*10^5 with 3*10^7 232
+// and 236.  Heavy rows first: 10^6 with 2*10^7 118 and 118, 1.5*10^6 with 3*10^7
+// 158 and 164, 3*10^6 with 6*10^7 298 and 315, 5*10^6 with 10^8 477 and 501.
+// 3 or 12 blocks ahead: 139 and 129 for 10^6 agents with 2*10^7 edges, 160 and 176
+// for the power-law graph of 3*10^7.
 constexpr unsigned AHEAD_BLOCKS = 6;
-constexpr uint64_t AHEAD_EDGES = 24000000;
 // which slices and hub rows take a block each, in a launch over `edges`
 // edges; returns the grid of the other blocks
 static unsigned split_long(OpinionArgs &p, uint64_t edges) {
@@ -893,7 +900,8 @@ static unsigned split_long(OpinionArgs &p, uint64_t edges) {
   p.slice_blocks = (unsigned)((p.nslices + (TPB / 32) - 1) / (TPB / 32));
   p.wblocks = (1u << p.csr->wshift) / TPB;
   p.nwindows = p.wblocks ? p.slice_blocks / p.wblocks : 0;
-  p.ahead = edges < AHEAD_EDGES && p.wblocks > AHEAD_BLOCKS && p.nwindows ? AHEAD_BLOCKS : 0;
+  p.ahead = p.csr->tail_slots >= p.long_slots / 3 && p.wblocks > AHEAD_BLOCKS && p.nwindows
+                ? AHEAD_BLOCKS : 0;
   return (unsigned)p.nbig + p.hub_blocks + (unsigned)((p.nslices + (TPB / 32) - 1) / (TPB / 32));
 }
 
