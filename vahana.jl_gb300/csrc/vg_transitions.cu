@@ -754,7 +754,7 @@ __global__ void k_move_to(Sweep s, MoveArgs m, int call_pos) {
 // (p_k from the host table, built by the same repeated multiplication);
 // an infected agent recovers when days reaches `recovery`.
 constexpr int SIR_U = 16;
-constexpr uint64_t SIR_EARLY_EDGES = 1000000;
+constexpr uint64_t SIR_EARLY_EDGES = 400000;
 
 // One SIR step.  Launched with programmatic dependent launch when the
 // contact rows cannot be written by the preceding kernel (Sim::csr_epoch):
@@ -763,17 +763,23 @@ constexpr uint64_t SIR_EARLY_EDGES = 1000000;
 // sources, before griddepcontrol.wait; the states (written by the previous
 // step) and every output are touched only after it.  Without the launch
 // attribute the wait returns at once.  SIR_U sources are requested together,
-// then their states: two memory round trips for a row of up to SIR_U in-edges.
+// then what they name: for a row of up to SIR_U in-edges two memory round trips
+// with EARLY (beside the agent's own state, and the neighbours), else three.
 //
 // A step that follows a step reads its neighbours from the mask that one left
 // (MASK), an eighth of the state bytes: every SM fetches what its rows name once
 // per step.  EARLY hides a round trip, but reads the rows of agents that turn
 // out not to be susceptible: below SIR_EARLY_EDGES edges the round trip is the
 // larger part.  Bound: latency there, else the random reads of the rows.
-// Measured, us per step over the first 60 steps of an epidemic, state bytes with
-// EARLY, mask with EARLY, mask without: 20 000 agents of degree 10 3.37, 3.17,
-// 3.32; 50 000 of 20 5.63, 5.48, 4.30; 100 000 of 10 5.88, 5.43, 5.34; 100 000 of
-// 25 7.27, 6.89, 5.34; 10^6 of 10 22.5, 19.2, 17.9; 10^6 of 30 40.2, 35.5, 17.8.
+// Measured, us per step over the first 60 steps of an epidemic (agents x degree).
+// Mask, with EARLY and without: 20 000 x 10 3.17 and 3.28; 40 000 x 7 3.84, 4.04;
+// 10 000 x 30 2.82, 2.58; 40 000 x 10 3.90, 3.91; 20 000 x 20 3.80, 3.70; 50 000 x
+// 10 4.92, 4.71; 25 000 x 20 3.99, 3.81; 100 000 x 5 5.39, 5.44; 24 000 x 30 3.32,
+// 2.71; 40 000 x 20 4.73, 4.05; 100 000 x 10 5.30, 5.38; 50 000 x 20 5.49, 4.26;
+// 100 000 x 25 6.89, 5.34; 10^6 x 10 19.2, 17.9; 10^6 x 30 35.5, 17.8: the two
+// cross near 4*10^5 edges.  State bytes: 20 000 x 10 3.25, 3.35; 40 000 x 10 4.30,
+// 4.03; 60 000 x 10 5.33, 4.95; 100 000 x 10 5.90, 5.50; 100 000 x 25 7.14, 5.50;
+// 10^6 x 10 22.6, 20.8; 10^6 x 30 40.1, 22.3.
 template <bool MASK, bool EARLY>
 __global__ void k_sir(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ src,
                       const uint8_t *st_rd, const int32_t *d_rd, uint8_t *st_wr, int32_t *d_wr,
