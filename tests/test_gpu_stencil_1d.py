@@ -1,12 +1,12 @@
-"""Automata on rasters of one dimension by rows (k_life_rows), at lengths where
-the row kernel is the form that is chosen: every remainder modulo a word, one
-tile, two, and many, distances 1 to 4, against a numpy count."""
+"""Automata on rasters of one dimension, which have no neighbouring rows: lengths
+of every remainder modulo a word, below, at and above the row kernel's tiles, as
+long as its rule asks for, distances 1 to 4, against a numpy count."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-# (8 offsets go by rows from 9 cells on, fewer from 10^6 cells x offsets on)
+# (in two dimensions 8 offsets go by rows from 9 cells on, fewer from 10^6 cells x offsets on)
 CASES = [(n, 4) for n in (9, 10, 11, 12, 123, 124, 125, 126, 130, 131, 132, 133, 249, 1000,
                           1_000_001)] + \
         [(166_667, 3), (166_670, 3), (250_000, 2), (250_003, 2), (500_002, 1)]
