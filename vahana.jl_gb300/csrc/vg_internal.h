@@ -669,11 +669,12 @@ inline Sim &peek(vg_sim *h) {
 }
 // and for all others.  What a step left for the very next one (Sim::infected)
 // holds only while no call came between; a call that is being recorded into a
-// CUDA graph may run again, unseen, at any time after.
+// CUDA graph may run again, unseen, at any time after (only queued calls can be
+// recorded: the others wait for the stream).
 inline Sim &enter(vg_sim *h) {
   Sim &s = peek(h);
   s.calls++;
-  if (s.device_ready && !s.columns_shared) {
+  if (s.async && s.device_ready && !s.columns_shared) {
     cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s.stream, &recording) != cudaSuccess) cudaGetLastError();
     else s.columns_shared = recording != cudaStreamCaptureStatusNone;
