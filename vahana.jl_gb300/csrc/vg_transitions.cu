@@ -1772,18 +1772,58 @@ void tr_sir(ApplyCtx &c) {
   s.sir_epoch = s.csr_epoch;
 }
 
-// Where k_life_rows is the faster form.  Measured, us per step, rows and the
-// cell-per-thread kernels: Moore neighbourhood (k_life2d) 601 x 600 8.0 and
-// 7.8, 801 x 800 9.0 and 9.0, 1001 x 1000 9.0 and 11.1; 4 offsets
-// (k_life_stencil) 101 x 100 7.0 and 6.9, 401 x 400 7.0 and 7.0, 601 x 600
-// 7.1 and 10.8; 12 offsets 101 x 100 7.0 and 10.0; 26 offsets 11^3 9.5 and
-// 23.4.  Short rows leave a tile's lanes idle: 4 offsets 9 x 40000 17.2 and
-// 11.1, 17 x 40000 17.3 and 17.2, 33 x 40000 17.3 and 28.5; 12 offsets
-// 5 x 100000 36.9 and 33.0, 9 x 40000 19.2 and 25.5.
-bool rows_pay(const StencilDesc &st, uint64_t ncells, bool moore2d) {
-  if (moore2d) return ncells >= 640000 && st.dims[0] >= 9;
-  return st.noff * std::min<int64_t>(st.dims[0], ROW_TX) >= 72 &&
-         (st.noff >= 8 || ncells * st.noff >= 1000000);
+// Where k_life_rows is the faster form: estimates, in us per launch, of both
+// forms, fitted to 2881 pairs of a raster and a stencil that were measured in both (2
+// to 4 dimensions, 45 to 2.4*10^7 cells, rows of 2 to 10^6 cells, 1 to 10^6 rows, 4
+// to 124 offsets, bounded and periodic).  A tile takes a pass per plane, longer for
+// each of its up to 32 rows; four tiles run on an SM at once, so up to 608 tiles the
+// launch takes what one SM's tiles take beside one another, beyond that the tiles'
+// number times their share.  Whole tiles cost what they cost however few cells they
+// hold.  A cell per thread costs each offset's index arithmetic, growing with the
+// dimensions, and on a periodic raster a division per coordinate that leaves it, for
+// the whole warp when one of its cells does; k_life2d (Moore neighbourhood) costs
+// the lanes of its 32-cell blocks.  With these the chosen form is 0.3 % behind the
+// faster one on average; at worst it is by rows and takes 21.3 us for 18.7 (27 x 195 x
+// 25, 24 offsets), or is not and takes 127 for 95 (11 x 5 x 6 x 256, 88 offsets,
+// periodic).  Measured, rows and a cell per thread: 4 offsets 400 x 64 4.2 and 6.3, 33
+// x 121212 36 and 57, 1000001 x 2 33 and 29; 12 offsets 2001 x 1000 6.8 and 66; Moore
+// 1001 x 1000 5.8 and 10.4, 9 x 111111 35 and 27, 300001 x 3 12.7 and 10.4; 6 offsets 20
+// x 8 x 18750 238 and 74, 20 x 33 x 4545 144 and 74, 248 x 32 x 37 8.9 and 12.5, 62 x 24
+// x 20 7.8 and 6.3; 26 offsets 9 x 8 x 41666 577 and 260, 300 x 100 x 10 10.4 and 33; 8
+// offsets in four dimensions 20 x 32 x 10 x 46 22 and 17; 40 offsets, periodic, 4 x 3 x
+// 3535 x 32 5493 and 385.
+double rows_us(const RowStencil &rs) {
+  const double tiles = (double)rs.tx * rs.ty * rs.dims[2] * rs.dims[3], planes = rs.nplanes;
+  const double full = std::min<int64_t>(rs.dims[1], ROW_TY);      // rows of a whole tile
+  const double mean = (double)rs.dims[1] / rs.ty;                 // and on average
+  const double few = 1.3 + 1.43 * planes + (0.009 + 0.03 * planes) * full +
+                     std::min(tiles, 608.0) / 152 *
+                         (0.05 + 0.084 * planes + (0.005 + 0.0117 * planes) * full);
+  const double many = 1.5 + 1.25 * planes +
+                      tiles / 1e3 * (3.2 * planes + (0.08 + 0.09 * planes) * mean);
+  return std::max(few, many);
+}
+double cells_us(const StencilDesc &st, int reach, uint64_t ncells, bool moore2d) {
+  const double n = (double)ncells / 1e6;
+  // periodic: coordinates of the offsets that may leave the raster, and the share
+  // of the warps that hold a cell whose do
+  int coords = 0;
+  double share = 0;
+  if (st.periodic) {
+    for (int v : st.offsets) coords += v != 0;
+    double before = (double)st.dims[0];
+    share = (31 + reach) / before;
+    for (int i = 1; i < st.ndims; i++) {
+      share += std::min(1.0, reach / (double)st.dims[i] * std::max(1.0, 32 / before));
+      before *= (double)st.dims[i];
+    }
+    share = std::min(share, 1.0);
+  }
+  if (moore2d)
+    return std::max(4.0, 3.7 + n * (6.4 * ((st.dims[0] + 31) / 32 * 32) / st.dims[0] + 6 * share));
+  return std::max(4.3 + 0.33 * st.noff + (0.12 * st.ndims - 0.03) * std::max(0, coords - st.noff),
+                  3.5 + 0.19 * st.noff +
+                      n * (5 + (0.5 + 0.83 * st.ndims) * st.noff + share * coords));
 }
 
 // The stencil as rows for k_life_rows; false when it is none (an offset
@@ -1892,8 +1932,8 @@ void tr_life(ApplyCtx &c) {
     launch_dependent(ad.fields[0].dtype == VG_BOOL ? k_life2d_x4<true> : k_life2d_x4<false>, grd,
                      blk, 0, s.stream, (const uint32_t *)in, (uint32_t *)out, (int)Wq, st.dims[1],
                      st.periodic);
-  } else if (ad.fields[0].dtype == VG_BOOL && rows_pay(st, R.ncells, moore2d) &&
-             row_stencil(st, birth, survive, rs, reach)) {
+  } else if (ad.fields[0].dtype == VG_BOOL && row_stencil(st, birth, survive, rs, reach) &&
+             1.06 * rows_us(rs) < cells_us(st, reach, R.ncells, moore2d)) {
     const uint64_t blocks = (uint64_t)rs.tx * rs.ty * rs.dims[2] * rs.dims[3];
     dim3 blk(32, 8);
     const int code = rs.nplanes == 1 ? rs.plane[0].code : -1;
