@@ -206,6 +206,7 @@ void check_device_status(Sim &s, const char *what) {
   if (h) {
     VG_CUDA(cudaMemsetAsync(s.d_status.p, 0, 4, s.stream));
     if (s.pin) *(volatile int *)s.pin = 0;
+    if (h == STATUS_NO_AGENT) fail(VG_ERR_ASSERT, "an edge targets an agent that does not exist");
     fail(VG_ERR_DEVICE, std::string(what) + ": device status " + std::to_string(h));
   }
 }

@@ -423,6 +423,7 @@ struct StatusWord {
   int code, pad;
   int *host;  // may be null
 };
+constexpr int STATUS_NO_AGENT = 501;  // an edge to an agent that does not exist (VG_ERR_ASSERT)
 constexpr size_t PIN_FETCH = 192, PIN_RESULTS = 256, PIN_BYTES = 64 + PIN_FETCH + PIN_RESULTS;
 #ifdef __CUDACC__
 // programmatic dependent launches: the next kernel of the stream may start

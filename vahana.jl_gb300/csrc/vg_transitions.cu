@@ -615,7 +615,7 @@ __global__ void k_link_slots(Sweep s, DevCSRView c, Append ap, int pl_dt, int ha
     const uint32_t id = r0 + owner;
     uint32_t nid = c.src[e];
     if (swept && nid >= s.a.n) {  // an edge from an agent that does not exist
-      set_status(s.status, 501);
+      set_status(s.status, STATUS_NO_AGENT);
       nid = id;
     }
     ((uint2 *)ap.rows)[e] = swept ? make_uint2(id, nid) : make_uint2(BK_HOLE, BK_HOLE);
