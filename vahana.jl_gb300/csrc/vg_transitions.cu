@@ -187,16 +187,35 @@ __global__ void k_neighbor_op(Sweep s, DevCSRView c, SrcTable t, int dst,
 }
 
 // modes 0 and 1 where all sources are of one type, its column of type E:
-// NB_U edges of a row in flight (sources, then values and died flags), folded
-// in the row's order.  One edge at a time, its source's type and the column's
-// looked up for each, left one load in flight per lane.  Bound: the random
-// reads, for a row beyond the others the chain of its additions.  Measured, us,
-// before and now: 10^5 agents with 2*10^6 edges 20.9 and 15.0, 10^6 with 2*10^7
-// 229 and 168, one row of 10^6 edges 434 000 and 108 000; 16 in flight 16.3,
-// 185 and 115 000.
-constexpr int NB_U = 8;
+// U edges of a row in flight (sources, then values and died flags), folded in
+// the row's order.  One edge at a time, its source's type and the column's
+// looked up for each (k_neighbor_op), left one load in flight per lane.  Bound:
+// the random reads; for short rows the rows' own words, for a row beyond the
+// others the chain of its additions.
+//
+// Rows of few edges take 4, long ones 8.  The registers of 8 (40 and 48, of 4
+// 32) leave fewer warps to hide a short row's reads, and what a lane adds beyond
+// its row's end costs the binary64 pipe (additions, conversions) as much as an
+// edge: with 4 the warp stops at its longest rest.  us, k_neighbor_op, 8 and 4
+// edges in flight, f32 column into f64, then i32 column:
+//   5*10^6 agents, 10^5 edges       65  122  64    65   96  64
+//   10^6 agents, 5*10^5 edges       21   38  18    18   17  13
+//   10^6 agents, 4*10^6 edges       46   55  42    33   27  25
+//   10^6 agents, 1.4*10^7 edges    103  106  93    90   64  63
+// and, f64 column and i32 column, where 8 are the better ones:
+//   20000 agents, 6*10^5 edges      26   11  13    24    9  11
+//   one row of 2*10^5 edges (ms)    70   19  22    67   14  16
+// 6 in flight lie between the two.
+constexpr int NB_SHORT = 4, NB_LONG = 8;
 
-template <class E>
+// NB_LONG: a container of 16 edges a row (f64 column, 20000 agents of 14
+// edges, us: 9.0 and, with NB_SHORT, 9.2; of 20 edges 9.6 and 11.2), or one
+// whose longest row is known to have 1024 and so outlasts the others
+inline bool neighbor_rows_long(uint64_t nrows, uint64_t nedges, uint32_t longest) {
+  return nedges / 16 >= nrows || longest >= 1024;
+}
+
+template <class E, int U>
 __global__ void __launch_bounds__(256) k_neighbor_typed(Sweep s, DevCSRView c,
                                                         const E *__restrict__ val,
                                                         const uint8_t *died, int dst, int mode) {
@@ -212,27 +231,38 @@ __global__ void __launch_bounds__(256) k_neighbor_typed(Sweep s, DevCSRView c,
     b = c.row_ptr[i];
     e = c.row_ptr[i + 1];
   }
-  for (uint32_t k = b; k < e; k += NB_U) {
-    uint32_t j[NB_U];
-    E v[NB_U];
+  for (uint32_t k = b; k < e; k += U) {
+    uint32_t j[U];
+    E v[U];
 #pragma unroll
-    for (int u = 0; u < NB_U; u++) j[u] = k + u < e ? c.src[k + u] : 0u;
+    for (int u = 0; u < U; u++) j[u] = k + u < e ? c.src[k + u] : 0u;
 #pragma unroll
-    for (int u = 0; u < NB_U; u++) v[u] = k + u < e ? val[j[u]] : E(0);
+    for (int u = 0; u < U; u++) v[u] = k + u < e ? val[j[u]] : E(0);
     if (died) {
 #pragma unroll
-      for (int u = 0; u < NB_U; u++) gone |= k + u < e && died[j[u]];
+      for (int u = 0; u < U; u++) gone |= k + u < e && died[j[u]];
     }
-    if (sums) {
+    if constexpr (U == NB_SHORT) {
+      const unsigned lanes = __activemask();
 #pragma unroll
-      for (int u = 0; u < NB_U; u++)
+      for (int u = 0; u < U; u++) {
+        if (u && !__any_sync(lanes, k + u < e)) break;
+        if (k + u < e) {
+          if (sums) sf = __dadd_rn(sf, (double)v[u]);
+          else if (mode == 0) si = (int64_t)((uint64_t)si + (uint64_t)(int64_t)v[u]);
+          else si |= (int64_t)v[u];
+        }
+      }
+    } else if (sums) {
+#pragma unroll
+      for (int u = 0; u < U; u++)
         if (k + u < e) sf = __dadd_rn(sf, (double)v[u]);
     } else if (mode == 0) {
 #pragma unroll
-      for (int u = 0; u < NB_U; u++) si = (int64_t)((uint64_t)si + (uint64_t)(int64_t)v[u]);
+      for (int u = 0; u < U; u++) si = (int64_t)((uint64_t)si + (uint64_t)(int64_t)v[u]);
     } else {
 #pragma unroll
-      for (int u = 0; u < NB_U; u++) si |= (int64_t)v[u];
+      for (int u = 0; u < U; u++) si |= (int64_t)v[u];
     }
   }
   if (gone) set_status(s.status, 203);
@@ -1438,11 +1468,16 @@ void launch_neighbor_op(ApplyCtx &c, int mode) {
   if (w.a.n == 0) return;
   const int T = v.src_type || mode == 2 ? 0 : v.src_type_const;
   const unsigned g = nblk(w.a.n);
+  const CSR *rows = c.call_type < (int)s.edges[e].csr.size() ? &s.edges[e].csr[c.call_type] : nullptr;
+  const bool rows_long =
+      neighbor_rows_long(w.a.n, v.nedges, rows && !rows->max_degree_pending ? rows->max_degree : 0);
   auto typed = [&](auto zero) {
     using E = decltype(zero);
-    k_neighbor_typed<E><<<g, TPB, 0, s.stream>>>(w, v, (const E *)t.ptr[T], t.died[T], df, mode);
+    auto k = rows_long ? k_neighbor_typed<E, NB_LONG> : k_neighbor_typed<E, NB_SHORT>;
+    k<<<g, TPB, 0, s.stream>>>(w, v, (const E *)t.ptr[T], t.died[T], df, mode);
   };
-  if (T > 0 && T < MAX_AGENT_TYPES && t.ptr[T] && v.src) {
+  // (the last rows' edge indices plus a batch stay below 2^32)
+  if (T > 0 && T < MAX_AGENT_TYPES && t.ptr[T] && v.src && v.nedges < UINT32_MAX - NB_LONG) {
     switch (t.dt[T]) {
       case VG_BOOL: case VG_U8: typed(uint8_t()); break;
       case VG_I8: typed(int8_t()); break;
